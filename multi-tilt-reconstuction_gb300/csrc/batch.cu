@@ -8,8 +8,8 @@
 //   residual        item = (axis, 64 Ki pixels)     residual_batch_kernel
 //   back-projection item = (axis, brick)            bp_batch_kernel
 //   MACE consensus  item = (instance, 64 Ki voxels) mace_batch_kernel
-// so small instances no longer leave SMs idle.  An axis with enough bricks to
-// fill the GPU for kOwnWaves waves, an axis tuned to patch tiles, and an axis
+// so small instances no longer leave SMs idle.  An axis on line kernels, one with
+// enough bricks to fill the GPU for kOwnWaves waves, one tuned to patch tiles and one
 // whose window fits no TMA box keep their own launches instead (arguments in
 // the constant bank, which the persistent kernels have to stage through
 // shared memory): each such axis' forward -> residual -> back-projection
@@ -106,7 +106,7 @@ mtr_status mtr::build_sirt_tables(mtr_context* ctx, const std::vector<mtr_recon*
       const bool fwd_ok = a.ftma && !tma_disabled() && fp.lanes != 2 &&
                           (long long)fgx * fgy * ((v.NZ + fp.nz - 1) / fp.nz) <
                               (long long)kOwnWaves * ctx->num_sms * forward_ctas_per_sm(ck, fp.smem);
-      if (!bp_ok || !fwd_ok) {  // the whole SIRT chain of this axis runs on its own launches
+      if (a.lines || !bp_ok || !fwd_ok) {  // the whole SIRT chain of this axis runs on its own launches
         t.own.push_back({r, k});
         continue;
       }

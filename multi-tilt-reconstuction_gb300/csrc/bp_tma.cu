@@ -106,6 +106,8 @@ cudaError_t launch_backproject_batch(const BpBatchDesc* descs, const long long* 
   return le;
 }
 
+unsigned pipeline_wait_limit() { return g_wait_iters.load(std::memory_order_relaxed); }
+
 void set_pipeline_wait_limit(long long polls) {
   g_wait_iters.store(polls < 0 ? (1u << 24) : (unsigned)std::min<long long>(polls, 0xffffffffLL),
                      std::memory_order_relaxed);

@@ -156,6 +156,7 @@ cudaError_t launch_backproject_tma(const CUtensorMap& map, const BpPlan& plan, c
 // Polls a pipeline wait of the windowed back-projection makes before it
 // gives up and flags the launch (negative: the default, 2^24); read at launch.
 void set_pipeline_wait_limit(long long polls);
+unsigned pipeline_wait_limit();
 
 // 3-D tiled tensor map over [depth][height][pitch] fp32/fp16 elements with
 // logical width `width`, box (bw, bh, 1), zero fill (bp_tma.cu).

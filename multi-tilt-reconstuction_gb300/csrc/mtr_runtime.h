@@ -9,6 +9,7 @@
 #include <string>
 #include <vector>
 
+#include "line.cuh"
 #include "mtr_internal.h"
 
 struct mtr_context {
@@ -286,6 +287,18 @@ struct AxisState {
   FwdPlan fplan;          // windowed forward splat plan
   CUtensorMap map_s{}, map_cf{};  // tensor maps over s and cf (valid when ftma)
   bool ftma = false;
+  // Axes whose maps separate run on line images instead of windows (line.cuh):
+  // the line sums live in s ([A][PX][line.Wp]), the residual's (before the
+  // first SIRT iteration, the projections') line image in r.
+  LinePlan line;
+  CUtensorMap map_ls{}, map_lr{}, map_lb{};  // over s; over r for the SIRT update and the WBP
+  DevBuf line_tab;
+  bool lines = false;
+  LineTab tab() const {
+    const int* t = line_tab.as<int>();
+    return LineTab{reinterpret_cast<const int2*>(t), reinterpret_cast<const int2*>(t + line.off_rows),
+                   reinterpret_cast<const float*>(t + line.off_weight), line.n_tab > 1 ? 1 : 0};
+  }
   DevBuf xc, yc;          // [A*4] doubles
   DevBuf b;               // projections: float (FP32) or half (mixed)
   DevBuf s;               // forward accumulator, float
@@ -325,6 +338,11 @@ bool tma_disabled();
 // the forward splat for one axis, timing candidates on the axis' buffers
 // before they hold data, and encodes the tensor maps.
 bool autotune_enabled();
+// MTR_FORCE_DEPTHS pins the windowed kernels' tiles (no axis runs on lines).
+bool windows_forced();
+// An axis on line kernels is not tuned; the cache file lists the windowed
+// kernels' heuristic tile for it under a key of its own.
+void record_untimed_tiles(const AxisState& a, const VolDev& v, int precision);
 // Candidates run over the frame v on device scratch: scratch_vol / scratch_cbp
 // (FP32) and, in mixed precision, scratch_copy (the BF16 / FP16 copy the
 // forward splat reads); none of them holds data yet.

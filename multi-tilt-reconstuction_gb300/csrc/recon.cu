@@ -139,6 +139,15 @@ mtr_status enqueue_geometry(mtr_recon* r) {
   for (auto& a : r->ax) {
     MTR_CK(ctx, cudaMemsetAsync(a.cf.p, 0, (size_t)a.np * 4, ctx->stream));
     ProfScope ps(ctx, MTR_KERNEL_OTHER);
+    if (a.lines) {
+      cudaError_t e = launch_line_forward<float>(a.map_ls, a.line, a.dev(), v, nullptr, v.Zs, v.Zs + v.NZ, ctx->stream);
+      if (e == cudaSuccess)
+        e = launch_line_rows<float>(1, a.line, a.tab(), a.dev(), nullptr, a.s.as<float>(), a.cf.as<float>(), nullptr,
+                                    nullptr, ctx->stream);
+      g_launches.fetch_add(2);
+      if (e != cudaSuccess) return cuda_error(ctx, e, "forward row sums (lines)");
+      continue;
+    }
     if (a.ftma) {
       cudaError_t e = launch_forward_tma<float>(a.map_cf, a.fplan, a.dev(), v, nullptr, v.Zs, v.Zs + v.NZ,
                                                 r->err.as<int>(), ctx->stream);
@@ -161,6 +170,20 @@ mtr_status enqueue_forward(mtr_recon* r, AxisState& a, const VolSpan& sp) {
   const VolDev& v = r->vol;
   const int z0 = sp.z0, z1 = sp.z1;
   ProfScope ps(ctx, MTR_KERNEL_FORWARD);
+  if (a.lines) {
+    cudaError_t e;
+    switch (copy_kind_of(r->p.precision)) {
+      case 1: e = launch_line_forward<__nv_bfloat16>(a.map_ls, a.line, a.dev(), v,
+                                                      static_cast<const __nv_bfloat16*>(sp.xcopy), z0, z1,
+                                                      ctx->stream); break;
+      case 2: e = launch_line_forward<__half>(a.map_ls, a.line, a.dev(), v, static_cast<const __half*>(sp.xcopy), z0,
+                                               z1, ctx->stream); break;
+      default: e = launch_line_forward<float>(a.map_ls, a.line, a.dev(), v, sp.x, z0, z1, ctx->stream); break;
+    }
+    g_launches.fetch_add(1);
+    if (e != cudaSuccess) return cuda_error(ctx, e, "line sums");
+    return MTR_OK;
+  }
   if (a.ftma) {
     cudaError_t e;
     switch (copy_kind_of(r->p.precision)) {
@@ -192,6 +215,18 @@ mtr_status enqueue_residual(mtr_recon* r, AxisState& a, double* norm) {
   mtr_context* ctx = r->ctx;
   ProfScope ps(ctx, MTR_KERNEL_RESIDUAL);
   const long long rows = (long long)a.A * a.PY;
+  if (a.lines) {
+    cudaError_t e;
+    if (mixed(r->p.precision))
+      e = launch_line_rows<__half>(0, a.line, a.tab(), a.dev(), a.b.as<__half>(), a.s.as<float>(), a.cf.as<float>(),
+                                   a.r.as<float>(), norm, ctx->stream);
+    else
+      e = launch_line_rows<float>(0, a.line, a.tab(), a.dev(), a.b.as<float>(), a.s.as<float>(), a.cf.as<float>(),
+                                  a.r.as<float>(), norm, ctx->stream);
+    g_launches.fetch_add(1);
+    if (e != cudaSuccess) return cuda_error(ctx, e, "line residual");
+    return MTR_OK;
+  }
   if (a.tma && a.plan.pairs) {  // this axis' windowed update reads (value, next - value) pairs
     if (mixed(r->p.precision))
       launch_residual_pairs<__half>(rows, a.pitch, a.pitch2, a.b.as<__half>(), a.s.as<float>(), a.cf.as<float>(),
@@ -210,9 +245,20 @@ mtr_status enqueue_residual(mtr_recon* r, AxisState& a, double* norm) {
   return MTR_OK;
 }
 
-// Mixed precision: the windowed WBP gathers FP32 windows, so the FP16
-// projections are first widened into r (free until the first residual).
+// What the WBP gathers, prepared in r (free until the first residual): with
+// line kernels the projections' line image, and in mixed precision the FP16
+// projections widened for the FP32 windows.
 mtr_status enqueue_widen_for_wbp(mtr_recon* r, AxisState& a) {
+  if (a.lines) {  // the WBP gathers the projections' line image
+    const cudaError_t e =
+        mixed(r->p.precision)
+            ? launch_line_rows<__half>(2, a.line, a.tab(), a.dev(), a.b.as<__half>(), nullptr, nullptr,
+                                       a.r.as<float>(), nullptr, r->ctx->stream)
+            : launch_line_rows<float>(2, a.line, a.tab(), a.dev(), a.b.as<float>(), nullptr, nullptr,
+                                      a.r.as<float>(), nullptr, r->ctx->stream);
+    g_launches.fetch_add(1);
+    return e == cudaSuccess ? MTR_OK : cuda_error(r->ctx, e, "projections' line image");
+  }
   if (!(a.tma_b && mixed(r->p.precision))) return MTR_OK;
   launch_widen(a.b.as<__half>(), a.r.as<float>(), a.np, r->ctx->stream);
   MTR_CK_LAUNCH(r->ctx, "widen projections");
@@ -230,6 +276,18 @@ mtr_status enqueue_bp(mtr_recon* r, AxisState& a, int mode, const VolSpan& sp, b
   ProfScope ps(ctx, mode == 0 ? MTR_KERNEL_WBP : MTR_KERNEL_BACKPROJECT);
   // WBP reads the projections (fp16 when mixed), SIRT reads the FP32 residual.
   const bool half_img = mode == 0 && mixed(r->p.precision);
+  if (a.lines) {
+    if (mode == 0 && widen) {
+      const mtr_status s = enqueue_widen_for_wbp(r, a);
+      if (s != MTR_OK) return s;
+    }
+    const cudaError_t e = launch_line_backproject(mode == 0 ? a.map_lb : a.map_lr, a.line, a.tab(), a.dev(), v, mode,
+                                                  r->p.sirt_step, sp.x, sp.cbp, sp.xcopy, ck, z0, z1,
+                                                  r->err.as<int>(), ctx->stream);
+    g_launches.fetch_add(1);
+    if (e != cudaSuccess) return cuda_error(ctx, e, "line back-projection");
+    return MTR_OK;
+  }
   if (mode == 0 ? a.tma_b : a.tma) {
     if (half_img && widen) {
       mtr_status s = enqueue_widen_for_wbp(r, a);
@@ -388,6 +446,25 @@ mtr_status enqueue_run(mtr_recon* r) {
   return enqueue_outer(r, 0, r->p.iter_times);
 }
 
+// Line plan, tables and tensor maps of an axis whose maps separate (`depth`:
+// planes of a launch, a whole volume or a streamed slab).
+mtr_status setup_lines(mtr_recon* r, AxisState& a, int depth) {
+  mtr_context* ctx = r->ctx;
+  VolDev v = r->vol;
+  a.line = plan_lines(a.hxc, a.hyc, a.A, a.PX, a.PY, a.pitch, v, depth, ctx->num_sms);
+  LinePlan& p = a.line;
+  if (!p.ok) return MTR_OK;
+  if (!encode_tensor_map_3d(&a.map_ls, a.s.p, false, p.W, p.Wp, a.PX, a.A, 32 * p.fwd_vl, p.fwd_rows) ||
+      !encode_tensor_map_3d(&a.map_lr, a.r.p, false, p.W, p.Wp, a.PX, a.A, 32 * p.bp_vl, p.bp_rows) ||
+      !encode_tensor_map_3d(&a.map_lb, a.r.p, false, p.W, p.Wp, a.PX, a.A, 32 * p.wbp_vl, p.wbp_rows))
+    return MTR_OK;
+  MTR_CK(ctx, a.line_tab.alloc_pooled(p.tables.size() * sizeof(int), ctx));
+  MTR_CK(ctx, cudaMemcpyAsync(a.line_tab.p, p.tables.data(), p.tables.size() * sizeof(int), cudaMemcpyHostToDevice,
+                              ctx->stream));
+  a.lines = true;
+  return MTR_OK;
+}
+
 // Checkpoint file: header, then w_avg and w_k of every axis (float32, x fastest).
 struct CkptHeader {
   char magic[8];  // "MTRCKPT1"
@@ -519,8 +596,15 @@ mtr_status mtr_recon_create(mtr_context* ctx, int n_axes, const mtr_axis* axes, 
     } else {  // zero until mtr_recon_upload / mtr_recon_upload_half
       MTR_CK(ctx, cudaMemsetAsync(a.b.p, 0, (size_t)a.np * pe, ctx->stream));
     }
-    // TMA kernels where the window geometry fits (else the plain kernels run).
-    if (!tma_disabled()) {
+    // Line kernels where the maps separate, else TMA-windowed kernels where the
+    // window geometry fits (else the plain kernels run).
+    if (!tma_disabled() && !windows_forced()) {
+      s = setup_lines(r.get(), a, streamed ? r->slabs->depth : r->vol.NZ);
+      if (s != MTR_OK) return s;
+    }
+    if (a.lines) {
+      record_untimed_tiles(a, r->vol, params->precision);
+    } else if (!tma_disabled()) {
       // WBP over b; with FP16 projections over their FP32 widening in r (r is
       // free until the first residual), so the WBP gathers FP32 like SIRT.
       // SIRT back-projection over the FP32 residual and the forward splat: tuned depths
@@ -848,6 +932,17 @@ mtr_status mtr_recon_describe(const mtr_recon* r, char* buf, int cap) {
   for (size_t k = 0; k < r->ax.size(); ++k) {
     const AxisState& a = r->ax[k];
     char t[512];
+    if (a.lines) {
+      const char* dir = a.line.along_x ? "line x" : "line y";
+      std::snprintf(t, sizeof(t),
+                    "%s{\"axis\":%zu,\"back_projection\":{\"tma\":true,\"depth\":%d,\"window\":[%d,%d],\"lanes\":\"%s\","
+                    "\"window_format\":\"line image\"},"
+                    "\"forward\":{\"tma\":true,\"depth\":%d,\"window\":[%d,%d],\"lanes\":\"%s\",\"y_has_z\":false}}",
+                    k ? "," : "", k, a.line.bp_nz, 32 * a.line.bp_vl, a.line.bp_rows, dir, a.line.fwd_nz,
+                    32 * a.line.fwd_vl, a.line.fwd_rows, dir);
+      s += t;
+      continue;
+    }
     std::snprintf(t, sizeof(t),
                   "%s{\"axis\":%zu,\"back_projection\":{\"tma\":%s,\"depth\":%d,\"window\":[%d,%d],\"lanes\":\"%s\","
                   "\"window_format\":\"%s\"},"

@@ -174,6 +174,21 @@ bool autotune_enabled() {
   return !(e && e[0] == '0');
 }
 
+bool windows_forced() {
+  const char* f = std::getenv("MTR_FORCE_DEPTHS");
+  int bp = 0, fwd = 0;
+  return f && std::sscanf(f, "%d,%d", &bp, &fwd) == 2;
+}
+
+void record_untimed_tiles(const AxisState& a, const VolDev& v, int precision) {
+  if (!cache_path()) return;
+  Choice c;
+  c.bp_lane = c.fwd_lane = a.line.along_x ? 0 : 1;
+  std::lock_guard<std::mutex> lock(g_mu);
+  load_file();
+  if (g_cache.emplace(geometry_key(a, v, precision) + "_lines", c).second) save_file();
+}
+
 // Chooses a.plan (SIRT back-projection over r) and a.fplan (forward splat
 // over s) for one axis and encodes the matching tensor maps.  Leaves s zeroed.
 bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, int precision, float* scratch_vol,
