@@ -246,6 +246,38 @@ __device__ __forceinline__ void bp_column_blended(float (&s)[NZ], const float2* 
   }
 }
 
+// A column whose y-map has a Z term and whose taps all lie in the window: a
+// position, its floor (one addition that rounds down) and its fraction per
+// coordinate and voxel, and the taps without a check of their own.
+template <int NZ, bool PAIR, bool HALF, typename WT>
+__device__ __forceinline__ void bp_column_zy(float (&s)[NZ], const WT* win, int WX, float xr, float yr,
+                                             const WinConst& k) {
+  const uint32_t base = smem_u32(win);
+  const uint32_t es = sizeof(WT), dr = es * (uint32_t)WX;
+#pragma unroll
+  for (int z = 0; z < NZ; ++z) {
+    const float x = fmaf(k.a3, (float)z, xr), y = fmaf(k.b3, (float)z, yr);
+    const float tx = __fadd_rd(x, kMagic), ty = __fadd_rd(y, kMagic);  // floor, in the low bits
+    const float fx = x - (tx - kMagic), fy = y - (ty - kMagic);
+    const uint32_t p = base + es * (uint32_t)((__float_as_int(ty) + k.lym) * WX + (__float_as_int(tx) + k.lxm));
+    float r0, r1;
+    if constexpr (HALF) {
+      const float2 q0 = lds_h2_widened<0>(p), q1 = lds_h2_widened<0>(p + dr);
+      r0 = fmaf(fx, q0.y, q0.x);
+      r1 = fmaf(fx, q1.y, q1.x);
+    } else if constexpr (PAIR) {
+      const float2 q0 = lds_f32x2<0>(p), q1 = lds_f32x2<0>(p + dr);
+      r0 = fmaf(fx, q0.y, q0.x);
+      r1 = fmaf(fx, q1.y, q1.x);
+    } else {
+      const float p00 = lds_f32<0>(p), p10 = lds_f32<4>(p), p01 = lds_f32<0>(p + dr), p11 = lds_f32<4>(p + dr);
+      r0 = fmaf(fx, p10 - p00, p00);
+      r1 = fmaf(fx, p11 - p01, p01);
+    }
+    s[z] = fmaf(fy, r1 - r0, s[z] + r0);
+  }
+}
+
 // One brick (bx, by, bz) of one axis.  LANES: 0 = each warp a line of 32
 // voxels along X (brick 32x8), 1 = a line along Y (brick 8x32, used when the
 // detector x follows Y), 2 = an 8x4 patch (brick 32x8: on oblique axes the
@@ -413,6 +445,23 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
       __syncwarp();
     }
     bool done = !active;
+    if (active && !BZ0) {
+      // x and y are affine in z: the column's end voxels bound every tap, so
+      // the window (and for the WBP the detector) is checked once per column
+      const float xe = fmaf(k.a3, (float)(NZ - 1), xr), ye = fmaf(k.b3, (float)(NZ - 1), yr);
+      const int ixa = magic_int(floorf(xr)) + k.lxm, ixb = magic_int(floorf(xe)) + k.lxm;
+      const int iya = magic_int(floorf(yr)) + k.lym, iyb = magic_int(floorf(ye)) + k.lym;
+      bool inside = (unsigned)min(ixa, ixb) < lim_x && (unsigned)max(ixa, ixb) < lim_x &&
+                    (unsigned)min(iya, iyb) < lim_y && (unsigned)max(iya, iyb) < lim_y;
+      if (MODE == 0)
+        inside = inside && min(ixa, ixb) + k.ox >= 0 && max(ixa, ixb) + 1 + k.ox < P.ax.PX &&
+                 min(iya, iyb) + k.oy >= 0 && max(iya, iyb) + 1 + k.oy < P.ax.PY;
+      if (inside) {
+        bp_column_zy<NZ, PAIR, HALF>(s, w, WX, xr, yr, k);
+        if (MODE == 0) ++n_inside;
+        done = true;
+      }
+    }
     if (active && BZ0 && fabsf(k.a3) < 0.999f) {
       // x is affine in z: the column's end voxels bound every tap index, so
       // the window bound is checked once per column instead of per voxel; the

@@ -30,7 +30,8 @@
 // (2-16x fewer shared-memory adds than four per voxel, depending on the tilt),
 // in branch-free chunks where the slope allows, with red.shared adds on 32-bit
 // shared addresses; bricks at the detector edge check each add against the
-// window.  The per-tap path remains for z-dependent y-maps and slopes >= 0.999.
+// window.  Where the y-map has a Z term the walk carries two rows.  The per-tap
+// path remains for slopes >= 0.999.
 //
 // Windows are clamped inside the detector (TMA reduces must not start at a
 // negative coordinate), so a tap is on the detector iff it lies in the valid
@@ -212,6 +213,77 @@ __device__ __forceinline__ void splat_column(uint32_t row, int WX, const float (
   else stream_column<NZ, 1, ROW, CHK>(row, WX, v, xr, a3, lxm, wy0, wy1, span, y0ok, y1ok);
 }
 
+// The same for a y-map with a Z term: the column also moves by |b3| < 1 per
+// voxel through the detector rows (mirrored where b3 < 0, as x is where a3 <
+// 0), so four sums are carried: the weight not yet emitted of the current row
+// and the next (S0, S1), and its parts on the next pixel (X0, X1).  At a pixel
+// crossing one pixel is emitted in both rows; at a row crossing the two pixels
+// of the row left are, and the next row's sums move down.  Two shared-memory
+// adds per pixel and two per row crossed, against four per voxel tap by tap:
+// 320x300x72 voxels, 51 angles, rows crossed every ~100 voxels, 0.55 ms
+// against 0.72 ms (bound by issue: 40 instructions per voxel and angle, half
+// of them in the crossings that some lane of a warp takes at almost every voxel).
+// CHK as in stream_column.
+template <int NZ, bool CHK>
+__device__ __forceinline__ void stream_column_zy(uint32_t win, int WX, int WY, const float (&v)[NZ], float xr,
+                                                 float yr, const FwdConst& k) {
+  const int dir = k.a3 >= 0.f ? 1 : -1, diry = k.b3 >= 0.f ? 1 : -1;
+  const float u = dir > 0 ? xr : -xr, t = diry > 0 ? yr : -yr;
+  const float flu = floorf(u), flt = floorf(t);
+  float fx = u - flu, fy = t - flt;
+  const float step = fabsf(k.a3), stepy = fabsf(k.b3);
+  const int col = (k.lxm + kMagicBits) + dir * (magic_int(flu) - kMagicBits);
+  int row = (k.lym + kMagicBits) + diry * (magic_int(flt) - kMagicBits);
+  uint32_t rowa = win + 4u * (uint32_t)(row * WX);  // address of the current row
+  uint32_t at = rowa + 4u * (uint32_t)col;
+  const uint32_t dstep = dir > 0 ? 4u : 0xFFFFFFFCu;
+  const uint32_t drow = diry > 0 ? 4u * (uint32_t)WX : 0u - 4u * (uint32_t)WX;
+  const uint32_t span = 4u * (uint32_t)k.wlx;
+  auto emit0 = [&](uint32_t q, float e) {  // current row
+    if (!CHK || (q - rowa < span && (unsigned)row < (unsigned)WY)) red_shared(q, fixq(1.f, e));
+  };
+  auto emit1 = [&](uint32_t q, float e) {  // next row
+    if (!CHK || (q - rowa < span && (unsigned)(row + diry) < (unsigned)WY)) red_shared(q + drow, fixq(1.f, e));
+  };
+  float g1 = fy * v[0], g0 = v[0] - g1;
+  float S0 = g0, S1 = g1, X0 = fx * g0, X1 = fx * g1;
+#pragma unroll
+  for (int z = 1; z < NZ; ++z) {
+    fx += step;
+    fy += stepy;
+    if (fy >= 1.f) {  // the column left the current row
+      emit0(at, S0 - X0);
+      emit0(at + dstep, X0);
+      S0 = S1;
+      X0 = X1;
+      S1 = X1 = 0.f;
+      fy -= 1.f;
+      at += drow;
+      rowa += drow;
+      if (CHK) row += diry;
+    }
+    if (fx >= 1.f) {  // the column left the current pixel
+      emit0(at, S0 - X0);
+      emit1(at, S1 - X1);
+      S0 = X0;
+      S1 = X1;
+      X0 = X1 = 0.f;
+      fx -= 1.f;
+      at += dstep;
+    }
+    g1 = fy * v[z];
+    g0 = v[z] - g1;
+    S0 += g0;
+    S1 += g1;
+    X0 = fmaf(fx, g0, X0);
+    X1 = fmaf(fx, g1, X1);
+  }
+  emit0(at, S0 - X0);
+  emit1(at, S1 - X1);
+  emit0(at + dstep, X0);
+  emit1(at + dstep, X1);
+}
+
 // One brick (bx, by, zb) and angle group g of one axis; `smem` is the CTA's
 // dynamic shared memory.  On return every bulk reduce it issued is complete.
 template <typename VT, int LANES, bool BZ0, int NZ>
@@ -375,6 +447,11 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
         red_shared(a1, fixq(wx0, g1));
         red_shared(a1 + 4u, fixq(fx, g1));
       }
+    } else if (active && !BZ0 && fabsf(k.a3) < 0.999f && fabsf(k.b3) < 0.999f) {
+      const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
+      const float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
+      if (k.interior) stream_column_zy<NZ, false>(smem_u32(wi), WX, WY, v, xr, yr, k);
+      else stream_column_zy<NZ, true>(smem_u32(wi), WX, WY, v, xr, yr, k);
     } else if (active) {
       const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
       const float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
@@ -475,17 +552,12 @@ cudaError_t launch_one(const CUtensorMap& map, FwdArgs P, size_t smem, int num_s
   return le;
 }
 
-// Z-dependent y-maps take the per-tap path and use one depth.
 template <typename VT, int LY, bool BZ>
 cudaError_t launch_nz(const CUtensorMap& map, const FwdArgs& P, const FwdPlan& plan, int sms, cudaStream_t st) {
-  if constexpr (!BZ) {
-    return launch_one<VT, LY, false, 16>(map, P, plan.smem, sms, st);
-  } else {
-    if (plan.nz == 16) return launch_one<VT, LY, true, 16>(map, P, plan.smem, sms, st);
-    if (plan.nz == 8) return launch_one<VT, LY, true, 8>(map, P, plan.smem, sms, st);
-    if (plan.nz == 32) return launch_one<VT, LY, true, 32>(map, P, plan.smem, sms, st);
-    return cudaErrorInvalidValue;
-  }
+  if (plan.nz == 16) return launch_one<VT, LY, BZ, 16>(map, P, plan.smem, sms, st);
+  if (plan.nz == 8) return launch_one<VT, LY, BZ, 8>(map, P, plan.smem, sms, st);
+  if (plan.nz == 32) return launch_one<VT, LY, BZ, 32>(map, P, plan.smem, sms, st);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace
@@ -501,8 +573,12 @@ namespace {
 template <typename VT, int NZ>
 __device__ __forceinline__ void fwd_batch_item(const CUtensorMap* map, const FwdArgs& P, const int* b,
                                                unsigned char* smem) {
-  if (b[4] == 3) fwd_brick<VT, 1, true, NZ>(map, P, b[0], b[1], b[2], 0, smem);
-  else fwd_brick<VT, 0, true, NZ>(map, P, b[0], b[1], b[2], 0, smem);
+  switch (b[4]) {
+    case 0: fwd_brick<VT, 0, false, NZ>(map, P, b[0], b[1], b[2], 0, smem); break;  // z-dependent y-map
+    case 1: fwd_brick<VT, 0, true, NZ>(map, P, b[0], b[1], b[2], 0, smem); break;
+    case 2: fwd_brick<VT, 1, false, NZ>(map, P, b[0], b[1], b[2], 0, smem); break;
+    default: fwd_brick<VT, 1, true, NZ>(map, P, b[0], b[1], b[2], 0, smem); break;
+  }
 }
 
 template <typename VT>
@@ -528,14 +604,9 @@ fwd_batch_kernel(const FwdBatchDesc* __restrict__ descs, const long long* __rest
       sB[4] = D.lane_y * 2 + D.bz0;
     }
     __syncthreads();
-    switch (sB[4]) {
-      case 0: fwd_brick<VT, 0, false, 16>(sMap, sP, sB[0], sB[1], sB[2], 0, smem); break;  // z-dependent y-map
-      case 2: fwd_brick<VT, 1, false, 16>(sMap, sP, sB[0], sB[1], sB[2], 0, smem); break;
-      default:
-        if (sB[3] == 8) fwd_batch_item<VT, 8>(sMap, sP, sB, smem);
-        else if (sB[3] == 32) fwd_batch_item<VT, 32>(sMap, sP, sB, smem);
-        else fwd_batch_item<VT, 16>(sMap, sP, sB, smem);
-    }
+    if (sB[3] == 8) fwd_batch_item<VT, 8>(sMap, sP, sB, smem);
+    else if (sB[3] == 32) fwd_batch_item<VT, 32>(sMap, sP, sB, smem);
+    else fwd_batch_item<VT, 16>(sMap, sP, sB, smem);
   }
 }
 
@@ -589,7 +660,7 @@ FwdPlan plan_forward_uncached(const std::vector<double>& xc, const std::vector<d
   // lane: -1 heuristic (lines along X or Y), 0 lines along X, 1 along Y, 2 8x4 patches
   p.lanes = lane < 0 ? (sy > sx ? 1 : 0) : std::min(lane, 2);
   p.bz0 = bz0;
-  p.nz = bz0 ? nz : 16;  // Z-dependent y-maps use one depth
+  p.nz = nz;
   const int BX = p.lanes == 1 ? kWarps : 32, BY = p.lanes == 1 ? 32 : kWarps, BZ = p.nz;
   double ex = 0, ey = 0;
   for (int a = 0; a < A; ++a) {

@@ -201,7 +201,7 @@ struct FwdBatchDesc {
   VolDev vol;
   int WX, WY, mass_shift;
   int gx, gy;
-  int lane_y, bz0, nz;   // brick depth 8, 16 or 32 (16 when the y-map depends on z)
+  int lane_y, bz0, nz;   // brick depth 8, 16 or 32
   const void* x;         // volume read by the splat (float / bf16 / f16)
   const CUtensorMap* map;  // device address of the ray-sum tensor map
 };

@@ -111,7 +111,7 @@ std::string geometry_key(const AxisState& a, const VolDev& v, int precision) {
   }
   char buf[256];
   // the trailing tag names the timing method, so choices cached by an older one are not reused
-  std::snprintf(buf, sizeof(buf), "p%dx%dx%d_v%dx%dx%d_m%.2f,%.2f,%.2f,%.2f,%.2f,%.2f_z%d_prec%d_t8", a.PX, a.PY,
+  std::snprintf(buf, sizeof(buf), "p%dx%dx%d_v%dx%dx%d_m%.2f,%.2f,%.2f,%.2f,%.2f,%.2f_z%d_prec%d_t9", a.PX, a.PY,
                 a.A, v.NX, v.NY, v.NZ, m[0], m[1], m[2], m[3], m[4], m[5], bz0 ? 0 : 1, precision);
   return buf;
 }
@@ -286,7 +286,7 @@ bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, int precision, f
       for (int nz : kFwdDepths) {
         FwdPlan p = plan_forward(a.hxc, a.hyc, a.A, a.PX, a.PY, a.pitch, nz, lane);
         CUtensorMap m;
-        if (!p.ok || p.nz != nz || !encode_tensor_map_3d(&m, a.s.p, false, a.pitch, a.pitch, a.PY, a.A, p.WX, p.WY))
+        if (!p.ok || !encode_tensor_map_3d(&m, a.s.p, false, a.pitch, a.pitch, a.PY, a.A, p.WX, p.WY))
           continue;
         fps.push_back(p);
         fmaps.push_back(m);
