@@ -4,8 +4,8 @@
 // The reference adds every voxel's four bilinear weights into the projection
 // with global float atomics (FunctionOnGPU.cu:27-52, 316-333): eight atomics
 // per voxel and angle, contending along every ray.  Here one CTA owns a
-// brick of BX x BY x NZ voxels, held in registers for the whole launch.  For
-// each of its angles it splats the brick into a private detector window in
+// brick of BX x BY x NZ voxels for the whole launch (prefix sums in shared
+// memory, or voxels in registers where the y-map has a Z term).  For each of its angles it splats the brick into a private detector window in
 // shared memory, then one thread flushes the window into the ray-sum array
 // with a single 3-D tiled cp.reduce.async.bulk.tensor add (the L2 reduces
 // whole sectors).  Three window stages rotate: the flush of one angle
@@ -14,24 +14,19 @@
 //
 // Window accumulation is fixed point: shared-memory float atomicAdd is not a
 // single native operation on this part, integer adds are.  Each CTA scales
-// its voxels by a power of two S with S * max|v| < 2^b, b <= 21 - log2(depth),
-// so every added value (a tap, or a column's merged run of at most depth
-// voxels) rounds to an integer below 2^21 (rounded with the 1.5*2^23 trick,
-// no float->int conversion) with an absolute error of at most
-// 2^-(b+1) * max|v|.  The host bounds the weight one pixel can receive from
+// its values by a power of two S with S * max|v| < 2^b and b <= 21 - log2(weight
+// one pixel can receive from one column), so every added value rounds to an
+// integer below 2^21 (rounded with the 1.5*2^23 trick, no float->int
+// conversion) with an absolute error of at most 2^-(b+1) * max|v|.  The host bounds the weight one pixel can receive from
 // one brick by 2^mass_shift (lattice points in the preimage of a 2x2-pixel
 // square, times the brick depth) and b <= 30 - mass_shift keeps every window
 // sum below 2^30.  Before the flush the window is converted back to float and
 // divided by S (exact: S is a power of two).
 //
-// When the y-map has no Z term, a voxel column's y weights are common to the
-// column and its x advances by |a3| < 1 per voxel: the column walk merges
-// the column's 1-D splat in registers and adds one value per pixel it leaves
-// (2-16x fewer shared-memory adds than four per voxel, depending on the tilt),
-// in branch-free chunks where the slope allows, with red.shared adds on 32-bit
-// shared addresses; bricks at the detector edge check each add against the
-// window.  Where the y-map has a Z term the walk carries two rows.  The per-tap
-// path remains for slopes >= 0.999.
+// A voxel column is merged along its length before it is added: pixel by pixel
+// from prefix sums, or voxel by voxel in registers where the y-map has a Z term
+// (2-16x fewer shared-memory adds than four per voxel, depending on the tilt);
+// bricks at the detector edge check each add against the window.
 //
 // Windows are clamped inside the detector (TMA reduces must not start at a
 // negative coordinate), so a tap is on the detector iff it lies in the valid
@@ -66,8 +61,8 @@ struct FwdArgs {
   int groups;      // angle groups (grid.z = z-blocks * groups)
   int max_angles;  // angles per group (shared-memory constants sized for it)
   int mass_shift;  // log2 bound of one pixel's total weight from one brick
+  int nz;          // brick depth (voxels per column)
   const void* x;   // volume (nullptr: ones)
-  int* err;
 };
 
 __device__ __forceinline__ int magic_int(float integral) { return __float_as_int(__fadd_rn(integral, kMagic)); }
@@ -88,6 +83,31 @@ __device__ __forceinline__ void red_shared(uint32_t addr, int v) {
   asm volatile("red.shared.add.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
+// Ends an angle's splat into window stage `wi`: the fixed-point sums are
+// converted in place and reduced into the ray sums with one bulk reduce-add;
+// `next`, the stage of the following angle, is zeroed meanwhile (the bulk
+// reduce of angle j - 2, its last reader, must be done reading).
+__device__ __forceinline__ void flush_window(const CUtensorMap* smap, int* wi, int* next, int win_elems, float invS,
+                                             int j, bool more, int ox, int oy, int a) {
+  float* wf = reinterpret_cast<float*>(wi);
+  if (threadIdx.x == 0 && j >= 2) bulk_wait_read<1>();
+  __syncthreads();
+  // fixed point -> float (exact power-of-two scale), in place, 16 bytes a step
+  for (int i = threadIdx.x * 4; i < win_elems; i += kThreads * 4) {  // (WX is a multiple of 4)
+    const int4 q = *reinterpret_cast<const int4*>(wi + i);
+    *reinterpret_cast<float4*>(wf + i) =
+        make_float4((float)q.x * invS, (float)q.y * invS, (float)q.z * invS, (float)q.w * invS);
+    if (more) *reinterpret_cast<int4*>(next + i) = make_int4(0, 0, 0, 0);
+  }
+  fence_proxy_async_smem();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    tma_reduce_add_3d(smap, wf, ox, oy, a);
+    bulk_commit();
+  }
+}
+template <int N> struct Off { static constexpr int value = N; };
+
 template <typename VT> __device__ __forceinline__ float ldv(const void* p, long long i);
 template <> __device__ __forceinline__ float ldv<float>(const void* p, long long i) {
   return __ldg(static_cast<const float*>(p) + i);
@@ -99,131 +119,302 @@ template <> __device__ __forceinline__ float ldv<__half>(const void* p, long lon
   return __half2float(__ldg(static_cast<const __half*>(p) + i));
 }
 
-// Streaming splat of one voxel column (fixed X, Y; y-map without a Z term):
-// its detector y (rows and weights wy0 / wy1) is common to the column and
-// its detector x moves by |a3| < 1 per voxel, so consecutive voxels reach at
-// most one new pixel.  The column's 1-D splat is accumulated in registers and
-// a pixel is emitted (one integer add per detector row) only once the column
-// has left it.  ROW: the warp's lanes share their rows and weights, so the
-// unsplit values go into the warp's row buffer `row` (one add per pixel; the
-// warp splits the row afterwards), else into detector rows `row` and
-// `row + WX`.
+// Integer add with a constant byte offset.
+template <int OFF> __device__ __forceinline__ void red_shared_at(uint32_t addr, int v) {
+  asm volatile("red.shared.add.s32 [%0+%2], %1;" ::"r"(addr), "r"(v), "n"(OFF) : "memory");
+}
+
+// ---- y-maps without a Z term: pixel by pixel over prefix sums ----------------
 //
-// The walk always runs z upwards.  Where a3 < 0 it runs in the mirrored
-// coordinate u = -x, which grows by |a3| per voxel: a voxel at u with
-// fraction f splats (1 - f, f) onto mirrored pixels (p, p + 1), which are the
-// original pixels (-p, -p - 1) with the original splat's weights, so the
-// emissions go to window column (xi - ox) - p.  One code path serves both
-// slope signs (half the unrolled code of a walk per sign).
+// A thread owns one voxel column and splats it pixel by pixel, not voxel by
+// voxel.  Along the column the detector x is affine in z, so the voxels that
+// fall between two neighbouring pixels p and p + 1 are a run of z, and what
+// the run adds to the two pixels needs only its sums of v and of z v: two
+// differences of prefix sums, which the CTA forms once, before its angles, and
+// keeps in shared memory ([index][thread]: conflict-free whatever index each
+// lane reads).  With z_p the place where x reaches p,
+//     G = D1 - z_p D0,   part on p + 1: a3 G,   part on p: D0 - a3 G,
+// and a pixel is added to the window when its right neighbour's run ends:
+// E = D0 + a3 (G of the run before - G).  All lanes run in step (their pixel
+// counts differ by at most one), where a walk along the voxels diverges at
+// every pixel crossing.  A voxel that rounding puts on the wrong side of a
+// boundary is harmless: its weights run on linearly past it.
 //
-// L > 1 (slope below 1 / L): a chunk of L voxels crosses at most one pixel
-// boundary, so it accumulates without a branch and the column emits at most
-// once per chunk; branching per voxel made the warp run the emission on
-// almost every voxel (its lanes cross at different voxels).  S is the weight
-// not yet emitted (pixels p and p + 1), a1 its part on p + 1.  Inside a chunk
-// the fraction runs on past 1: a voxel beyond the crossing (fraction f in
-// [1, 2)) is first added as if it were not (1 - f on p, f on p + 1) and C
-// collects (f - 1) v, which moves it to its true pixels (2 - f on p + 1,
-// f - 1 on p + 2) when the chunk ends.
-//
-// CHK: the brick's window is clamped at the detector edge (or reaches past
-// it), so some of the column's pixels are off the detector: each emission
-// checks its window column against the valid columns (span = 4 * valid
-// columns, in bytes) and each detector row against the window (y0ok, y1ok),
-// and drops what falls outside, as the reference drops off-detector taps.
-template <int NZ, int L, bool ROW, bool CHK>
-__device__ __forceinline__ void stream_column(uint32_t row, int WX, const float (&v)[NZ], float xr, float a3, int lxm,
-                                              float wy0, float wy1, uint32_t span, bool y0ok, bool y1ok) {
-  const int dir = a3 >= 0.f ? 1 : -1;
-  const float u = a3 >= 0.f ? xr : -xr;
-  const float flu = floorf(u);
-  float fx = u - flu;
-  const float step = fabsf(a3);
-  // window column of pixel p: (xi - ox) + dir * p, with xi - ox = lxm + kMagicBits;
-  // `at` is the shared address of the current pixel, `dstep` the next pixel's offset
-  uint32_t at = row + 4u * (uint32_t)((lxm + kMagicBits) + dir * (magic_int(flu) - kMagicBits));
-  const uint32_t dstep = dir > 0 ? 4u : 0xFFFFFFFCu, drow = 4u * (uint32_t)WX;
-  auto emit = [&](uint32_t q, float e) {
-    if (ROW) {
-      red_shared(q, fixq(1.f, e));
-    } else if (CHK) {
-      const bool xok = q - row < span;  // (a column left of the window wraps to a large offset)
-      if (xok && y0ok) red_shared(q, fixq(wy0, e));
-      if (xok && y1ok) red_shared(q + drow, fixq(wy1, e));
+// Bound by shared-memory wavefronts (4.3 per 32 voxels and angle at depth 32:
+// 2.2 for the adds, which conflict 2.1 times whatever the window's pitch or
+// the lanes' layout, 1.1 for the prefix, the rest the window and constants)
+// with 14 instructions per voxel and angle, where the walk along the voxels was
+// bound by the issue of 22.  512x512x64 at 60 degrees, 61 angles: 0.675 against
+// 0.70 ms; 320x288x48, 45 angles: 0.16 against 0.21 ms; 512x512x128 read from
+// FP16: 1.34 against 1.49 ms.
+struct __align__(16) PreConst {  // per-angle constants of a brick
+  float xf, a1, a2, a3;   // (|a3| at least 1e-7: 2e-6 px over a column)
+  float yf, b1, b2, inv;  // inv = 1 / a3
+  int lxm, lym;           // window-local integer base minus the magic bits
+  int nx;                 // pixel boundaries that every column crosses: floor(|a3| (depth - 1))
+  float scale;            // fixed-point scale of this angle (power of two)
+  int ox, oy;             // window origin (clamped inside the detector, ox aligned)
+  int wlx;                // valid window columns; negative where every tap is valid (window not clamped)
+  float inv_scale;
+};
+constexpr uint32_t kPreStride = kThreads * 8u;  // bytes from one prefix index to the next
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 lds_pair(uint32_t a) {
+  f32x2 v;
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float2 sub2(f32x2 a, f32x2 b) {  // a - b in one packed instruction
+  f32x2 r;
+  float2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(b), "l"(0xBF800000BF800000ull), "l"(a));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(r));
+  return d;
+}
+
+// One column of depth nz at one angle: its prefix sums at `pre` (index i: sums
+// over voxels z < i of v and (z - nz / 2) v), detector rows at shared address
+// `row` and `row` + drow with weights wy0, wy1 (scaled).  CHK: the brick's
+// window is clamped at the detector edge (or reaches past it): each addition
+// checks its window column against the valid columns (span, in bytes) and each
+// detector row against the window, and drops what falls outside, as the
+// reference drops off-detector taps.
+template <bool CHK>
+__device__ __forceinline__ void splat_column(uint32_t pre, int nz, uint32_t row, uint32_t drow, float xr,
+                                             const PreConst& k, float wy0, float wy1, uint32_t span, bool y0ok,
+                                             bool y1ok) {
+  const bool asc = k.a3 >= 0.f;
+  const int c0 = nz >> 1;  // origin of the moments
+  const float lo = (float)-c0, hi = (float)(nz - c0);  // the column's ends, in centred z
+  const float xs = asc ? xr : fmaf(k.a3, (float)(nz - 1), xr);  // x of the first voxel met
+  const float fl = floorf(xs);
+  float zp = fmaf(fl - xr, k.inv, lo);  // where x reaches the current pixel
+  float tb = zp + k.inv;                // and the next one
+  const float ceil_at = kMagic + (float)c0;  // rounding up to an index, in the low bits
+  const uint32_t base = pre - (uint32_t)kMagicBits * kPreStride;
+  const uint32_t end = pre + (asc ? (uint32_t)nz * kPreStride : 0u);
+  f32x2 prev = 0ull;
+  if (!asc) {  // read backwards, the prefix gives the negated sums
+    prev = lds_pair(pre + (uint32_t)nz * kPreStride);
+    wy0 = -wy0;
+    wy1 = -wy1;
+  }
+  uint32_t at = row + 4u * (uint32_t)((k.lxm + kMagicBits) + (magic_int(fl) - kMagicBits)), at1 = at + drow;
+  float before = 0.f;  // G of the run before
+  auto index_at = [&](float t) { return base + __float_as_uint(__fadd_ru(t, ceil_at)) * kPreStride; };
+  auto add = [&](auto off, float e) {
+    constexpr int OFF = decltype(off)::value;
+    if (CHK) {
+      const bool xok = at + (uint32_t)OFF - row < span;  // (a column left of the window wraps to a large offset)
+      if (xok && y0ok) red_shared_at<OFF>(at, fixq(wy0, e));
+      if (xok && y1ok) red_shared_at<OFF>(at1, fixq(wy1, e));
     } else {
-      red_shared(q, fixq(wy0, e));
-      red_shared(q + drow, fixq(wy1, e));
+      red_shared_at<OFF>(at, fixq(wy0, e));
+      red_shared_at<OFF>(at1, fixq(wy1, e));
     }
   };
-  if constexpr (L == 1) {
-    float acc0 = (1.f - fx) * v[0], acc1 = fx * v[0];
+  auto run = [&](auto off, f32x2 s, float z) {  // the run from z (the current pixel's place) to prefix s
+    const float2 d = sub2(s, prev);
+    prev = s;
+    const float g = fmaf(-z, d.x, d.y);
+    add(off, fmaf(k.a3, before - g, d.x));
+    before = g;
+  };
+  // The boundaries that every column crosses lie inside it; four prefix loads
+  // are in flight at a time.
+  int n = k.nx;
+#pragma unroll 1
+  for (; n >= 4; n -= 4) {
+    const float t1 = tb + k.inv, t2 = fmaf(2.f, k.inv, tb), t3 = fmaf(3.f, k.inv, tb);
+    const f32x2 s0 = lds_pair(index_at(tb)), s1 = lds_pair(index_at(t1)), s2 = lds_pair(index_at(t2)),
+                s3 = lds_pair(index_at(t3));
+    run(Off<0>{}, s0, zp);
+    run(Off<4>{}, s1, tb);
+    run(Off<8>{}, s2, t1);
+    run(Off<12>{}, s3, t2);
+    zp = t3;
+    tb = fmaf(4.f, k.inv, tb);
+    at += 16u;
+    at1 += 16u;
+  }
+  if (n & 2) {
+    const float t1 = tb + k.inv;
+    const f32x2 s0 = lds_pair(index_at(tb)), s1 = lds_pair(index_at(t1));
+    run(Off<0>{}, s0, zp);
+    run(Off<4>{}, s1, tb);
+    zp = t1;
+    tb = t1 + k.inv;
+    at += 8u;
+    at1 += 8u;
+  }
+  if (n & 1) {
+    run(Off<0>{}, lds_pair(index_at(tb)), zp);
+    zp = tb;
+    tb += k.inv;
+    at += 4u;
+    at1 += 4u;
+  }
+  // Some columns cross one more; the next run ends the column, and where the
+  // one before ended it already, its pixel has only the carried part.
+  const uint32_t last = index_at(asc ? fminf(tb, hi) : fmaxf(tb, lo));
+  const f32x2 s0 = lds_pair(last), s1 = lds_pair(end);
+  run(Off<0>{}, s0, zp);
+  run(Off<4>{}, s1, tb);
+  if (last != end) add(Off<8>{}, k.a3 * before);
+}
+
+// One brick (bx, by, zb) and angle group g of one axis whose y-map has no Z
+// term; `smem` is the CTA's dynamic shared memory.  On return every bulk
+// reduce it issued is complete.
+template <typename VT>
+__device__ __forceinline__ void prefix_brick(const CUtensorMap* smap, const FwdArgs& P, int lanes, int bx, int by,
+                                             int zb, int g, unsigned char* smem) {
+  const int BX = forward_brick_x(lanes), BY = forward_brick_y(lanes), NZ = P.nz;
+  PreConst* kc = reinterpret_cast<PreConst*>(smem);
+  const size_t kc_bytes = ((size_t)P.max_angles * sizeof(PreConst) + 127) & ~(size_t)127;
+  const int WX = P.WX, WY = P.WY;
+  const int win_elems = WX * WY;
+  const size_t stage_bytes = ((size_t)win_elems * 4 + 127) & ~(size_t)127;
+  unsigned char* win0 = smem + kc_bytes + 128;
+  float* red = reinterpret_cast<float*>(smem + kc_bytes);  // 32 floats for the block max
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int A = P.ax.A;
+  const int a_begin = (int)((long long)A * g / P.groups), a_end = (int)((long long)A * (g + 1) / P.groups);
+  const int na = a_end - a_begin;
+  const int X0 = P.vol.Xs + bx * BX, Y0 = P.vol.Ys + by * BY, Z0 = P.z0 + zb * NZ;
+
+  // own column, read once (coalesced along lanes): prefix sums, and the brick's max |v|
+  const int tx = lanes == 0 ? lane : lanes == 1 ? warp : (warp & 1) * 8 + (lane & 7);
+  const int ty = lanes == 0 ? warp : lanes == 1 ? lane : (warp >> 1) * 4 + (lane >> 3);
+  const bool active = (X0 + tx < P.vol.Xs + P.vol.NX) && (Y0 + ty < P.vol.Ys + P.vol.NY);
+  float2* pre = reinterpret_cast<float2*>(win0 + kStages * stage_bytes) + tid;
+  float vmax = 0.f;
+  {
+    const long long sx = P.vol.NX, sxy = (long long)P.vol.NX * P.vol.NY;
+    const long long base = (long long)(X0 + tx - P.vol.Xs) + (long long)(Y0 + ty - P.vol.Ys) * sx;
+    const int c0 = NZ >> 1;
+    float s0 = 0.f, s1 = 0.f;
+    pre[0] = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int z8 = 0; z8 < NZ; z8 += 8) {  // eight loads in flight
+      float v[8];
 #pragma unroll
-    for (int z = 1; z < NZ; ++z) {
-      // the fraction is stepped (rounding < 4e-6 px over 32 voxels; the window
-      // keeps one pixel of slack past the last exact tap on either side)
-      fx += step;
-      if (fx >= 1.f) {  // the column left the pixel at `at`
-        fx -= 1.f;
-        emit(at, acc0);
-        acc0 = acc1;
-        acc1 = 0.f;
-        at += dstep;
+      for (int q = 0; q < 8; ++q) {
+        const int z = z8 + q;
+        v[q] = 0.f;
+        if (active && z < NZ && Z0 + z < P.z1)
+          v[q] = P.x ? ldv<VT>(P.x, base + (long long)(Z0 + z - P.z0) * sxy) : 1.f;
       }
-      acc0 = fmaf(1.f - fx, v[z], acc0);
-      acc1 = fmaf(fx, v[z], acc1);
-    }
-    emit(at, acc0);
-    emit(at + dstep, acc1);
-  } else {
-    float S = v[0], a1 = fx * v[0];
 #pragma unroll
-    for (int z0 = 1; z0 < NZ; z0 += L) {
-      float C = 0.f;
-#pragma unroll
-      for (int j = 0; j < L; ++j) {
-        if (z0 + j < NZ) {
-          fx += step;
-          S += v[z0 + j];
-          a1 = fmaf(fx, v[z0 + j], a1);
-          C = fmaf(__saturatef(fx - 1.f), v[z0 + j], C);  // f - 1 < 1: saturation is max(f - 1, 0)
+      for (int q = 0; q < 8; ++q) {
+        const int z = z8 + q;
+        if (z < NZ) {
+          vmax = fmaxf(vmax, fabsf(v[q]));
+          s0 += v[q];
+          s1 = fmaf((float)(z - c0), v[q], s1);
+          pre[(z + 1) * kThreads] = make_float2(s0, s1);
         }
       }
-      if (fx >= 1.f) {  // the chunk left the pixel at `at`
-        emit(at, (S - a1) + C);
-        S = a1 - C;
-        a1 = C;
-        fx -= 1.f;
-        at += dstep;
-      }
     }
-    emit(at, S - a1);
-    emit(at + dstep, a1);
   }
+  for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+  if (lane == 0) red[warp] = vmax;
+  zero_window(reinterpret_cast<int*>(win0), win_elems);  // the first angle's stage
+  if (tid == 0) prefetch_tensormap(smap);
+  __syncthreads();
+  vmax = red[0];
+  for (int w = 1; w < kWarps; ++w) vmax = fmaxf(vmax, red[w]);
+  int e2 = 0;
+  if (vmax > 0.f && isfinite(vmax)) frexpf(vmax, &e2);
+
+  for (int j = tid; j < na; j += kThreads) {
+    const int a = a_begin + j;
+    const double* cx = P.ax.xc + 4 * a;
+    const double* cy = P.ax.yc + 4 * a;
+    const double xb = cx[0] + cx[1] * X0 + cx[2] * Y0 + cx[3] * Z0 - 1.0;
+    const double yb = cy[0] + cy[1] * X0 + cy[2] * Y0 + cy[3] * Z0 - 1.0;
+    const double fxb = floor(fmin(fmax(xb, -1.0e9), 1.0e9)), fyb = floor(fmin(fmax(yb, -1.0e9), 1.0e9));
+    PreConst k;
+    k.xf = (float)(xb - fxb);
+    k.yf = (float)(yb - fyb);
+    k.a1 = (float)cx[1]; k.a2 = (float)cx[2];
+    const float st = fmaxf(fabsf((float)cx[3]), 1e-7f);
+    k.a3 = cx[3] >= 0.0 ? st : -st;
+    k.b1 = (float)cy[1]; k.b2 = (float)cy[2];
+    k.inv = 1.f / k.a3;
+    const int xi = (int)fxb, yi = (int)fyb;
+    const float xmin = k.xf + fminf(0.f, k.a1 * (BX - 1)) + fminf(0.f, k.a2 * (BY - 1)) + fminf(0.f, k.a3 * (NZ - 1));
+    const float ymin = k.yf + fminf(0.f, k.b1 * (BX - 1)) + fminf(0.f, k.b2 * (BY - 1));
+    const int ox0 = floor_div(xi + (int)floorf(xmin) - 1, 4) * 4;
+    const int oy0 = yi + (int)floorf(ymin) - 1;
+    // clamp inside [0, pitch - WX] x [0, PY - WY]; the host checked both ranges exist
+    k.ox = min(max(ox0, 0), P.ax.pitch - WX);
+    k.oy = min(max(oy0, 0), P.ax.PY - WY);
+    k.lxm = xi - k.ox - kMagicBits;
+    k.lym = yi - k.oy - kMagicBits;
+    // An unclamped window holds the whole footprint; inside the detector every tap is kept.
+    const bool interior = k.ox == ox0 && k.oy == oy0 && k.ox + WX <= P.ax.PX;
+    k.wlx = interior ? -1 : max(0, min(WX, P.ax.PX - k.ox));
+    k.nx = (int)(st * (float)(NZ - 1));
+    // S = 2^(b-e) with max |v| < 2^e, so |v S| < 2^b.  A pixel receives at most
+    // the weight w = min(depth, 1 + 1/slope) <= 2^lw from one column:
+    // |addition| < 2^(b + lw) <= 2^21, the range of the magic rounding.  A
+    // pixel's window sum stays below 2^(b + mass_shift) <= 2^30 (no overflow).
+    int lw = 0;
+    frexpf(fminf((float)NZ, 1.f + 1.f / st), &lw);
+    const int bits = min(21 - lw, 30 - P.mass_shift);
+    const int sexp = max(-120, min(120, bits - e2));
+    k.scale = ldexpf(1.f, sexp);
+    k.inv_scale = ldexpf(1.f, -sexp);
+    kc[j] = k;
+  }
+  __syncthreads();
+
+  // Three window stages as in fwd_brick.
+  const uint32_t pre_a = smem_u32(pre);
+#pragma unroll 1
+  for (int j = 0; j < na; ++j) {
+    const int st = j % kStages;
+    int* wi = reinterpret_cast<int*>(win0 + st * stage_bytes);
+    const PreConst k = kc[j];  // (a copy: the adds order memory)
+    if (active) {
+      const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
+      const float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
+      const float fly = floorf(yr);
+      const float fy = yr - fly;
+      const int rowi = magic_int(fly) + k.lym;
+      const uint32_t rowa = smem_u32(wi) + 4u * (uint32_t)(rowi * WX);
+      const float wy0 = (1.f - fy) * k.scale, wy1 = fy * k.scale;
+      if (k.wlx < 0)
+        splat_column<false>(pre_a, NZ, rowa, 4u * (uint32_t)WX, xr, k, wy0, wy1, 0u, true, true);
+      else
+        splat_column<true>(pre_a, NZ, rowa, 4u * (uint32_t)WX, xr, k, wy0, wy1, 4u * (uint32_t)k.wlx,
+                           (unsigned)rowi < (unsigned)WY, (unsigned)(rowi + 1) < (unsigned)WY);
+    }
+    flush_window(smap, wi, reinterpret_cast<int*>(win0 + ((j + 1) % kStages) * stage_bytes), win_elems, k.inv_scale, j,
+                 j + 1 < na, k.ox, k.oy, a_begin + j);
+  }
+  if (tid == 0) bulk_wait_all();
 }
 
-// stream_column with the longest chunk the slope allows (the bounds leave
-// room for the stepped fraction's rounding: a chunk's fraction stays below 2).
-template <int NZ, bool ROW, bool CHK>
-__device__ __forceinline__ void splat_column(uint32_t row, int WX, const float (&v)[NZ], float xr, float a3, int lxm,
-                                             float wy0, float wy1, uint32_t span = 0, bool y0ok = true,
-                                             bool y1ok = true) {
-  const float st = fabsf(a3);
-  if (st < 0.2499f) stream_column<NZ, 4, ROW, CHK>(row, WX, v, xr, a3, lxm, wy0, wy1, span, y0ok, y1ok);
-  else if (st < 0.4999f) stream_column<NZ, 2, ROW, CHK>(row, WX, v, xr, a3, lxm, wy0, wy1, span, y0ok, y1ok);
-  else stream_column<NZ, 1, ROW, CHK>(row, WX, v, xr, a3, lxm, wy0, wy1, span, y0ok, y1ok);
-}
-
-// The same for a y-map with a Z term: the column also moves by |b3| < 1 per
-// voxel through the detector rows (mirrored where b3 < 0, as x is where a3 <
-// 0), so four sums are carried: the weight not yet emitted of the current row
-// and the next (S0, S1), and its parts on the next pixel (X0, X1).  At a pixel
+// ---- y-maps with a Z term: voxel by voxel ---------------------------------------
+//
+// Streaming splat of one voxel column (fixed X, Y), held in registers: its
+// detector x moves by |a3| < 1 and its y by |b3| < 1 per voxel, so consecutive
+// voxels reach at most one new pixel and one new row.  The walk always runs z
+// upwards; where a3 < 0 it runs in the mirrored coordinate u = -x, which grows
+// by |a3| per voxel (a voxel at u with fraction f splats (1 - f, f) onto
+// mirrored pixels (p, p + 1), which are the original pixels (-p, -p - 1) with
+// the original weights), and likewise in y.  Four sums are carried: the weight
+// not yet emitted of the current row and the next (S0, S1), and its parts on
+// the next pixel (X0, X1).  At a pixel
 // crossing one pixel is emitted in both rows; at a row crossing the two pixels
 // of the row left are, and the next row's sums move down.  Two shared-memory
 // adds per pixel and two per row crossed, against four per voxel tap by tap:
 // 320x300x72 voxels, 51 angles, rows crossed every ~100 voxels, 0.55 ms
 // against 0.72 ms (bound by issue: 40 instructions per voxel and angle, half
 // of them in the crossings that some lane of a warp takes at almost every voxel).
-// CHK as in stream_column.
+// CHK as in splat_column.
 template <int NZ, bool CHK>
 __device__ __forceinline__ void stream_column_zy(uint32_t win, int WX, int WY, const float (&v)[NZ], float xr,
                                                  float yr, const FwdConst& k) {
@@ -286,11 +477,10 @@ __device__ __forceinline__ void stream_column_zy(uint32_t win, int WX, int WY, c
 
 // One brick (bx, by, zb) and angle group g of one axis; `smem` is the CTA's
 // dynamic shared memory.  On return every bulk reduce it issued is complete.
-template <typename VT, int LANES, bool BZ0, int NZ>
-__device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs& P, int bx, int by, int zb, int g,
+template <typename VT, int NZ>
+__device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs& P, int lanes, int bx, int by, int zb, int g,
                                           unsigned char* smem) {
-  constexpr int BX = LANES == 1 ? kWarps : 32;
-  constexpr int BY = LANES == 1 ? 32 : kWarps;
+  const int BX = forward_brick_x(lanes), BY = forward_brick_y(lanes);
   FwdConst* kc = reinterpret_cast<FwdConst*>(smem);
   const size_t kc_bytes = ((size_t)P.max_angles * sizeof(FwdConst) + 127) & ~(size_t)127;
   const int WX = P.WX, WY = P.WY;
@@ -298,9 +488,6 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
   const size_t stage_bytes = ((size_t)win_elems * 4 + 127) & ~(size_t)127;
   unsigned char* win0 = smem + kc_bytes + 128;
   float* red = reinterpret_cast<float*>(smem + kc_bytes);  // 32 floats for the block max
-  // per-warp row buffers of the uniform-row angles (kept zero between uses)
-  int* urow = reinterpret_cast<int*>(win0 + kStages * stage_bytes) + (threadIdx.x >> 5) * WX;
-  for (int i = threadIdx.x & 31; i < WX; i += 32) urow[i] = 0;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int A = P.ax.A;
@@ -342,9 +529,9 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
   }
 
   // own voxels, loaded once (coalesced along lanes), and the brick's max |v|
-  // LANES: 0 each warp a line along X, 1 a line along Y, 2 an 8x4 patch
-  const int tx = LANES == 0 ? lane : LANES == 1 ? warp : (warp & 3) * 8 + (lane & 7);
-  const int ty = LANES == 0 ? warp : LANES == 1 ? lane : (warp >> 2) * 4 + (lane >> 3);
+  // lanes: 0 each warp a line along X, 1 a line along Y, 2 an 8x4 patch
+  const int tx = lanes == 0 ? lane : lanes == 1 ? warp : (warp & 1) * 8 + (lane & 7);
+  const int ty = lanes == 0 ? warp : lanes == 1 ? lane : (warp >> 1) * 4 + (lane >> 3);
   const bool active = (X0 + tx < P.vol.Xs + P.vol.NX) && (Y0 + ty < P.vol.Ys + P.vol.NY);
   float v[NZ];
   float vmax = 0.f;
@@ -387,67 +574,8 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
     const int a = a_begin + j;
     const int st = j % kStages;
     int* wi = reinterpret_cast<int*>(win0 + st * stage_bytes);
-    float* wf = reinterpret_cast<float*>(wi);
     const FwdConst k = kc[j];
-    // Uniform rows: the detector y does not move along the lanes (|slope| * 31
-    // below 1e-6 px), so the lanes of a warp share their two rows and weights.
-    if (BZ0 && LANES != 2 && k.interior && fabsf(k.a3) < 0.999f && fabsf(LANES == 1 ? k.b2 : k.b1) < 3e-8f) {
-      const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
-      const float yr = __shfl_sync(0xffffffffu, fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf)), 0);
-      if (active) splat_column<NZ, true, false>(smem_u32(urow), WX, v, xr, k.a3, k.lxm, 1.f, 0.f);
-      __syncwarp();
-      // split the warp's row into the two detector rows (values up to 2^30:
-      // rounded with a conversion, the magic-number rounding needs < 2^22)
-      const float fly = floorf(yr);
-      const float fy = yr - fly;
-      int* rowp = wi + (magic_int(fly) + k.lym) * WX;
-      for (int i = lane; i < WX; i += 32) {
-        const int q = urow[i];
-        if (q != 0) {
-          const float uf = (float)q;
-          red_shared(smem_u32(rowp + i), __float2int_rn((1.f - fy) * uf));
-          red_shared(smem_u32(rowp + WX + i), __float2int_rn(fy * uf));
-          urow[i] = 0;
-        }
-      }
-    } else if (active && BZ0 && fabsf(k.a3) < 0.999f) {
-      // stream the column; at an interior window every tap lands in the
-      // window and on the detector, elsewhere each emission is checked
-      const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
-      const float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
-      const float fly = floorf(yr);
-      const float fy = yr - fly;
-      const int rowi = magic_int(fly) + k.lym;
-      const uint32_t rowa = smem_u32(wi) + 4u * (uint32_t)(rowi * WX);
-      if (k.interior)
-        splat_column<NZ, false, false>(rowa, WX, v, xr, k.a3, k.lxm, 1.f - fy, fy);
-      else
-        splat_column<NZ, false, true>(rowa, WX, v, xr, k.a3, k.lxm, 1.f - fy, fy, 4u * (uint32_t)k.wlx,
-                                      (unsigned)rowi < (unsigned)WY, (unsigned)(rowi + 1) < (unsigned)WY);
-    } else if (active && BZ0 && k.interior) {
-      // every tap lands in the window and on the detector: no per-tap tests
-      const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
-      const float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
-      const float fly = floorf(yr);
-      const float fy = yr - fly;
-      const int rowi = magic_int(fly) + k.lym;
-      const float wy0 = 1.f - fy, wy1 = fy;
-      int* rowp = wi + rowi * WX;
-#pragma unroll
-      for (int z = 0; z < NZ; ++z) {
-        const float x = fmaf(k.a3, (float)z, xr);
-        const float flx = floorf(x);
-        const float fx = x - flx;
-        int* r0 = rowp + (magic_int(flx) + k.lxm);
-        const float g0 = wy0 * v[z], g1 = wy1 * v[z];
-        const float wx0 = 1.f - fx;
-        const uint32_t a0 = smem_u32(r0), a1 = a0 + 4u * (uint32_t)WX;
-        red_shared(a0, fixq(wx0, g0));
-        red_shared(a0 + 4u, fixq(fx, g0));
-        red_shared(a1, fixq(wx0, g1));
-        red_shared(a1 + 4u, fixq(fx, g1));
-      }
-    } else if (active && !BZ0 && fabsf(k.a3) < 0.999f && fabsf(k.b3) < 0.999f) {
+    if (active && fabsf(k.a3) < 0.999f && fabsf(k.b3) < 0.999f) {
       const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
       const float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
       if (k.interior) stream_column_zy<NZ, false>(smem_u32(wi), WX, WY, v, xr, yr, k);
@@ -455,30 +583,15 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
     } else if (active) {
       const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
       const float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
-      float wy0 = 0.f, wy1 = 0.f;
-      int rowi = 0;
-      bool y0ok = false, y1ok = false;
-      if (BZ0) {
-        const float fly = floorf(yr);
-        const float fy = yr - fly;
-        rowi = magic_int(fly) + k.lym;
-        wy0 = 1.f - fy;
-        wy1 = fy;
-        y0ok = (unsigned)rowi < (unsigned)WY;
-        y1ok = (unsigned)(rowi + 1) < (unsigned)WY;
-      }
 #pragma unroll
       for (int z = 0; z < NZ; ++z) {
-        if (!BZ0) {
-          const float y = fmaf(k.b3, (float)z, yr);
-          const float fly = floorf(y);
-          const float fy = y - fly;
-          rowi = magic_int(fly) + k.lym;
-          wy0 = 1.f - fy;
-          wy1 = fy;
-          y0ok = (unsigned)rowi < (unsigned)WY;
-          y1ok = (unsigned)(rowi + 1) < (unsigned)WY;
-        }
+        const float y = fmaf(k.b3, (float)z, yr);
+        const float fly = floorf(y);
+        const float fy = y - fly;
+        const int rowi = magic_int(fly) + k.lym;
+        const float wy0 = 1.f - fy, wy1 = fy;
+        const bool y0ok = (unsigned)rowi < (unsigned)WY;
+        const bool y1ok = (unsigned)(rowi + 1) < (unsigned)WY;
         const float x = fmaf(k.a3, (float)z, xr);
         const float flx = floorf(x);
         const float fx = x - flx;
@@ -498,71 +611,54 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
         }
       }
     }
-    // the bulk reduce of angle j - 2 (the next stage's last reader) must be done reading
-    if (tid == 0 && j >= 2) bulk_wait_read<1>();
-    __syncthreads();
-    // fixed point -> float (exact power-of-two scale), in place, 16 bytes a step
-    for (int i = tid * 4; i < win_elems; i += kThreads * 4) {
-      if (i + 3 < win_elems) {
-        const int4 q = *reinterpret_cast<const int4*>(wi + i);
-        *reinterpret_cast<float4*>(wf + i) =
-            make_float4((float)q.x * invS, (float)q.y * invS, (float)q.z * invS, (float)q.w * invS);
-      } else {
-        for (int e = i; e < win_elems; ++e) wf[e] = (float)wi[e] * invS;
-      }
-    }
-    if (j + 1 < na) zero_window(reinterpret_cast<int*>(win0 + ((j + 1) % kStages) * stage_bytes), win_elems);
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      tma_reduce_add_3d(smap, wf, k.ox, k.oy, a);
-      bulk_commit();
-    }
+    flush_window(smap, wi, reinterpret_cast<int*>(win0 + ((j + 1) % kStages) * stage_bytes), win_elems, invS, j,
+                 j + 1 < na, k.ox, k.oy, a);
   }
   if (tid == 0) bulk_wait_all();
 }
 
-// One CTA per (brick, angle group) of one axis.
-template <typename VT, int LANES, bool BZ0, int NZ>
+// One CTA per (brick, angle group) of one axis.  NZ: the depth of the voxel
+// walk (z-dependent y-maps), or 0 for the prefix sums, whose depth is P.nz.
+template <typename VT, int NZ>
 __global__ void __launch_bounds__(kThreads)
-fwd_tma_kernel(const __grid_constant__ CUtensorMap smap, const FwdArgs P) {
+fwd_tma_kernel(const __grid_constant__ CUtensorMap smap, const __grid_constant__ FwdArgs P, int lanes) {
   extern __shared__ __align__(128) unsigned char smem[];
-  fwd_brick<VT, LANES, BZ0, NZ>(&smap, P, blockIdx.x, blockIdx.y, blockIdx.z / P.groups, blockIdx.z % P.groups,
-                                 smem);
+  if constexpr (NZ == 0)
+    prefix_brick<VT>(&smap, P, lanes, blockIdx.x, blockIdx.y, blockIdx.z / P.groups, blockIdx.z % P.groups, smem);
+  else
+    fwd_brick<VT, NZ>(&smap, P, lanes, blockIdx.x, blockIdx.y, blockIdx.z / P.groups, blockIdx.z % P.groups, smem);
 }
 
-template <typename VT, int LY, bool BZ, int NZ>
-cudaError_t launch_one(const CUtensorMap& map, FwdArgs P, size_t smem, int num_sms, cudaStream_t st) {
-  auto kern = fwd_tma_kernel<VT, LY, BZ, NZ>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  const int BX = LY == 1 ? kWarps : 32, BY = LY == 1 ? 32 : kWarps;
-  const long long bricks = (long long)((P.vol.NX + BX - 1) / BX) * ((P.vol.NY + BY - 1) / BY) *
-                           ((P.z1 - P.z0 + NZ - 1) / NZ);
+// Dynamic shared memory: per-angle constants, block-max scratch, window stages
+// and, where the y-map has no Z term, the columns' prefix sums.
+size_t fwd_smem(int WX, int WY, int nz, bool bz0, int angles) {
+  const size_t stage = (((size_t)WX * WY * 4) + 127) & ~(size_t)127;
+  const size_t k = (size_t)angles * (bz0 ? sizeof(PreConst) : sizeof(FwdConst));
+  return ((k + 127) & ~(size_t)127) + 128 + kStages * stage + (bz0 ? (size_t)(nz + 1) * kPreStride : 0);
+}
+
+template <typename VT, int NZ>
+cudaError_t launch_one(const CUtensorMap& map, FwdArgs P, int lanes, int num_sms, cudaStream_t st) {
+  auto kern = fwd_tma_kernel<VT, NZ>;
+  const int BX = forward_brick_x(lanes), BY = forward_brick_y(lanes);
+  const dim3 b3((P.vol.NX + BX - 1) / BX, (P.vol.NY + BY - 1) / BY, (P.z1 - P.z0 + P.nz - 1) / P.nz);
+  const long long bricks = (long long)b3.x * b3.y * b3.z;
   // split the angles over several CTAs when there are too few bricks to fill the GPU
   const long long target = (long long)num_sms * 8;
   int groups = (int)std::min<long long>((target + bricks - 1) / bricks, (long long)P.ax.A);
   if (groups < 1) groups = 1;
   P.groups = groups;
   P.max_angles = (P.ax.A + groups - 1) / groups;
-  const dim3 grid((P.vol.NX + BX - 1) / BX, (P.vol.NY + BY - 1) / BY, ((P.z1 - P.z0 + NZ - 1) / NZ) * groups);
-  kern<<<grid, kThreads, smem, st>>>(map, P);
+  const size_t smem = fwd_smem(P.WX, P.WY, P.nz, NZ == 0, P.max_angles);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  kern<<<dim3(b3.x, b3.y, b3.z * groups), kThreads, smem, st>>>(map, P, lanes);
   const cudaError_t le = cudaGetLastError();
   if (le == cudaSuccess) g_windowed_launches.fetch_add(1, std::memory_order_relaxed);
   return le;
 }
 
-template <typename VT, int LY, bool BZ>
-cudaError_t launch_nz(const CUtensorMap& map, const FwdArgs& P, const FwdPlan& plan, int sms, cudaStream_t st) {
-  if (plan.nz == 16) return launch_one<VT, LY, BZ, 16>(map, P, plan.smem, sms, st);
-  if (plan.nz == 8) return launch_one<VT, LY, BZ, 8>(map, P, plan.smem, sms, st);
-  if (plan.nz == 32) return launch_one<VT, LY, BZ, 32>(map, P, plan.smem, sms, st);
-  return cudaErrorInvalidValue;
-}
-
 }  // namespace
-
-const int kFwdDepths[3] = {8, 16, 32};
 
 namespace {
 
@@ -570,17 +666,6 @@ namespace {
 // brick): each CTA takes items blockIdx.x, blockIdx.x + gridDim.x, ...; every
 // brick ends with its bulk reduces complete, so the next one reuses the
 // shared-memory windows after a barrier.
-template <typename VT, int NZ>
-__device__ __forceinline__ void fwd_batch_item(const CUtensorMap* map, const FwdArgs& P, const int* b,
-                                               unsigned char* smem) {
-  switch (b[4]) {
-    case 0: fwd_brick<VT, 0, false, NZ>(map, P, b[0], b[1], b[2], 0, smem); break;  // z-dependent y-map
-    case 1: fwd_brick<VT, 0, true, NZ>(map, P, b[0], b[1], b[2], 0, smem); break;
-    case 2: fwd_brick<VT, 1, false, NZ>(map, P, b[0], b[1], b[2], 0, smem); break;
-    default: fwd_brick<VT, 1, true, NZ>(map, P, b[0], b[1], b[2], 0, smem); break;
-  }
-}
-
 template <typename VT>
 __global__ void __launch_bounds__(kThreads)
 fwd_batch_kernel(const FwdBatchDesc* __restrict__ descs, const long long* __restrict__ first, int n_desc,
@@ -589,24 +674,25 @@ fwd_batch_kernel(const FwdBatchDesc* __restrict__ descs, const long long* __rest
   // The item's arguments are staged in shared memory (no registers held).
   __shared__ FwdArgs sP;
   __shared__ const CUtensorMap* sMap;
-  __shared__ int sB[5];  // brick x, y, z, depth, lane_y * 2 + bz0
+  __shared__ int sB[5];  // brick x, y, z, depth, lanes * 2 + bz0
   for (long long it = blockIdx.x; it < n_items; it += gridDim.x) {
     __syncthreads();
     if (threadIdx.x == 0) {
       const int2 item = work_item(first, n_desc, it);
       const FwdBatchDesc& D = descs[item.x];
-      sP = FwdArgs{D.ax, D.vol, D.vol.Zs, D.vol.Zs + D.vol.NZ, D.WX, D.WY, 1, D.ax.A, D.mass_shift, D.x, nullptr};
+      sP = FwdArgs{D.ax, D.vol, D.vol.Zs, D.vol.Zs + D.vol.NZ, D.WX, D.WY, 1, D.ax.A, D.mass_shift, D.nz, D.x};
       sMap = D.map;
       sB[0] = item.y % D.gx;
       sB[1] = (item.y / D.gx) % D.gy;
       sB[2] = item.y / (D.gx * D.gy);
       sB[3] = D.nz;
-      sB[4] = D.lane_y * 2 + D.bz0;
+      sB[4] = D.lanes * 2 + D.bz0;
     }
     __syncthreads();
-    if (sB[3] == 8) fwd_batch_item<VT, 8>(sMap, sP, sB, smem);
-    else if (sB[3] == 32) fwd_batch_item<VT, 32>(sMap, sP, sB, smem);
-    else fwd_batch_item<VT, 16>(sMap, sP, sB, smem);
+    if (sB[4] & 1) prefix_brick<VT>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
+    else if (sB[3] == 8) fwd_brick<VT, 8>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
+    else if (sB[3] == 32) fwd_brick<VT, 32>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
+    else fwd_brick<VT, 16>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
   }
 }
 
@@ -661,7 +747,7 @@ FwdPlan plan_forward_uncached(const std::vector<double>& xc, const std::vector<d
   p.lanes = lane < 0 ? (sy > sx ? 1 : 0) : std::min(lane, 2);
   p.bz0 = bz0;
   p.nz = nz;
-  const int BX = p.lanes == 1 ? kWarps : 32, BY = p.lanes == 1 ? 32 : kWarps, BZ = p.nz;
+  const int BX = forward_brick_x(p.lanes), BY = forward_brick_y(p.lanes), BZ = p.nz;
   double ex = 0, ey = 0;
   for (int a = 0; a < A; ++a) {
     ex = std::max(ex, std::fabs(xc[4 * a + 1]) * (BX - 1) + std::fabs(xc[4 * a + 2]) * (BY - 1) +
@@ -671,13 +757,7 @@ FwdPlan plan_forward_uncached(const std::vector<double>& xc, const std::vector<d
   }
   const int wx_min = ((int)std::ceil(ex) + 4 + 4 + 3) / 4 * 4;
   p.WY = (int)std::ceil(ey) + 4;
-  auto smem_for = [&](int WX) {
-    const size_t stage = (((size_t)WX * p.WY * 4) + 127) & ~(size_t)127;
-    // constants for up to A angles (one group) + block-max scratch + window
-    // stages + per-warp row buffers of the uniform-row angles
-    return ((((size_t)A * sizeof(FwdConst)) + 127) & ~(size_t)127) + 128 + kStages * stage +
-           (size_t)kWarps * WX * sizeof(int);
-  };
+  auto smem_for = [&](int WX) { return fwd_smem(WX, p.WY, p.nz, bz0, A); };  // (one angle group)
   // Row pitch (= box width) with the fewest shared-memory bank conflicts of
   // the warp's splat atomics, searched over a few widths only: a wider window
   // leaves the interior fast path at more bricks near the detector edge.
@@ -707,7 +787,7 @@ FwdPlan plan_forward_uncached(const std::vector<double>& xc, const std::vector<d
   }
   p.mass_shift = (int)std::ceil(std::log2(std::max(1.0, count * BZ)));
   p.ok = !singular && p.mass_shift <= 16 && p.WX <= 256 && p.WY <= 256 && p.WX <= pitch && p.WY <= PY &&
-         p.smem <= 200 * 1024 && (p.nz == 8 || p.nz == 16 || p.nz == 32);
+         p.smem <= 227 * 1024 && (bz0 ? p.nz >= 1 && p.nz <= 32 : p.nz == 8 || p.nz == 16 || p.nz == 32);
   (void)PX;
   return p;
 }
@@ -724,22 +804,20 @@ FwdPlan plan_forward(const std::vector<double>& xc, const std::vector<double>& y
 
 template <typename VT>
 cudaError_t launch_forward_tma(const CUtensorMap& smap, const FwdPlan& plan, const AxisDev& ax, const VolDev& vol,
-                               const VT* x, int z0, int z1, int* err, cudaStream_t st) {
+                               const VT* x, int z0, int z1, cudaStream_t st) {
   const int sms = device_sm_count();
-  FwdArgs P{ax, vol, z0, z1, plan.WX, plan.WY, 1, ax.A, plan.mass_shift, x, err};
-  if (plan.lanes == 2) return plan.bz0 ? launch_nz<VT, 2, true>(smap, P, plan, sms, st)
-                                       : launch_nz<VT, 2, false>(smap, P, plan, sms, st);
-  if (plan.lanes == 1) return plan.bz0 ? launch_nz<VT, 1, true>(smap, P, plan, sms, st)
-                                       : launch_nz<VT, 1, false>(smap, P, plan, sms, st);
-  return plan.bz0 ? launch_nz<VT, 0, true>(smap, P, plan, sms, st) : launch_nz<VT, 0, false>(smap, P, plan, sms, st);
+  const FwdArgs P{ax, vol, z0, z1, plan.WX, plan.WY, 1, ax.A, plan.mass_shift, plan.nz, x};
+  if (plan.bz0) return launch_one<VT, 0>(smap, P, plan.lanes, sms, st);
+  if (plan.nz == 8) return launch_one<VT, 8>(smap, P, plan.lanes, sms, st);
+  if (plan.nz == 32) return launch_one<VT, 32>(smap, P, plan.lanes, sms, st);
+  return launch_one<VT, 16>(smap, P, plan.lanes, sms, st);
 }
 
 template cudaError_t launch_forward_tma<float>(const CUtensorMap&, const FwdPlan&, const AxisDev&, const VolDev&,
-                                               const float*, int, int, int*, cudaStream_t);
+                                               const float*, int, int, cudaStream_t);
 template cudaError_t launch_forward_tma<__nv_bfloat16>(const CUtensorMap&, const FwdPlan&, const AxisDev&,
-                                                       const VolDev&, const __nv_bfloat16*, int, int, int*,
-                                                       cudaStream_t);
+                                                       const VolDev&, const __nv_bfloat16*, int, int, cudaStream_t);
 template cudaError_t launch_forward_tma<__half>(const CUtensorMap&, const FwdPlan&, const AxisDev&, const VolDev&,
-                                                const __half*, int, int, int*, cudaStream_t);
+                                                const __half*, int, int, cudaStream_t);
 
 }  // namespace mtr

@@ -170,15 +170,23 @@ struct FwdPlan {
   bool bz0 = false;
   int WX = 0, WY = 0;
   int mass_shift = 0;  // log2 bound of a pixel's weight from one brick
-  int nz = 16;         // brick depth: 8, 16 or 32
+  int nz = 16;         // brick depth: 8, 16 or 32; up to 32 where the y-map has no Z term
   size_t smem = 0;
 };
-extern const int kFwdDepths[3];  // candidate brick depths of the forward splat
+// Brick of 256 columns: lines along X (32x8) or Y (8x32), or 8x4 patches in a
+// 16x16 square, whose footprint on an oblique axis is the smallest.
+#ifdef __CUDACC__
+#define MTR_HD __host__ __device__
+#else
+#define MTR_HD
+#endif
+MTR_HD constexpr int forward_brick_x(int lanes) { return lanes == 0 ? 32 : lanes == 1 ? 8 : 16; }
+MTR_HD constexpr int forward_brick_y(int lanes) { return lanes == 0 ? 8 : lanes == 1 ? 32 : 16; }
 FwdPlan plan_forward(const std::vector<double>& xc, const std::vector<double>& yc, int A, int PX, int PY, int pitch,
                      int nz, int lane = -1);
 template <typename VT>
 cudaError_t launch_forward_tma(const CUtensorMap& smap, const FwdPlan& plan, const AxisDev& ax, const VolDev& vol,
-                               const VT* x, int z0, int z1, int* err, cudaStream_t st);
+                               const VT* x, int z0, int z1, cudaStream_t st);
 
 // ---- persistent batched launches over many axes (batch.cu) -----------------
 // One descriptor per (instance, axis); one work item per brick, (descriptor,
@@ -201,7 +209,7 @@ struct FwdBatchDesc {
   VolDev vol;
   int WX, WY, mass_shift;
   int gx, gy;
-  int lane_y, bz0, nz;   // brick depth 8, 16 or 32
+  int lanes, bz0, nz;    // warp layout, z-independent y-map, brick depth
   const void* x;         // volume read by the splat (float / bf16 / f16)
   const CUtensorMap* map;  // device address of the ray-sum tensor map
 };

@@ -150,7 +150,7 @@ mtr_status enqueue_geometry(mtr_recon* r) {
     }
     if (a.ftma) {
       cudaError_t e = launch_forward_tma<float>(a.map_cf, a.fplan, a.dev(), v, nullptr, v.Zs, v.Zs + v.NZ,
-                                                r->err.as<int>(), ctx->stream);
+                                                ctx->stream);
       g_launches.fetch_add(1);
       if (e != cudaSuccess) return cuda_error(ctx, e, "forward row sums (tma)");
       continue;
@@ -189,11 +189,10 @@ mtr_status enqueue_forward(mtr_recon* r, AxisState& a, const VolSpan& sp) {
     switch (copy_kind_of(r->p.precision)) {
       case 1: e = launch_forward_tma<__nv_bfloat16>(a.map_s, a.fplan, a.dev(), v,
                                                      static_cast<const __nv_bfloat16*>(sp.xcopy), z0, z1,
-                                                     r->err.as<int>(), ctx->stream); break;
+                                                     ctx->stream); break;
       case 2: e = launch_forward_tma<__half>(a.map_s, a.fplan, a.dev(), v, static_cast<const __half*>(sp.xcopy), z0,
-                                              z1, r->err.as<int>(), ctx->stream); break;
-      default: e = launch_forward_tma<float>(a.map_s, a.fplan, a.dev(), v, sp.x, z0, z1, r->err.as<int>(),
-                                              ctx->stream); break;
+                                              z1, ctx->stream); break;
+      default: e = launch_forward_tma<float>(a.map_s, a.fplan, a.dev(), v, sp.x, z0, z1, ctx->stream); break;
     }
     g_launches.fetch_add(1);
     if (e != cudaSuccess) return cuda_error(ctx, e, "forward splat (tma)");

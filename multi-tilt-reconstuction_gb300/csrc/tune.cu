@@ -111,7 +111,7 @@ std::string geometry_key(const AxisState& a, const VolDev& v, int precision) {
   }
   char buf[256];
   // the trailing tag names the timing method, so choices cached by an older one are not reused
-  std::snprintf(buf, sizeof(buf), "p%dx%dx%d_v%dx%dx%d_m%.2f,%.2f,%.2f,%.2f,%.2f,%.2f_z%d_prec%d_t9", a.PX, a.PY,
+  std::snprintf(buf, sizeof(buf), "p%dx%dx%d_v%dx%dx%d_m%.2f,%.2f,%.2f,%.2f,%.2f,%.2f_z%d_prec%d_t10", a.PX, a.PY,
                 a.A, v.NX, v.NY, v.NZ, m[0], m[1], m[2], m[3], m[4], m[5], bz0 ? 0 : 1, precision);
   return buf;
 }
@@ -283,7 +283,7 @@ bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, int precision, f
     fps.reserve(9);
     fmaps.reserve(9);
     for (int lane = 0; lane < 3; ++lane)
-      for (int nz : kFwdDepths) {
+      for (int nz : {8, 16, 32}) {
         FwdPlan p = plan_forward(a.hxc, a.hyc, a.A, a.PX, a.PY, a.pitch, nz, lane);
         CUtensorMap m;
         if (!p.ok || !encode_tensor_map_3d(&m, a.s.p, false, a.pitch, a.pitch, a.PY, a.A, p.WX, p.WY))
@@ -295,12 +295,12 @@ bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, int precision, f
         cands.push_back([=, &a, &tv] {
           if (copy_kind == 1)
             return launch_forward_tma<__nv_bfloat16>(*mp, *pp, a.dev(), tv,
-                                                     static_cast<const __nv_bfloat16*>(scratch_copy), z0, z1, err,
+                                                     static_cast<const __nv_bfloat16*>(scratch_copy), z0, z1,
                                                      ctx->stream);
           if (copy_kind == 2)
             return launch_forward_tma<__half>(*mp, *pp, a.dev(), tv, static_cast<const __half*>(scratch_copy), z0, z1,
-                                              err, ctx->stream);
-          return launch_forward_tma<float>(*mp, *pp, a.dev(), tv, scratch_vol, z0, z1, err, ctx->stream);
+                                              ctx->stream);
+          return launch_forward_tma<float>(*mp, *pp, a.dev(), tv, scratch_vol, z0, z1, ctx->stream);
         });
         Choice c;
         c.fwd_nz = nz;
