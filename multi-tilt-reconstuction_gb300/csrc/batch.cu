@@ -5,7 +5,7 @@
 // launch whose CTAs (a grid sized to the GPU's resident capacity) take the
 // items of a work list covering the small axes of every instance:
 //   forward splat   item = (axis, brick)            fwd_batch_kernel
-//   residual        item = (axis, 64 Ki pixels)     residual_batch_kernel
+//   residual        item = (axis, 64 strips)        residual_batch_kernel
 //   back-projection item = (axis, brick)            bp_batch_kernel
 //   MACE consensus  item = (instance, 64 Ki voxels) mace_batch_kernel
 // so small instances no longer leave SMs idle.  An axis on line kernels, one with
@@ -96,8 +96,8 @@ mtr_status mtr::build_sirt_tables(mtr_context* ctx, const std::vector<mtr_recon*
       const FwdPlan& fp = a.fplan;
       const int bgx = (v.NX + (bp.lanes == 1 ? 8 : 32) - 1) / (bp.lanes == 1 ? 8 : 32);
       const int bgy = (v.NY + (bp.lanes == 1 ? 32 : 8) - 1) / (bp.lanes == 1 ? 32 : 8);
-      const int fgx = (v.NX + forward_brick_x(fp.lanes) - 1) / forward_brick_x(fp.lanes);
-      const int fgy = (v.NY + forward_brick_y(fp.lanes) - 1) / forward_brick_y(fp.lanes);
+      const int fgx = (v.NX + brick_x(fp.lanes) - 1) / brick_x(fp.lanes);
+      const int fgy = (v.NY + brick_y(fp.lanes) - 1) / brick_y(fp.lanes);
       // the persistent kernels take lines along X or Y over FP32 windows,
       // depths up to 16, of small axes
       const bool bp_ok = a.tma && !tma_disabled() && bp.lanes != 2 && !bp.pairs && bp.nz <= 16 &&
@@ -110,8 +110,9 @@ mtr_status mtr::build_sirt_tables(mtr_context* ctx, const std::vector<mtr_recon*
         t.own.push_back({r, k});
         continue;
       }
-      resd.push_back(ResBatchDesc{a.b.p, a.s.as<float>(), a.cf.as<float>(), a.r.as<float>(), a.np});
-      res_count.push_back((a.np + kBatchChunk - 1) / kBatchChunk);
+      resd.push_back(ResBatchDesc{a.b.p, a.s.as<float>(), a.cf.as<float>(), a.r.as<float>(), a.A, a.PY, a.pitch,
+                                  row_pair_pitch(a.PX)});
+      res_count.push_back(residual_batch_items(resd.back()));
       res_cost.push_back(1);
       const int j = (int)maps.size() / 2;
       maps.push_back(a.map_r);

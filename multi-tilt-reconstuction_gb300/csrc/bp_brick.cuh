@@ -47,15 +47,16 @@ constexpr uint32_t kDrainIters = 1u << 24;
 constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: x + kMagic holds round(x) in its low bits
 constexpr int kMagicBits = 0x4B400000;
 
-struct WinConst {
+struct __align__(16) WinConst {
   float xf, a1, a2, a3;  // x map relative to the CTA base voxel (fractional base)
   float yf, b1, b2, b3;
   int lxm, lym;          // window-local integer base minus the magic bits
   int ox, oy;            // window origin on the detector (ox aligned for TMA)
+  int flags, pad[3];     // row pairs: kHolds, kOnDetector
 };
-
-template <typename PT> __device__ __forceinline__ float to_f(PT v);
-template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
+// The window holds every tap of the brick at this angle (else the plan is wrong:
+// the angle is skipped and the launch flagged); every tap lies on the detector.
+constexpr int kHolds = 1, kOnDetector = 2;
 
 __device__ __forceinline__ int floor_div(int a, int b) { return (a >= 0) ? a / b : -((-a + b - 1) / b); }
 
@@ -81,63 +82,52 @@ template <int OFF> __device__ __forceinline__ float2 lds_h2_widened(uint32_t a) 
   return __half22float2(h);
 }
 
-// Gather of one voxel column (fixed X, Y; y-map without a Z term) from
-// detector rows `row0` and `row0 + WX`, adding into s[0..NZ).  x advances by
-// |a3| < 1 per voxel, so the fraction is stepped by one add and the tap
-// address by a predicated increment instead of a floor per voxel.  ASC walks
-// z upwards (a3 >= 0), else downwards, so that x never decreases.  Rounding
-// of the stepped fraction stays below 4e-6 px over 32 voxels; the caller
-// leaves one pixel of window slack for it.
-template <bool ASC, int NZ, typename PT>
-__device__ __forceinline__ void bp_column(float (&s)[NZ], const PT* row0, int WX, float xr, float a3, int lxm,
-                                          float wy0, float wy1) {
-  constexpr int zf = ASC ? 0 : NZ - 1;
-  const float x = fmaf(a3, (float)zf, xr);
-  const float flx = floorf(x);
-  float fx = x - flx;
+// Gather of one voxel column (fixed X, Y; y-map without a Z term) from a row of
+// row pairs (`row0`: elements (r[y], r[y + 1]) of one detector row), adding
+// into s[0..NZ).  x advances by |a3| < 1 per voxel.  The column carries the
+// y-interpolated value at its current pixel (B0) and the step to the next (D),
+// so a voxel costs two operations beside its fraction, and a pixel is loaded
+// (one 8-byte load for both rows, a crossing ahead of its use) and interpolated
+// in y once per pixel entered instead of at every voxel.  Some lane of a warp
+// crosses at almost every voxel, so the crossing is a few predicated
+// instructions and the load is not conditional (the next pixel's again where
+// the column stayed).  Bound by issue, 12 instructions a voxel where the four
+// taps took 17: 512x512x64 at 60 degrees, 61 angles, 0.52 against 0.70 ms; WBP
+// 0.55 against 0.89 ms.  The walk
+// runs z upwards; where a3 < 0 in the mirrored coordinate u = -x, whose pixels
+// p and p + 1 are the window's columns -p and -p - 1, so that one copy of the
+// code serves both signs.  Rounding of the stepped fraction stays below 4e-6 px
+// over 32 voxels; the window has one pixel of slack for it.
+template <int NZ>
+__device__ __forceinline__ void bp_column_rows(float (&s)[NZ], const float2* row0, float xr, float a3, int lxm,
+                                               float fy) {
+  const bool up = a3 >= 0.f;
+  const float u = up ? xr : -xr;
+  const float tu = __fadd_rd(u, kMagic);  // floor, in the low bits
+  float fx = u - (tu - kMagic);
   const float step = fabsf(a3);
-  static_assert(sizeof(PT) == 4, "FP32 windows");
-  uint32_t p = smem_u32(row0) + 4u * (uint32_t)(magic_int(flx) + lxm);
-  const uint32_t dr = 4u * (uint32_t)WX;
+  const int pix = __float_as_int(tu) - kMagicBits;
+  const uint32_t dp = up ? 8u : 0u - 8u;
+  uint32_t p = smem_u32(row0) + 8u * (uint32_t)((lxm + kMagicBits) + (up ? pix : -pix));
+  const float2 q0 = lds_f32x2<0>(p), q1 = lds_f32x2<0>(p + dp);
+  p += 2u * dp;
+  float2 n = lds_f32x2<0>(p);  // the pixel after the next (not used unless the column reaches it)
+  float b0 = fmaf(fy, q0.y - q0.x, q0.x), b1 = fmaf(fy, q1.y - q1.x, q1.x);
+  float d = b1 - b0;
 #pragma unroll
-  for (int i = 0; i < NZ; ++i) {
-    const int z = ASC ? i : NZ - 1 - i;
-    if (i > 0) {
+  for (int z = 0; z < NZ; ++z) {
+    if (z > 0) {
       fx += step;
-      const bool adv = fx >= 1.f;
-      fx = adv ? fx - 1.f : fx;
-      p += adv ? 4u : 0u;
+      if (fx >= 1.f) {
+        fx -= 1.f;
+        b0 = b1;
+        b1 = fmaf(fy, n.y - n.x, n.x);
+        p += dp;
+      }
+      d = b1 - b0;
+      n = lds_f32x2<0>(p);
     }
-    const float p00 = lds_f32<0>(p), p10 = lds_f32<4>(p);
-    const float p01 = lds_f32<0>(p + dr), p11 = lds_f32<4>(p + dr);
-    const float r0 = fmaf(fx, p10 - p00, p00);
-    const float r1 = fmaf(fx, p11 - p01, p01);
-    s[z] = fmaf(wy0, r0, s[z]);
-    s[z] = fmaf(wy1, r1, s[z]);
-  }
-}
-
-// The same column gather from a row pre-blended by the warp: b[i] holds the
-// y-interpolated detector value at window column i, so a voxel needs 2 taps.
-template <bool ASC, int NZ>
-__device__ __forceinline__ void bp_column_blended(float (&s)[NZ], const float* b, float xr, float a3, int lxm) {
-  constexpr int zf = ASC ? 0 : NZ - 1;
-  const float x = fmaf(a3, (float)zf, xr);
-  const float flx = floorf(x);
-  float fx = x - flx;
-  const float step = fabsf(a3);
-  uint32_t p = smem_u32(b) + 4u * (uint32_t)(magic_int(flx) + lxm);
-#pragma unroll
-  for (int i = 0; i < NZ; ++i) {
-    const int z = ASC ? i : NZ - 1 - i;
-    if (i > 0) {
-      fx += step;
-      const bool adv = fx >= 1.f;
-      fx = adv ? fx - 1.f : fx;
-      p += adv ? 4u : 0u;
-    }
-    const float p0 = lds_f32<0>(p), p1 = lds_f32<4>(p);
-    s[z] += fmaf(fx, p1 - p0, p0);
+    s[z] = fmaf(fx, d, s[z] + b0);
   }
 }
 
@@ -224,6 +214,8 @@ __device__ __forceinline__ void bp_column_half(float (&s)[NZ], const __half2* ro
   }
 }
 
+// The same column gather from a row pre-blended by the warp: b[i] holds the
+// y-interpolated pair of window column i.
 template <bool ASC, int NZ>
 __device__ __forceinline__ void bp_column_blended(float (&s)[NZ], const float2* b, float xr, float a3, int lxm) {
   constexpr int zf = ASC ? 0 : NZ - 1;
@@ -256,6 +248,7 @@ __device__ __forceinline__ void bp_column_zy(float (&s)[NZ], const WT* win, int 
   const uint32_t es = sizeof(WT), dr = es * (uint32_t)WX;
 #pragma unroll
   for (int z = 0; z < NZ; ++z) {
+    asm volatile("" : "+f"(xr), "+f"(yr));  // (one voxel's position at a time: no registers for all of them)
     const float x = fmaf(k.a3, (float)z, xr), y = fmaf(k.b3, (float)z, yr);
     const float tx = __fadd_rd(x, kMagic), ty = __fadd_rd(y, kMagic);  // floor, in the low bits
     const float fx = x - (tx - kMagic), fy = y - (ty - kMagic);
@@ -270,19 +263,31 @@ __device__ __forceinline__ void bp_column_zy(float (&s)[NZ], const WT* win, int 
       r0 = fmaf(fx, q0.y, q0.x);
       r1 = fmaf(fx, q1.y, q1.x);
     } else {
-      const float p00 = lds_f32<0>(p), p10 = lds_f32<4>(p), p01 = lds_f32<0>(p + dr), p11 = lds_f32<4>(p + dr);
-      r0 = fmaf(fx, p10 - p00, p00);
-      r1 = fmaf(fx, p11 - p01, p01);
+      const float2 q0 = lds_f32x2<0>(p), q1 = lds_f32x2<8>(p);  // both rows at two pixels
+      r0 = fmaf(fx, q1.x - q0.x, q0.x);
+      r1 = fmaf(fx, q1.y - q0.y, q0.y);
     }
     s[z] = fmaf(fy, r1 - r0, s[z] + r0);
   }
 }
 
+// Weight of a coordinate's two taps that lie on [0, n) (off: its integer base
+// minus the magic bits).
+__device__ __forceinline__ float tap_weight(float x, int off, int n) {
+  const float t = __fadd_rd(x, kMagic);
+  const float f = x - (t - kMagic);
+  const int i = __float_as_int(t) + off;
+  const bool in0 = (unsigned)i < (unsigned)n, in1 = (unsigned)(i + 1) < (unsigned)n;
+  return in0 ? (in1 ? 1.f : 1.f - f) : in1 ? f : 0.f;
+}
+
 // One brick (bx, by, bz) of one axis.  LANES: 0 = each warp a line of 32
 // voxels along X (brick 32x8), 1 = a line along Y (brick 8x32, used when the
-// detector x follows Y), 2 = an 8x4 patch (brick 32x8: on oblique axes the
-// taps of a line fall on a diagonal of the window that maps several lanes to
-// one shared-memory bank; a patch keeps them compact).  `smem` is the CTA's
+// detector x follows Y), 2 = an 8x4 patch (on oblique axes the taps of a line
+// fall on a diagonal of the window that maps several lanes to one shared-memory
+// bank; a patch keeps them compact).  Patches fill a 16x16 square, the smallest
+// footprint, or with the smaller elements of pairs along x a 32x8 brick (FP16
+// pairs, 512x512x64 at 60 degrees: 0.60 against 0.63 ms).  `smem` is the CTA's
 // dynamic shared memory; `reinit` re-initialises the mbarriers of a CTA that
 // already ran a brick.  PF (pair format, with PAIR): 0 interleaved FP32
 // pairs; 1 planar FP32 pairs, each detector row as two FP32 rows, its values
@@ -290,18 +295,17 @@ __device__ __forceinline__ void bp_column_zy(float (&s)[NZ], const WT* win, int 
 template <typename PT, int MODE, bool PAIR, int LANES, bool BZ0, int NZ, int PF = 0>
 __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& P, int bx, int by, int bz,
                                          unsigned char* smem, bool reinit) {
-  constexpr int BX = LANES == 1 ? kConsumerWarps : 32;
-  constexpr int BY = LANES == 1 ? 32 : kConsumerWarps;
-  // The SIRT update's windows hold residual pairs (value, next - value), one
-  // per pixel, from a pair array whose column c is pixel c - 1; the WBP's
-  // windows hold the projections.
+  constexpr int BX = bp_brick_x(LANES, PAIR), BY = bp_brick_y(LANES, PAIR);
+  // Windows hold row pairs (of the residual, or for the WBP of the
+  // projections), an element (x, y) the pixels (x, y) and (x, y + 1); or, with
+  // PAIR, residual pairs along x (value, next - value), one per pixel, from a
+  // pair array whose column c is pixel c - 1.
   static_assert(!PAIR || MODE == 1, "residual pairs feed the SIRT update only");
   constexpr bool PLANAR = PAIR && PF == 1, HALF = PAIR && PF == 2;
   static_assert(!PLANAR || BZ0, "planar windows are a pair format, for y-maps without a Z term");
   using WT = typename std::conditional<
       PLANAR, float,
-      typename std::conditional<HALF, __half2, typename std::conditional<PAIR, float2, PT>::type>::type>::type;
-  using BT = typename std::conditional<PAIR, float2, float>::type;  // blended-row element
+      typename std::conditional<HALF, __half2, float2>::type>::type;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
   uint64_t* empty = full + NST;
   WinConst* kc = reinterpret_cast<WinConst*>(smem + 128);
@@ -311,7 +315,7 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
   const size_t stage_bytes = (((size_t)win_elems * sizeof(WT)) + 127) & ~(size_t)127;
   WT* win0 = reinterpret_cast<WT*>(smem + 128 + kc_bytes);
   // per-warp blended row (uniform-row angles)
-  BT* blend = reinterpret_cast<BT*>(smem + 128 + kc_bytes + NST * stage_bytes) + (threadIdx.x >> 5) * P.WX;
+  float2* blend = reinterpret_cast<float2*>(smem + 128 + kc_bytes + NST * stage_bytes) + (threadIdx.x >> 5) * P.WX;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31;
@@ -354,6 +358,16 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
     k.oy = oy;
     k.lxm = xi - ox - kMagicBits;
     k.lym = yi - oy - kMagicBits;
+    k.flags = 0;
+    if (!PAIR) {
+      const float xmax = k.xf + fmaxf(0.f, k.a1 * (BX - 1)) + fmaxf(0.f, k.a2 * (BY - 1)) + fmaxf(0.f, k.a3 * (NZ - 1));
+      const float ymax = k.yf + fmaxf(0.f, k.b1 * (BX - 1)) + fmaxf(0.f, k.b2 * (BY - 1)) + fmaxf(0.f, k.b3 * (NZ - 1));
+      // first and last tap, with a pixel of slack for the rounding of a thread's own position
+      const int x0 = xi + (int)floorf(xmin) - 1, x1 = xi + (int)floorf(xmax) + 2;
+      const int y0 = yi + (int)floorf(ymin) - 1, y1 = yi + (int)floorf(ymax) + 2;
+      if (x0 >= ox && x1 < ox + P.WX && y0 >= oy && y1 <= oy + P.WY) k.flags |= kHolds;
+      if (x0 >= 0 && x1 < P.ax.PX && y0 >= 0 && y1 < P.ax.PY) k.flags |= kOnDetector;
+    }
     kc[a] = k;
   }
   __syncthreads();
@@ -373,10 +387,11 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
         }
         WT* dst = reinterpret_cast<WT*>(reinterpret_cast<unsigned char*>(win0) + s * stage_bytes);
         mbar_arrive_expect_tx(&full[s], bytes);
-        // interleaved pair arrays are mapped as FP32 pairs: x = 2 * (first pair
-        // column), a multiple of 4; planar ones as two FP32 rows per detector row
-        tma_load_3d(dst, tmap, (PLANAR || HALF) ? kc[a].ox + 1 : PAIR ? 2 * (kc[a].ox + 1) : kc[a].ox,
-                    PLANAR ? 2 * kc[a].oy : kc[a].oy, a, &full[s]);
+        // arrays of FP32 pairs are mapped as their floats: x = 2 * (first
+        // column), a multiple of 4; planar ones as two FP32 rows per detector
+        // row; row pairs have a row above the detector's first
+        tma_load_3d(dst, tmap, (PLANAR || HALF) ? kc[a].ox + 1 : PAIR ? 2 * (kc[a].ox + 1) : 2 * kc[a].ox,
+                    PLANAR ? 2 * kc[a].oy : PAIR ? kc[a].oy : kc[a].oy + 1, a, &full[s]);
         issued = a + 1;
       }
       // Drain: the last load issued into each stage must land before exit
@@ -390,17 +405,45 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
   }
 
   // ---------------- consumer warps
-  const int tx = LANES == 0 ? lane : LANES == 1 ? warp : (warp & 3) * 8 + (lane & 7);
-  const int ty = LANES == 0 ? warp : LANES == 1 ? lane : (warp >> 2) * 4 + (lane >> 3);
+  constexpr int kAcross = BX / 8;  // patches along X
+  const int tx = LANES == 0 ? lane : LANES == 1 ? warp : (warp % kAcross) * 8 + (lane & 7);
+  const int ty = LANES == 0 ? warp : LANES == 1 ? lane : (warp / kAcross) * 4 + (lane >> 3);
   const bool active = (X0 + tx < P.vol.Xs + P.vol.NX) && (Y0 + ty < P.vol.Ys + P.vol.NY);
   const int WX = P.WX;
-  // a tap at window column ix reads columns ix and ix + 1 (one pair column with pairs)
-  const unsigned lim_x = (unsigned)(PAIR ? WX : WX - 1), lim_y = (unsigned)(P.WY - 1);
-  float s[NZ], c[NZ];
+  // pairs along x: a tap at window (ix, iy) reads one pair of rows iy and iy + 1
+  const unsigned lim_x = (unsigned)WX, lim_y = (unsigned)(P.WY - 1);
+  const long long sx = P.vol.NX, sxy = (long long)P.vol.NX * P.vol.NY;
+  const long long base = (long long)(X0 + tx - P.vol.Xs) + (long long)(Y0 + ty - P.vol.Ys) * sx;
+  // WBP: the in-detector weight sums.  They depend on the geometry alone, and the
+  // weights of a voxel whose taps all lie on the detector sum to one, so they are
+  // formed first, from the angles at which the brick leaves the detector, and
+  // wait in cbp: the loop over the windows carries no second accumulator.
+  int n_inside = 0;  // angles at which the whole brick lies on the detector
+  if (MODE == 0) {
+    for (int a = 0; a < A; ++a) n_inside += (kc[a].flags & kOnDetector) ? 1 : 0;
+    if (n_inside < A) {
+      float c[NZ];
 #pragma unroll
-  for (int z = 0; z < NZ; ++z) { s[z] = 0.f; c[z] = 0.f; }
+      for (int z = 0; z < NZ; ++z) c[z] = (float)n_inside;
+      for (int a = 0; a < A; ++a) {
+        const WinConst k = kc[a];
+        if (k.flags & kOnDetector) continue;
+        const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
+        const float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
+#pragma unroll
+        for (int z = 0; z < NZ; ++z)
+          c[z] = fmaf(tap_weight(fmaf(k.a3, (float)z, xr), k.lxm + k.ox, P.ax.PX),
+                      tap_weight(fmaf(k.b3, (float)z, yr), k.lym + k.oy, P.ax.PY), c[z]);
+      }
+#pragma unroll
+      for (int z = 0; z < NZ; ++z)
+        if (active && Z0 + z < P.z1) P.cbp[base + (long long)(Z0 + z - P.z0) * sxy] = c[z];
+    }
+  }
+  float s[NZ];
+#pragma unroll
+  for (int z = 0; z < NZ; ++z) s[z] = 0.f;
   bool bad = false;
-  int n_inside = 0;  // WBP: angles whose taps of this column all lie on the detector
 
   for (int a = 0; a < A; ++a) {
     const int st = a % NST;
@@ -411,8 +454,25 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
     }
     const WT* w = reinterpret_cast<const WT*>(reinterpret_cast<const unsigned char*>(win0) + st * stage_bytes);
     const WinConst k = kc[a];
-    const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
+    float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
     float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
+    if constexpr (!PAIR) {
+      if (!(k.flags & kHolds)) {
+        bad = true;
+      } else if (active) {
+        if (BZ0 && fabsf(k.a3) < 0.999f) {
+          const float ty = __fadd_rd(yr, kMagic);  // floor, in the low bits
+          const float fy = yr - (ty - kMagic);
+          const WT* row0 = w + (__float_as_int(ty) + k.lym) * WX;
+          bp_column_rows<NZ>(s, row0, xr, k.a3, k.lxm, fy);
+        } else {
+          bp_column_zy<NZ, false, false>(s, w, WX, xr, yr, k);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[st]);
+      continue;
+    }
     // Uniform rows: the detector y does not move along the lanes (|slope| * 31
     // below 1e-6 px), so every lane of the warp reads the same two rows with
     // the same weights; the warp blends them once per angle.
@@ -432,12 +492,9 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
           } else if constexpr (HALF) {
             const float2 q0 = __half22float2(row0[i]), q1 = __half22float2(row0[i + WX]);
             blend[i] = make_float2(fmaf(fy, q1.x - q0.x, q0.x), fmaf(fy, q1.y - q0.y, q0.y));
-          } else if constexpr (PAIR) {
+          } else {
             const float2 q0 = row0[i], q1 = row0[i + WX];
             blend[i] = make_float2(fmaf(fy, q1.x - q0.x, q0.x), fmaf(fy, q1.y - q0.y, q0.y));
-          } else {
-            const float r0 = to_f(row0[i]);
-            blend[i] = fmaf(fy, to_f(row0[i + WX]) - r0, r0);
           }
         }
         blended = true;
@@ -447,18 +504,14 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
     bool done = !active;
     if (active && !BZ0) {
       // x and y are affine in z: the column's end voxels bound every tap, so
-      // the window (and for the WBP the detector) is checked once per column
+      // the window is checked once per column
       const float xe = fmaf(k.a3, (float)(NZ - 1), xr), ye = fmaf(k.b3, (float)(NZ - 1), yr);
       const int ixa = magic_int(floorf(xr)) + k.lxm, ixb = magic_int(floorf(xe)) + k.lxm;
       const int iya = magic_int(floorf(yr)) + k.lym, iyb = magic_int(floorf(ye)) + k.lym;
       bool inside = (unsigned)min(ixa, ixb) < lim_x && (unsigned)max(ixa, ixb) < lim_x &&
                     (unsigned)min(iya, iyb) < lim_y && (unsigned)max(iya, iyb) < lim_y;
-      if (MODE == 0)
-        inside = inside && min(ixa, ixb) + k.ox >= 0 && max(ixa, ixb) + 1 + k.ox < P.ax.PX &&
-                 min(iya, iyb) + k.oy >= 0 && max(iya, iyb) + 1 + k.oy < P.ax.PY;
       if (inside) {
         bp_column_zy<NZ, PAIR, HALF>(s, w, WX, xr, yr, k);
-        if (MODE == 0) ++n_inside;
         done = true;
       }
     }
@@ -472,13 +525,6 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
       const int ixa = magic_int(floorf(xr)) + k.lxm;
       const int ixb = magic_int(floorf(fmaf(k.a3, (float)(NZ - 1), xr))) + k.lxm;
       bool inside = (unsigned)rowi < lim_y && (unsigned)min(ixa, ixb) < lim_x && (unsigned)(max(ixa, ixb) + 1) < lim_x;
-      if (MODE == 0) {
-        // WBP also sums the in-detector weights: when both rows and every tap
-        // column of the voxel column lie on the detector, each voxel's four
-        // weights sum to one and the angle adds exactly 1 to its weight sum.
-        const int iy = rowi + k.oy, ix_lo = min(ixa, ixb) + k.ox, ix_hi = max(ixa, ixb) + 1 + k.ox;
-        inside = inside && iy >= 0 && iy + 1 < P.ax.PY && ix_lo >= 0 && ix_hi < P.ax.PX;
-      }
       if (inside) {
         if (blended) {
           if (k.a3 >= 0.f) bp_column_blended<true, NZ>(s, blend, xr, k.a3, k.lxm);
@@ -496,13 +542,12 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
           if (k.a3 >= 0.f) bp_column<true, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
           else bp_column<false, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
         }
-        if (MODE == 0) ++n_inside;
         done = true;
       }
     }
     if (!done) {
       // y part (per column when the map has no Z term)
-      float fy = 0.f, wy0 = 0.f, wy1 = 0.f, cy = 0.f;
+      float fy = 0.f, wy0 = 0.f, wy1 = 0.f;
       int rowi = 0;
       if (BZ0) {
         const float fly = floorf(yr);
@@ -511,10 +556,6 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
         if ((unsigned)rowi >= lim_y) bad = true;
         wy0 = 1.f - fy;
         wy1 = fy;
-        if (MODE == 0) {
-          const int iya = rowi + k.oy;
-          cy = ((unsigned)iya < (unsigned)P.ax.PY ? wy0 : 0.f) + ((unsigned)(iya + 1) < (unsigned)P.ax.PY ? wy1 : 0.f);
-        }
       }
 #pragma unroll
       for (int z = 0; z < NZ; ++z) {
@@ -526,11 +567,6 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
           if ((unsigned)rowi >= lim_y) bad = true;
           wy0 = 1.f - fy;
           wy1 = fy;
-          if (MODE == 0) {
-            const int iya = rowi + k.oy;
-            cy = ((unsigned)iya < (unsigned)P.ax.PY ? wy0 : 0.f) +
-                 ((unsigned)(iya + 1) < (unsigned)P.ax.PY ? wy1 : 0.f);
-          }
         }
         const float x = fmaf(k.a3, (float)z, xr);
         const float flx = floorf(x);
@@ -546,24 +582,13 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
           const float2 q0 = __half22float2(w[i0]), q1 = __half22float2(w[i0 + WX]);
           r0 = fmaf(fx, q0.y, q0.x);
           r1 = fmaf(fx, q1.y, q1.x);
-        } else if constexpr (PAIR) {
+        } else {
           const float2 q0 = w[i0], q1 = w[i0 + WX];
           r0 = fmaf(fx, q0.y, q0.x);
           r1 = fmaf(fx, q1.y, q1.x);
-        } else {
-          const float p00 = to_f(w[i0]), p10 = to_f(w[i0 + 1]);
-          const float p01 = to_f(w[i0 + WX]), p11 = to_f(w[i0 + WX + 1]);
-          r0 = fmaf(fx, p10 - p00, p00);
-          r1 = fmaf(fx, p11 - p01, p01);
         }
         s[z] = fmaf(wy0, r0, s[z]);
         s[z] = fmaf(wy1, r1, s[z]);
-        if (MODE == 0) {
-          const int ixa = ix + k.ox;
-          const float cx = ((unsigned)ixa < (unsigned)P.ax.PX ? 1.f - fx : 0.f) +
-                           ((unsigned)(ixa + 1) < (unsigned)P.ax.PX ? fx : 0.f);
-          c[z] = fmaf(cx, cy, c[z]);
-        }
       }
     }
     __syncwarp();
@@ -571,13 +596,6 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
   }
   if (bad) atomicExch(P.err, 5);
   if (!active) return;
-  if (MODE == 0) {
-#pragma unroll
-    for (int z = 0; z < NZ; ++z) c[z] += (float)n_inside;
-  }
-
-  const long long sx = P.vol.NX, sxy = (long long)P.vol.NX * P.vol.NY;
-  const long long base = (long long)(X0 + tx - P.vol.Xs) + (long long)(Y0 + ty - P.vol.Ys) * sx;
 #pragma unroll
   for (int z = 0; z < NZ; ++z) {
     const int zz = Z0 + z;
@@ -585,9 +603,10 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
     const long long vi = base + (long long)(zz - P.z0) * sxy;
     float out;
     if (MODE == 0) {
-      out = (c[z] != 0.f) ? s[z] / c[z] : 0.f;
+      const float c = n_inside < A ? P.cbp[vi] : (float)A;
+      out = c != 0.f ? s[z] / c : 0.f;
       P.vol_out[vi] = out;
-      P.cbp[vi] = c[z];
+      if (n_inside == A) P.cbp[vi] = c;
     } else {
       const float cv = P.cbp[vi];
       out = P.vol_out[vi];
@@ -605,9 +624,9 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
 // bricks of the same rows at all depths run together, so the detector rows
 // they read stay in L2 instead of being re-read from DRAM once per z layer.
 template <typename PT, int MODE, bool PAIR, int LANES, bool BZ0, int NZ, int PF = 0>
-// (FP32 pair windows take twice the shared memory: 4 CTAs per SM below depth 32;
-// at depth 32 the 32 accumulators fit the 56 registers of 4 CTAs per SM)
-__global__ void __launch_bounds__(kThreads, MODE == 1 ? (NZ >= 32 ? 4 : (PAIR && PF != 2 ? 4 : 5)) : 4)
+// (registers: 4 CTAs per SM leave 56, enough for 32 accumulators over x pairs;
+// the walk over row pairs takes 72 at depth 32)
+__global__ void __launch_bounds__(kThreads, !PAIR && NZ >= 32 ? 3 : MODE == 1 && NZ < 32 && PAIR && PF == 2 ? 5 : 4)
 bp_tma_kernel(const __grid_constant__ CUtensorMap tmap, const BpArgs P) {
   extern __shared__ __align__(128) unsigned char smem[];
   bp_brick<PT, MODE, PAIR, LANES, BZ0, NZ, PF>(&tmap, P, blockIdx.x, blockIdx.z, blockIdx.y, smem, false);
@@ -618,7 +637,7 @@ cudaError_t launch_one(const CUtensorMap& map, const BpArgs& P, size_t smem, cud
   auto kern = bp_tma_kernel<PT, MODE, PAIR, LANES, BZ0, NZ, PF>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const int BX = LANES == 1 ? kConsumerWarps : 32, BY = LANES == 1 ? 32 : kConsumerWarps;
+  constexpr int BX = bp_brick_x(LANES, PAIR), BY = bp_brick_y(LANES, PAIR);
   const dim3 grid((P.vol.NX + BX - 1) / BX, (P.z1 - P.z0 + NZ - 1) / NZ, (P.vol.NY + BY - 1) / BY);
   kern<<<grid, kThreads, smem, st>>>(map, P);
   const cudaError_t le = cudaGetLastError();
@@ -628,8 +647,8 @@ cudaError_t launch_one(const CUtensorMap& map, const BpArgs& P, size_t smem, cud
 
 template <typename PT, int MODE, bool PAIR, int LANES, bool BZ0, int PF = 0>
 cudaError_t launch_nz(const CUtensorMap& map, const BpArgs& P, const BpPlan& plan, cudaStream_t st) {
-  // WBP: depth 16 or 8 (it runs once per reconstruction).  SIRT: the tuned depth.
-  if constexpr (MODE == 0) {
+  if constexpr (MODE == 0) {  // the WBP has no depth 4
+    if (plan.nz == 32) return launch_one<PT, 0, PAIR, LANES, BZ0, 32>(map, P, plan.smem, st);
     if (plan.nz == 16) return launch_one<PT, 0, PAIR, LANES, BZ0, 16>(map, P, plan.smem, st);
     return launch_one<PT, 0, PAIR, LANES, BZ0, 8>(map, P, plan.smem, st);
   } else {

@@ -6,15 +6,12 @@
 // 3-D tiled cp.async.bulk.tensor loads (one box per angle; pixels outside
 // the detector are zero-filled by the TMA unit, which is exactly the
 // reference's "drop taps outside the detector" for the numerator).  Eight
-// consumer warps gather the four bilinear taps of every voxel from shared
+// consumer warps gather the bilinear taps of every voxel from shared
 // memory and accumulate over all angles in registers.
 //
-// Arithmetic per voxel and angle: one FFMA for the coordinate, FRND.FLOOR +
-// FADD for the fraction, an integer add to index the window (the float floor
-// is turned into an int by adding 1.5*2^23 and reading the bits, so no
-// float->int conversion runs in the loop), four LDS and six FFMA/FADD for the
-// interpolation.  When the y-map does not depend on Z (every synthetic and
-// single-axis TXBR geometry), the y-part is computed once per voxel column.
+// When the y-map does not depend on Z a voxel column stays between two
+// detector rows: the column is walked along x, and the rows are interpolated
+// once per pixel it enters (bp_column_rows).
 //
 // All mbarrier waits are bounded; a wait that gives up sets *err and the CTA
 // drains its own in-flight copies (bounded) before returning.
@@ -51,7 +48,7 @@ __device__ __forceinline__ void bp_batch_item(const CUtensorMap* map, const BpAr
   }
 }
 
-__global__ void __launch_bounds__(kThreads, 5)
+__global__ void __launch_bounds__(kThreads, 3)
 bp_batch_kernel(const BpBatchDesc* __restrict__ descs, const long long* __restrict__ first, int n_desc,
                 long long n_items, int* err, unsigned wait_iters) {
   extern __shared__ __align__(128) unsigned char smem[];
@@ -219,9 +216,9 @@ namespace {
 BpPlan plan_backproject_uncached(const std::vector<double>& xc, const std::vector<double>& yc, int A, int fmt,
                                  int nz, int lane) {
   BpPlan p;
-  // FP32, planar and FP16 pair windows start on a 4-element (16-byte)
-  // boundary; interleaved FP32 pair windows on an even pair column (16 bytes)
-  const bool pairs = fmt == 1;
+  // planar and FP16 pair windows start on a 4-element (16-byte) boundary;
+  // those of 8-byte elements (row pairs, interleaved pairs) on an even column
+  const bool pairs = fmt == 0 || fmt == 1;
   p.align = pairs ? 2 : 4;
   p.pairs = fmt != 0;
   p.planar = fmt == 2;
@@ -229,7 +226,7 @@ BpPlan plan_backproject_uncached(const std::vector<double>& xc, const std::vecto
   p.nz = nz;
   const size_t es = pairs ? 8 : 4;          // bytes per window element
   const int planes = p.planar ? 2 : 1;      // window rows per detector row
-  const size_t bes = p.pairs ? 8 : 4;       // bytes per blended-row element
+  const size_t bes = p.pairs ? 8 : 0;       // bytes per blended-row element (pairs along x)
   // Choose the lane axis so that consecutive lanes step along detector x.
   double sx = 0, sy = 0;
   bool bz0 = true;
@@ -241,7 +238,7 @@ BpPlan plan_backproject_uncached(const std::vector<double>& xc, const std::vecto
   // lane: -1 heuristic (lines along X or Y), 0 lines along X, 1 along Y, 2 patches
   p.lanes = lane < 0 ? (sy > sx ? 1 : 0) : std::min(lane, 2);
   p.bz0 = bz0;
-  const int BX = p.lanes == 1 ? kConsumerWarps : 32, BY = p.lanes == 1 ? 32 : kConsumerWarps, BZ = nz;
+  const int BX = bp_brick_x(p.lanes, p.pairs), BY = bp_brick_y(p.lanes, p.pairs), BZ = nz;
   double ex = 0, ey = 0;
   for (int a = 0; a < A; ++a) {
     ex = std::max(ex, std::fabs(xc[4 * a + 1]) * (BX - 1) + std::fabs(xc[4 * a + 2]) * (BY - 1) +
@@ -252,7 +249,7 @@ BpPlan plan_backproject_uncached(const std::vector<double>& xc, const std::vecto
   // taps span [floor(min)-1, floor(max)+1], origin rounded down to the alignment
   const int wx = (int)std::ceil(ex) + 4 + p.align;
   const int wx_min = (wx + p.align - 1) / p.align * p.align;
-  p.WY = (int)std::ceil(ey) + 4;
+  p.WY = (int)std::ceil(ey) + (fmt == 0 ? 3 : 4);  // (a row pair holds the next row)
   auto smem_for = [&](int WX) {
     const size_t stage = (((size_t)WX * p.WY * planes * es) + 127) & ~(size_t)127;
     return 128 + ((((size_t)A * sizeof(WinConst)) + 127) & ~(size_t)127) + NST * stage +

@@ -269,7 +269,7 @@ __device__ __forceinline__ void splat_column(uint32_t pre, int nz, uint32_t row,
 template <typename VT>
 __device__ __forceinline__ void prefix_brick(const CUtensorMap* smap, const FwdArgs& P, int lanes, int bx, int by,
                                              int zb, int g, unsigned char* smem) {
-  const int BX = forward_brick_x(lanes), BY = forward_brick_y(lanes), NZ = P.nz;
+  const int BX = brick_x(lanes), BY = brick_y(lanes), NZ = P.nz;
   PreConst* kc = reinterpret_cast<PreConst*>(smem);
   const size_t kc_bytes = ((size_t)P.max_angles * sizeof(PreConst) + 127) & ~(size_t)127;
   const int WX = P.WX, WY = P.WY;
@@ -480,7 +480,7 @@ __device__ __forceinline__ void stream_column_zy(uint32_t win, int WX, int WY, c
 template <typename VT, int NZ>
 __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs& P, int lanes, int bx, int by, int zb, int g,
                                           unsigned char* smem) {
-  const int BX = forward_brick_x(lanes), BY = forward_brick_y(lanes);
+  const int BX = brick_x(lanes), BY = brick_y(lanes);
   FwdConst* kc = reinterpret_cast<FwdConst*>(smem);
   const size_t kc_bytes = ((size_t)P.max_angles * sizeof(FwdConst) + 127) & ~(size_t)127;
   const int WX = P.WX, WY = P.WY;
@@ -640,7 +640,7 @@ size_t fwd_smem(int WX, int WY, int nz, bool bz0, int angles) {
 template <typename VT, int NZ>
 cudaError_t launch_one(const CUtensorMap& map, FwdArgs P, int lanes, int num_sms, cudaStream_t st) {
   auto kern = fwd_tma_kernel<VT, NZ>;
-  const int BX = forward_brick_x(lanes), BY = forward_brick_y(lanes);
+  const int BX = brick_x(lanes), BY = brick_y(lanes);
   const dim3 b3((P.vol.NX + BX - 1) / BX, (P.vol.NY + BY - 1) / BY, (P.z1 - P.z0 + P.nz - 1) / P.nz);
   const long long bricks = (long long)b3.x * b3.y * b3.z;
   // split the angles over several CTAs when there are too few bricks to fill the GPU
@@ -747,7 +747,7 @@ FwdPlan plan_forward_uncached(const std::vector<double>& xc, const std::vector<d
   p.lanes = lane < 0 ? (sy > sx ? 1 : 0) : std::min(lane, 2);
   p.bz0 = bz0;
   p.nz = nz;
-  const int BX = forward_brick_x(p.lanes), BY = forward_brick_y(p.lanes), BZ = p.nz;
+  const int BX = brick_x(p.lanes), BY = brick_y(p.lanes), BZ = p.nz;
   double ex = 0, ey = 0;
   for (int a = 0; a < A; ++a) {
     ex = std::max(ex, std::fabs(xc[4 * a + 1]) * (BX - 1) + std::fabs(xc[4 * a + 2]) * (BY - 1) +

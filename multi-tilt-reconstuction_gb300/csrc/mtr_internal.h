@@ -108,6 +108,19 @@ struct PlanMemo {
   }
 };
 
+// Brick of 256 columns: lines along X (32x8) or Y (8x32), or 8x4 patches in a
+// 16x16 square, whose footprint on an oblique axis is the smallest.
+#ifdef __CUDACC__
+#define MTR_HD __host__ __device__
+#else
+#define MTR_HD
+#endif
+MTR_HD constexpr int brick_x(int lanes) { return lanes == 0 ? 32 : lanes == 1 ? 8 : 16; }
+MTR_HD constexpr int brick_y(int lanes) { return lanes == 0 ? 8 : lanes == 1 ? 32 : 16; }
+// (the back-projection over pairs along x keeps its patches in a 32x8 brick)
+MTR_HD constexpr int bp_brick_x(int lanes, bool pairs) { return lanes == 2 && pairs ? 32 : brick_x(lanes); }
+MTR_HD constexpr int bp_brick_y(int lanes, bool pairs) { return lanes == 2 && pairs ? 8 : brick_y(lanes); }
+
 // ---- TMA-staged back-projection (bp_tma.cu) -------------------------------
 // Window geometry of one axis for the brick shape used by the TMA kernel.
 struct BpPlan {
@@ -115,9 +128,9 @@ struct BpPlan {
   int lanes = 0;       // warp layout: 0 lines along X, 1 lines along Y, 2 8x4 patches
   bool bz0 = false;    // y map independent of Z for every angle
   int WX = 0, WY = 0;  // window box (elements)
-  int align = 4;       // TMA x alignment (elements)
+  int align = 2;       // TMA x alignment (elements)
   int nz = 8;          // brick depth (voxels per thread along Z): 4, 8 or 16
-  bool pairs = false;  // windows of residual pairs (SIRT update) rather than FP32 projections (WBP)
+  bool pairs = false;  // windows of pairs along x (SIRT update) rather than row pairs
   bool planar = false; // pairs as two FP32 planes per row (values, differences) instead of interleaved
   bool half = false;   // pairs as FP16 (value, difference) in 32 bits (mixed precision)
   size_t smem = 0;     // dynamic shared memory per CTA
@@ -130,16 +143,24 @@ double window_bank_cost(const std::vector<double>& xc, const std::vector<double>
                         int WX, bool pairs = false);
 // lane: -1 picks lines along the larger x-map slope, 0 = lines along X,
 // 1 = lines along Y, 2 = 8x4 patches.
-// pairs: windows of residual pairs for the SIRT update (false: FP32 windows
-// of the projections for the WBP).
-// fmt: 0 FP32 windows, 1 interleaved residual pairs, 2 planar residual pairs,
-// 3 FP16 residual pairs (mixed precision).
+// fmt: 0 FP32 row pairs (also the WBP's windows of the projections), 1
+// interleaved residual pairs along x, 2 planar ones, 3 FP16 ones (mixed
+// precision).
 BpPlan plan_backproject(const std::vector<double>& xc, const std::vector<double>& yc, int A, int fmt, int nz,
                         int lane = -1);
 // Row pitch (pairs) of the residual pair array of a detector PX pixels wide:
 // pair column c holds (r[c-1], r[c] - r[c-1]) for c in [0, PX], zero beyond,
 // padded to a multiple of 4 pairs (32-byte rows).
 inline int pair_pitch(int px) { return (px + 1 + 3) / 4 * 4; }
+// An image in row pairs, for windows whose element at (x, y) holds pixels (x, y)
+// and (x, y + 1): rows 0..PY (row j the pixels of rows j - 1 and j, zero off the
+// detector) of row_pair_pitch(PX) FP32 pairs.
+inline int row_pair_pitch(int px) { return (px + 3) / 4 * 4; }
+// mode 0: of the residual b - s/c (c != 0, else b - s), s reset to zero, norm2:
+// FP64 sum of its squares (or null); mode 1: of b (s and c not read).
+template <typename BT>
+void launch_row_pairs(int mode, const AxisDev& ax, const BT* b, float* s, const float* c, float* out, double* norm2,
+                      cudaStream_t st);
 // Residual in pair form: r = b - s/c (c != 0, else b - s) per detector row
 // (`rows` rows of `pitch` elements), written as pitch2 pairs per row:
 // form 0 interleaved FP32 (value, difference), 1 planar (the row's values,
@@ -173,15 +194,6 @@ struct FwdPlan {
   int nz = 16;         // brick depth: 8, 16 or 32; up to 32 where the y-map has no Z term
   size_t smem = 0;
 };
-// Brick of 256 columns: lines along X (32x8) or Y (8x32), or 8x4 patches in a
-// 16x16 square, whose footprint on an oblique axis is the smallest.
-#ifdef __CUDACC__
-#define MTR_HD __host__ __device__
-#else
-#define MTR_HD
-#endif
-MTR_HD constexpr int forward_brick_x(int lanes) { return lanes == 0 ? 32 : lanes == 1 ? 8 : 16; }
-MTR_HD constexpr int forward_brick_y(int lanes) { return lanes == 0 ? 8 : lanes == 1 ? 32 : 16; }
 FwdPlan plan_forward(const std::vector<double>& xc, const std::vector<double>& yc, int A, int PX, int PY, int pitch,
                      int nz, int lane = -1);
 template <typename VT>
@@ -217,9 +229,11 @@ struct ResBatchDesc {
   const void* b;         // projections (float or half)
   float* s;
   const float* cf;
-  float* r;
-  long long n;
+  float* r;              // written in row pairs
+  int A, PY, pitch, pp;  // pp: row_pair_pitch of the detector
 };
+// Work items of one axis' residual in the persistent kernel.
+long long residual_batch_items(const ResBatchDesc& d);
 struct MaceBatchDesc {
   int K;
   void* w[MTR_MAX_AXES];  // MACE states: FP32, or FP16 deviations from wavg when w_half

@@ -282,7 +282,7 @@ struct AxisState {
   std::vector<double> hxc, hyc;  // host copies of the maps (kernel planning)
   BpPlan plan;            // TMA back-projection window plan over r (FP32)
   BpPlan plan_b;          // WBP plan (FP32 windows, depth 8)
-  CUtensorMap map_b{}, map_r{};  // WBP map over b (FP32) or over r holding b widened (mixed); map over r
+  CUtensorMap map_b{}, map_r{};  // WBP map over r holding b's row pairs; map over r in its SIRT update's form
   bool tma = false, tma_b = false;
   FwdPlan fplan;          // windowed forward splat plan
   CUtensorMap map_s{}, map_cf{};  // tensor maps over s and cf (valid when ftma)
@@ -303,8 +303,8 @@ struct AxisState {
   DevBuf b;               // projections: float (FP32) or half (mixed)
   DevBuf s;               // forward accumulator, float
   DevBuf cf;              // forward row sums A 1, float
-  DevBuf r;               // residual: FP32 [A][PY][pitch], or pairs [A][PY][pitch2] when the
-                          // windowed back-projection reads it (tma)
+  DevBuf r;               // residual: FP32 [A][PY][pitch], or in the windowed back-projection's form
+                          // (row pairs, pairs along x, a line image)
   DevBuf cbp;             // back-projection weight sums A^T 1 (volume), float
   DevBuf w;               // MACE state w_k (volume), float
   DevBuf x;               // SIRT iterate z_k -> v_k (volume), float
@@ -323,11 +323,12 @@ inline bool encode_pair_map(CUtensorMap* m, const AxisState& a, const BpPlan& p)
   if (p.planar) return encode_tensor_map_3d(m, a.r.p, false, a.pitch2, a.pitch2, 2 * a.PY, a.A, p.WX, 2 * p.WY);
   return encode_tensor_map_3d(m, a.r.p, false, 2 * a.pitch2, 2 * a.pitch2, a.PY, a.A, 2 * p.WX, p.WY);
 }
-// Tensor map over an axis' residual in the form its SIRT update reads: pairs,
-// or FP32 rows of `pitch` elements.
+// Tensor map over an axis' residual in the form its SIRT update reads: pairs
+// along x, or row pairs (PY + 1 rows of 2 * row_pair_pitch floats).
 inline bool encode_residual_map(CUtensorMap* m, const AxisState& a, const BpPlan& p) {
   return p.pairs ? encode_pair_map(m, a, p)
-                 : encode_tensor_map_3d(m, a.r.p, false, a.PX, a.pitch, a.PY, a.A, p.WX, p.WY);
+                 : encode_tensor_map_3d(m, a.r.p, false, 2 * a.PX, 2 * row_pair_pitch(a.PX), a.PY + 1, a.A, 2 * p.WX,
+                                        p.WY);
 }
 
 // Disable the TMA kernels (MTR_DISABLE_TMA=1 in the environment) to run the

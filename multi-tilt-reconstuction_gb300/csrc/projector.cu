@@ -13,6 +13,7 @@
 // thread adds float slope * (small offset) to the fraction.  The float part
 // stays below ~100 in magnitude, so the tap position carries ~1e-5 px of
 // error however large the detector is, and the inner loop is pure FP32.
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -358,20 +359,117 @@ residual_pairs_kernel(long long rows, int pitch, int pitch2, const BT* __restric
   }
 }
 
-// Residual over many axes: item = (descriptor, chunk of kBatchChunk pixels).
+// Row pairs of one strip of kStripRows detector rows by 128 columns, one warp:
+// each lane walks down four columns, so a row's value meets the next one in
+// registers; the pairs that straddle two strips are written half by each.
+// IMG: of b itself (the WBP's windows), else of the residual; returns the
+// lane's sum of squares.  Bound by HBM (24 bytes per pixel with the 8-byte
+// pairs): four rows' loads are in flight at a time.
+constexpr int kStripRows = 8;
+template <typename BT, bool IMG>
+__device__ __forceinline__ float row_pair_strip(const BT* __restrict__ b, float* __restrict__ s,
+                                                const float* __restrict__ c, float* __restrict__ out, int PY,
+                                                int pitch, int pp, int a, int y0, int col) {
+  if (col >= pp) return 0.f;
+  const long long in = (long long)a * PY * pitch + col;
+  float* o = out + 2 * ((long long)a * (PY + 1) * pp + col);
+  const int y1 = min(y0 + kStripRows, PY);
+  float prev[4] = {0.f, 0.f, 0.f, 0.f}, sq = 0.f;
+  for (int yb = y0; yb < y1; yb += 4) {
+    float bv[4][4];
+    float4 sv[4], cv[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const long long i = in + (long long)min(yb + q, y1 - 1) * pitch;
+      ld4(b + i, bv[q]);
+      if (!IMG) {
+        sv[q] = *reinterpret_cast<const float4*>(s + i);
+        cv[q] = __ldg(reinterpret_cast<const float4*>(c + i));
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int y = yb + q;
+      if (y >= y1) break;
+      float r[4] = {bv[q][0], bv[q][1], bv[q][2], bv[q][3]};
+      if (!IMG) {
+        r[0] -= cv[q].x != 0.f ? sv[q].x / cv[q].x : sv[q].x;
+        r[1] -= cv[q].y != 0.f ? sv[q].y / cv[q].y : sv[q].y;
+        r[2] -= cv[q].z != 0.f ? sv[q].z / cv[q].z : sv[q].z;
+        r[3] -= cv[q].w != 0.f ? sv[q].w / cv[q].w : sv[q].w;
+        *reinterpret_cast<float4*>(s + in + (long long)y * pitch) = make_float4(0.f, 0.f, 0.f, 0.f);
+        sq += r[0] * r[0] + r[1] * r[1] + r[2] * r[2] + r[3] * r[3];
+      }
+      float* p = o + 2LL * y * pp;  // row y: the pixels of rows y - 1 and y
+      if (y > y0 || y == 0) {
+        *reinterpret_cast<float4*>(p) = make_float4(prev[0], r[0], prev[1], r[1]);
+        *reinterpret_cast<float4*>(p + 4) = make_float4(prev[2], r[2], prev[3], r[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) p[2 * e + 1] = r[e];
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) prev[e] = r[e];
+    }
+  }
+  float* p = o + 2LL * y1 * pp;
+  if (y1 == PY) {
+    *reinterpret_cast<float4*>(p) = make_float4(prev[0], 0.f, prev[1], 0.f);
+    *reinterpret_cast<float4*>(p + 4) = make_float4(prev[2], 0.f, prev[3], 0.f);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) p[2 * e] = prev[e];
+  }
+  return sq;
+}
+__host__ __device__ inline int strips_of(int PY) { return (PY + kStripRows - 1) / kStripRows; }
+__host__ __device__ inline int blocks_of(int pp) { return (pp + 127) / 128; }
+
+template <typename BT, bool IMG, bool NORM>
+__global__ void __launch_bounds__(256)
+row_pairs_kernel(int A, int PY, int pitch, int pp, const BT* __restrict__ b, float* __restrict__ s,
+                 const float* __restrict__ c, float* __restrict__ out, double* __restrict__ norm2) {
+  const int lane = threadIdx.x & 31, nb = blocks_of(pp), ns = strips_of(PY);
+  const long long items = (long long)A * ns * nb, nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  double acc = 0.0;
+  for (long long it = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; it < items; it += nwarps) {
+    const int xb = (int)(it % nb), st = (int)(it / nb % ns), a = (int)(it / nb / ns);
+    const float sq = row_pair_strip<BT, IMG>(b, s, c, out, PY, pitch, pp, a, st * kStripRows, 128 * xb + 4 * lane);
+    if (NORM) acc += (double)sq;
+  }
+  if (NORM) {
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    __shared__ double red[8];
+    if (lane == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double t = 0.0;
+      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
+      atomicAdd(norm2, t);
+    }
+  }
+}
+
+// Residual over many axes: item = (descriptor, 64 strips, 8 per warp).
+constexpr int kStripsPerItem = 64;
+template <typename BT>
+__device__ __forceinline__ void residual_batch_item(const ResBatchDesc& D, int first) {
+  const int lane = threadIdx.x & 31, nb = blocks_of(D.pp), ns = strips_of(D.PY);
+  const int end = min(first + kStripsPerItem, D.A * ns * nb);
+  for (int it = first + (int)(threadIdx.x >> 5); it < end; it += 8) {
+    const int xb = it % nb, st = it / nb % ns, a = it / nb / ns;
+    row_pair_strip<BT, false>(static_cast<const BT*>(D.b), D.s, D.cf, D.r, D.PY, D.pitch, D.pp, a, st * kStripRows,
+                              128 * xb + 4 * lane);
+  }
+}
 template <bool HALF_B>
 __global__ void __launch_bounds__(256)
 residual_batch_kernel(const ResBatchDesc* __restrict__ descs, const long long* __restrict__ first, int n_desc,
                       long long n_items) {
   for (long long it = blockIdx.x; it < n_items; it += gridDim.x) {
     const int2 item = work_item(first, n_desc, it);
-    const ResBatchDesc& D = descs[item.x];
-    const long long i0 = (long long)item.y * kBatchChunk;
-    const long long i1 = min(D.n, i0 + kBatchChunk);  // both multiples of 8 (row pitch)
-    for (long long i = i0 + 4 * threadIdx.x; i < i1; i += 4 * blockDim.x) {
-      if (HALF_B) residual4(static_cast<const __half*>(D.b) + i, D.s + i, D.cf + i, D.r + i);
-      else residual4(static_cast<const float*>(D.b) + i, D.s + i, D.cf + i, D.r + i);
-    }
+    if (HALF_B) residual_batch_item<__half>(descs[item.x], item.y * kStripsPerItem);
+    else residual_batch_item<float>(descs[item.x], item.y * kStripsPerItem);
   }
 }
 
@@ -416,6 +514,26 @@ void launch_residual(long long n, const BT* b, float* s, const float* c, RT* r, 
   if (norm2) residual_kernel<BT, true><<<(unsigned)blocks, 256, 0, st>>>(n, n4, b, s, c, r, norm2);
   else residual_kernel<BT, false><<<(unsigned)blocks, 256, 0, st>>>(n, n4, b, s, c, r, nullptr);
 }
+
+long long residual_batch_items(const ResBatchDesc& d) {
+  return ((long long)d.A * strips_of(d.PY) * blocks_of(d.pp) + kStripsPerItem - 1) / kStripsPerItem;
+}
+
+template <typename BT>
+void launch_row_pairs(int mode, const AxisDev& ax, const BT* b, float* s, const float* c, float* out, double* norm2,
+                      cudaStream_t st) {
+  const int pp = row_pair_pitch(ax.PX);
+  const long long warps = (long long)ax.A * strips_of(ax.PY) * blocks_of(pp);
+  // grid-stride over the rest
+  const unsigned g = (unsigned)std::max(1LL, std::min((warps + 7) / 8, (long long)device_sm_count() * 16));
+  if (mode == 1) row_pairs_kernel<BT, true, false><<<g, 256, 0, st>>>(ax.A, ax.PY, ax.pitch, pp, b, s, c, out, nullptr);
+  else if (norm2) row_pairs_kernel<BT, false, true><<<g, 256, 0, st>>>(ax.A, ax.PY, ax.pitch, pp, b, s, c, out, norm2);
+  else row_pairs_kernel<BT, false, false><<<g, 256, 0, st>>>(ax.A, ax.PY, ax.pitch, pp, b, s, c, out, nullptr);
+}
+template void launch_row_pairs<float>(int, const AxisDev&, const float*, float*, const float*, float*, double*,
+                                      cudaStream_t);
+template void launch_row_pairs<__half>(int, const AxisDev&, const __half*, float*, const float*, float*, double*,
+                                       cudaStream_t);
 
 void launch_residual_batch(const ResBatchDesc* descs, const long long* first, int n_desc, long long n_items, int half_b,
                            int grid, cudaStream_t st) {

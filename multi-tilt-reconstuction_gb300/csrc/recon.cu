@@ -38,11 +38,12 @@ int copy_kind_of(int precision) {
 
 bool mixed(int precision) { return precision != MTR_PREC_FP32; }
 
-// Bytes of the residual array of an axis: room for the FP32 residual and for
-// its pair form (8 bytes per pixel plus one column), whichever the axis' back-
-// projection reads.
+// Bytes of the residual array of an axis: room for the FP32 residual, its
+// pairs along x (8 bytes per pixel plus one column) and its row pairs (plus one
+// row), whichever the axis' back-projection reads.
 long long residual_bytes(int PX, int PY, int A) {
-  return std::max((long long)projection_pitch(PX) * PY * A * 4, (long long)pair_pitch(PX) * PY * A * 8);
+  return std::max({(long long)projection_pitch(PX) * PY * A * 4, (long long)pair_pitch(PX) * PY * A * 8,
+                   (long long)row_pair_pitch(PX) * (PY + 1) * A * 8});
 }
 
 // Bytes per voxel of an axis' MACE state w_k: FP32, or in mixed precision its
@@ -233,6 +234,13 @@ mtr_status enqueue_residual(mtr_recon* r, AxisState& a, double* norm) {
     else
       launch_residual_pairs<float>(rows, a.pitch, a.pitch2, a.b.as<float>(), a.s.as<float>(), a.cf.as<float>(),
                                    a.r.as<float>(), a.plan.planar ? 1 : 0, norm, ctx->stream);
+  } else if (a.tma) {  // row pairs
+    if (mixed(r->p.precision))
+      launch_row_pairs<__half>(0, a.dev(), a.b.as<__half>(), a.s.as<float>(), a.cf.as<float>(), a.r.as<float>(), norm,
+                               ctx->stream);
+    else
+      launch_row_pairs<float>(0, a.dev(), a.b.as<float>(), a.s.as<float>(), a.cf.as<float>(), a.r.as<float>(), norm,
+                              ctx->stream);
   } else if (mixed(r->p.precision)) {
     launch_residual<__half, float>(a.np, a.b.as<__half>(), a.s.as<float>(), a.cf.as<float>(), a.r.as<float>(), norm,
                                    ctx->stream);
@@ -244,9 +252,8 @@ mtr_status enqueue_residual(mtr_recon* r, AxisState& a, double* norm) {
   return MTR_OK;
 }
 
-// What the WBP gathers, prepared in r (free until the first residual): with
-// line kernels the projections' line image, and in mixed precision the FP16
-// projections widened for the FP32 windows.
+// What the WBP gathers, prepared in r (free until the first residual): the
+// projections' line image, or their row pairs for the windows.
 mtr_status enqueue_widen_for_wbp(mtr_recon* r, AxisState& a) {
   if (a.lines) {  // the WBP gathers the projections' line image
     const cudaError_t e =
@@ -258,15 +265,18 @@ mtr_status enqueue_widen_for_wbp(mtr_recon* r, AxisState& a) {
     g_launches.fetch_add(1);
     return e == cudaSuccess ? MTR_OK : cuda_error(r->ctx, e, "projections' line image");
   }
-  if (!(a.tma_b && mixed(r->p.precision))) return MTR_OK;
-  launch_widen(a.b.as<__half>(), a.r.as<float>(), a.np, r->ctx->stream);
-  MTR_CK_LAUNCH(r->ctx, "widen projections");
+  if (!a.tma_b) return MTR_OK;
+  if (mixed(r->p.precision))
+    launch_row_pairs<__half>(1, a.dev(), a.b.as<__half>(), nullptr, nullptr, a.r.as<float>(), nullptr, r->ctx->stream);
+  else
+    launch_row_pairs<float>(1, a.dev(), a.b.as<float>(), nullptr, nullptr, a.r.as<float>(), nullptr, r->ctx->stream);
+  MTR_CK_LAUNCH(r->ctx, "projections' row pairs");
   return MTR_OK;
 }
 
 // mode 0: WBP (x = s/c, cbp = c); mode 1: SIRT update from the residual.
-// widen: for the windowed mixed-precision WBP, widen the projections first
-// (a caller that runs several WBP spans of one axis widens them once).
+// widen: prepare the WBP's image first (a caller that runs several WBP spans of
+// one axis prepares it once).
 mtr_status enqueue_bp(mtr_recon* r, AxisState& a, int mode, const VolSpan& sp, bool widen = true) {
   mtr_context* ctx = r->ctx;
   const VolDev& v = r->vol;
@@ -288,7 +298,7 @@ mtr_status enqueue_bp(mtr_recon* r, AxisState& a, int mode, const VolSpan& sp, b
     return MTR_OK;
   }
   if (mode == 0 ? a.tma_b : a.tma) {
-    if (half_img && widen) {
+    if (mode == 0 && widen) {
       mtr_status s = enqueue_widen_for_wbp(r, a);
       if (s != MTR_OK) return s;
     }
@@ -604,8 +614,7 @@ mtr_status mtr_recon_create(mtr_context* ctx, int n_axes, const mtr_axis* axes, 
     if (a.lines) {
       record_untimed_tiles(a, r->vol, params->precision);
     } else if (!tma_disabled()) {
-      // WBP over b; with FP16 projections over their FP32 widening in r (r is
-      // free until the first residual), so the WBP gathers FP32 like SIRT.
+      // WBP over the projections' row pairs in r (free until the first residual)
       // SIRT back-projection over the FP32 residual and the forward splat: tuned depths
       if (streamed) {  // candidates over one slab, in the slot arrays the run uses
         VolDev tv = r->vol;
@@ -618,12 +627,10 @@ mtr_status mtr_recon_create(mtr_context* ctx, int n_axes, const mtr_axis* axes, 
                   r->err.as<int>());
       }
       // The WBP gathers the same windows as the SIRT update: the lane layout
-      // tuned for it (lines or 8x4 patches), at depth 16 where the tuned depth
-      // is 16 or more, else 8.
-      a.plan_b = plan_backproject(a.hxc, a.hyc, a.A, 0, a.plan.ok && a.plan.nz >= 16 ? 16 : 8,
+      // tuned for it (lines or 8x4 patches) and its depth, at least 8.
+      a.plan_b = plan_backproject(a.hxc, a.hyc, a.A, 0, a.plan.ok ? std::max(8, a.plan.nz) : 8,
                                   a.plan.ok ? a.plan.lanes : -1);
-      a.tma_b = a.plan_b.ok && encode_tensor_map_3d(&a.map_b, mx ? a.r.p : a.b.p, false, a.PX, a.pitch, a.PY, a.A,
-                                                    a.plan_b.WX, a.plan_b.WY);
+      a.tma_b = a.plan_b.ok && encode_residual_map(&a.map_b, a, a.plan_b);
     }
   }
   if (params->flags & MTR_FLAG_RECORD_NORMS) {

@@ -10,13 +10,11 @@
 //    the volume axis that detector x follows keep shared-memory gathers free
 //    of bank conflicts, and (back-projection) 8x4 patches keep the taps of an
 //    oblique axis compact in the window;
-//  * the SIRT back-projection's window format: FP32 residual values, or
-//    (value, next - value) pairs that halve the tap loads but double the
-//    window and load 8 bytes per lane (faster where a warp's lanes share
-//    detector rows, slower where their 8-byte loads conflict in the banks),
-//    or the same pairs as two FP32 planes per row (4-byte loads with the FP32
-//    window's bank pattern, one FFMA per row), or (mixed precision) FP16
-//    pairs in 32 bits (one 4-byte load per row: half the shared-memory bytes).
+//  * the SIRT back-projection's window format: FP32 row pairs (a column is
+//    walked pixel by pixel along one row of pairs), (value, next - value) pairs
+//    along x (faster where a warp's lanes share detector rows), or the same
+//    pairs as two FP32 planes per row (4-byte loads); in mixed precision FP16
+//    pairs in 32 bits on large oblique axes (fp16_residual).
 // For each tilt axis the tuner times every candidate (3 formats x depth
 // 4/8/16/32 x lines along X / lines along Y / patches for the SIRT
 // back-projection, depth 8/16/32 x the same three layouts for the forward
@@ -25,9 +23,9 @@
 // (each candidate launch writes only scratch that the run overwrites), and
 // keeps the fastest.  Results are cached per process by a geometry key and,
 // when MTR_AUTOTUNE_CACHE names a file, persisted there as JSON ({"key":
-// [bp_depth, fwd_depth, bp_lane, fwd_lane, bp_format], ...}; bp_format 0 FP32
-// windows, 1 interleaved pairs, 2 planar pairs, 3 FP16 pairs in mixed precision).  MTR_AUTOTUNE=0 disables
-// tuning (depths 8 and 16, lane axis by slope, FP32 windows);
+// [bp_depth, fwd_depth, bp_lane, fwd_lane, bp_format], ...}; bp_format 0 row
+// pairs, 1 interleaved pairs, 2 planar pairs, 3 FP16 pairs in mixed precision).  MTR_AUTOTUNE=0 disables
+// tuning (depths 8 and 16, lane axis by slope, row pairs);
 // MTR_FORCE_DEPTHS=bp,fwd[,bp_lane,fwd_lane[,bp_format]] pins the choice;
 // MTR_AUTOTUNE_LOG=1 prints every candidate's time to stderr.
 #include <algorithm>
@@ -50,7 +48,7 @@ namespace {
 
 struct Choice {
   int bp_nz = 8, fwd_nz = 16, bp_lane = -1, fwd_lane = -1;
-  int bp_pairs = 0;  // SIRT update window format: 0 FP32, 1 interleaved residual pairs, 2 planar pairs
+  int bp_pairs = 0;  // SIRT update window format: 0 row pairs, 1 interleaved residual pairs, 2 planar pairs
 };
 
 std::mutex g_mu;
@@ -111,9 +109,24 @@ std::string geometry_key(const AxisState& a, const VolDev& v, int precision) {
   }
   char buf[256];
   // the trailing tag names the timing method, so choices cached by an older one are not reused
-  std::snprintf(buf, sizeof(buf), "p%dx%dx%d_v%dx%dx%d_m%.2f,%.2f,%.2f,%.2f,%.2f,%.2f_z%d_prec%d_t10", a.PX, a.PY,
+  std::snprintf(buf, sizeof(buf), "p%dx%dx%d_v%dx%dx%d_m%.2f,%.2f,%.2f,%.2f,%.2f,%.2f_z%d_prec%d_t12", a.PX, a.PY,
                 a.A, v.NX, v.NY, v.NZ, m[0], m[1], m[2], m[3], m[4], m[5], bz0 ? 0 : 1, precision);
   return buf;
+}
+
+// Mixed precision stores the residual of a large oblique axis as FP16 pairs
+// (half the bytes of the row pairs or FP32 pairs): part of that mode's
+// rounding, so it is decided by the geometry and not by a race between formats.
+// Axes whose rows lie within 6 degrees of a volume axis, z-dependent y-maps and
+// volumes of fewer than four 32x8x16 bricks per SM keep FP32, as the tuner
+// chose for them when it timed all formats (256x256x64 at 17-60 degrees FP16,
+// 128x128x32 and 1 or 89 degrees FP32).
+bool fp16_residual(const AxisState& a, const VolDev& v, int sms) {
+  for (int k = 0; k < a.A; ++k) {
+    const double* c = &a.hyc[4 * (size_t)k];
+    if (c[3] != 0.0 || std::min(std::fabs(c[1]), std::fabs(c[2])) < 0.1) return false;
+  }
+  return (long long)((v.NX + 31) / 32) * ((v.NY + 7) / 8) * ((v.NZ + 15) / 16) >= 4LL * sms;
 }
 
 // Times every candidate launch and returns the index of the fastest (-1 if
@@ -238,11 +251,11 @@ bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, int precision, f
     std::vector<BpPlan> bps;
     std::vector<CUtensorMap> bmaps;
     // (the candidates keep pointers into these: no reallocation)
-    // (FP16 residual pairs only in mixed precision)
-    const int n_fmt = copy_kind != 0 ? 4 : 3;
+    const bool fp16 = copy_kind != 0 && fp16_residual(a, v, ctx->num_sms);
+    const int fmt0 = fp16 ? 3 : 0, fmt1 = fp16 ? 4 : 3;
     bps.reserve(12 * std::size(kBpDepths));  // formats x 3 lane layouts x the depths
     bmaps.reserve(12 * std::size(kBpDepths));
-    for (int fmt = 0; fmt < n_fmt; ++fmt)
+    for (int fmt = fmt0; fmt < fmt1; ++fmt)
       for (int lane = 0; lane < 3; ++lane)
         for (int nz : kBpDepths) {
           BpPlan p = plan_backproject(a.hxc, a.hyc, a.A, fmt, nz, lane);
