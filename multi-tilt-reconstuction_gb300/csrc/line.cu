@@ -126,6 +126,8 @@ __device__ __forceinline__ int line_origin(const LineBase& b, float& xf, int& xi
 struct Walk {
   int pix, dir;        // first detector column relative to the window, direction
   unsigned cross;      // bit z: plane z lies one pixel further than plane z - 1
+  int lane_pix;        // the lane's plane: its detector column relative to the window,
+  float lane_f;        // and its fraction towards the next
 };
 template <int NZ>
 __device__ __forceinline__ Walk lay_out_walk(const LineConst& k, int m, int lane, float4* table) {
@@ -140,6 +142,8 @@ __device__ __forceinline__ Walk lay_out_walk(const LineConst& k, int m, int lane
   const float before = __shfl_up_sync(0xffffffffu, fl, 1);
   w.cross = __ballot_sync(0xffffffffu, lane > 0 && fl != before);
   w.pix = k.base + w.dir * (__float_as_int(__fadd_rn(floorf(u), kMagic)) - kMagicBits);
+  w.lane_pix = k.base + w.dir * (__float_as_int(__fadd_rn(fl, kMagic)) - kMagicBits);
+  w.lane_f = f;
   __syncwarp();
   return w;
 }
@@ -206,23 +210,29 @@ line_forward_kernel(const __grid_constant__ CUtensorMap map, const LineArgs P, c
     }
   } else {
     // lines along Y: the eight columns are eight neighbours in memory; a plane
-    // is read in 32-byte runs and handed to the warps through shared memory
-    float* tile = reinterpret_cast<float*>(win0);  // [BW][9]
+    // is read in 32-byte runs, two planes ahead, and handed to the warps through
+    // one of two shared-memory tiles
     const int tm = tid & 7, tw = tid >> 3;
-#pragma unroll
-    for (int z = 0; z < NZ; ++z) {
-      float t[VL];
+    auto load = [&](int z, float (&t)[VL]) {
 #pragma unroll
       for (int j = 0; j < VL; ++j) {
         t[j] = 0.f;
         const int w = w0 + 32 * j + tw;
-        if (m0 + tm < M && Z0 + z < P.z1 && w < W)
+        if (z < NZ && m0 + tm < M && Z0 + z < P.z1 && w < W)
           t[j] = x ? ldv<VT>(x, (long long)w * sx + (m0 + tm) + (long long)(Z0 + z - P.z0) * sxy) : 1.f;
         vmax = fmaxf(vmax, fabsf(t[j]));
       }
-      if (z > 0) __syncthreads();
+    };
+    float ta[VL], tb[VL];
+    load(0, ta);
+    load(1, tb);
+#pragma unroll
+    for (int z = 0; z < NZ; ++z) {
+      float* tile = reinterpret_cast<float*>(win0) + (z & 1) * BW * 9;  // [BW][9]
+      float(&t)[VL] = z & 1 ? tb : ta;
 #pragma unroll
       for (int j = 0; j < VL; ++j) tile[(32 * j + tw) * 9 + tm] = t[j];
+      load(z + 2, t);
       __syncthreads();
 #pragma unroll
       for (int q = 0; q < VP; ++q)
@@ -296,7 +306,7 @@ line_forward_kernel(const __grid_constant__ CUtensorMap map, const LineArgs P, c
           }
         };
         f32x2 c0[VP], c1[VP];  // sums of the current pixel and the next
-        Weights w = lds_weights(tab);
+        Weights w = lds_weights(tab), next = lds_weights(tab + 16u);  // (a plane ahead of their use)
 #pragma unroll
         for (int p = 0; p < VP; ++p) {
           c0[p] = mul2(w.a, v[0][p]);
@@ -304,7 +314,8 @@ line_forward_kernel(const __grid_constant__ CUtensorMap map, const LineArgs P, c
         }
 #pragma unroll
         for (int z = 1; z < NZ; ++z) {
-          w = lds_weights(tab + 16u * z);
+          w = next;
+          if (z + 1 < NZ) next = lds_weights(tab + 16u * (z + 1));
           if (s.cross & (1u << z)) {  // the column left the pixel
             emit(at, pix, c0);
             at += dstep;
@@ -365,6 +376,12 @@ line_forward_kernel(const __grid_constant__ CUtensorMap map, const LineArgs P, c
 // values leave 3 CTAs per SM, faster than 16 x 4 at two.  512x512x64, 61
 // angles: 0.25 ms against 0.47 ms for the windowed gather; 1024x1024x96, 121
 // angles: 2.5 against 4.9-5.5 ms.
+//
+// The WBP also sums the weights, which separate too: with one row table for all
+// angles, sum_a cx(a, m, z) * cy(w).  Lane z keeps the sum of plane z, one
+// register in place of one per voxel, and the WBP takes the update's shapes:
+// 512x512x64, 61 angles, 0.32 / 0.31 ms (lines along Y / X) against 0.43 / 0.42
+// with a sum per voxel, which only maps with a row table per angle still need.
 struct LineBpArgs {
   LineArgs l;
   LineTab tab;
@@ -377,6 +394,10 @@ struct LineBpArgs {
   int* err;
   unsigned wait_iters;
 };
+
+// Modes of the back-projection: WBP whose line positions keep their detector
+// weight at every angle, SIRT update, WBP with a row table per angle.
+constexpr int kWbp = 0, kSirt = 1, kWbpTables = 2;
 
 // The results of N voxels at offsets i from the brick's first voxel (negative:
 // none): WBP s/c (0 where c is 0), or the SIRT update, whose N loads are all
@@ -393,16 +414,16 @@ __device__ __forceinline__ void finish_voxels(const BrickOut& B, const int (&i)[
   float cv[N], xv[N];
 #pragma unroll
   for (int q = 0; q < N; ++q) {
-    cv[q] = MODE == 0 ? c[q] : i[q] >= 0 ? B.cbp[i[q]] : 0.f;
-    xv[q] = MODE == 0 || i[q] < 0 ? 0.f : B.x[i[q]];
+    cv[q] = MODE != kSirt ? c[q] : i[q] >= 0 ? B.cbp[i[q]] : 0.f;
+    xv[q] = MODE != kSirt || i[q] < 0 ? 0.f : B.x[i[q]];
   }
 #pragma unroll
   for (int q = 0; q < N; ++q) {
     if (i[q] < 0) continue;
     float out = xv[q];
-    if (cv[q] != 0.f) out = MODE == 0 ? s[q] / cv[q] : fmaf(B.step, s[q] / cv[q], out);
-    if (MODE == 0) B.cbp[i[q]] = cv[q];
-    if (MODE == 0 || cv[q] != 0.f) B.x[i[q]] = out;
+    if (cv[q] != 0.f) out = MODE != kSirt ? s[q] / cv[q] : fmaf(B.step, s[q] / cv[q], out);
+    if (MODE != kSirt) B.cbp[i[q]] = cv[q];
+    if (MODE != kSirt || cv[q] != 0.f) B.x[i[q]] = out;
     if (B.copy_kind == 1) static_cast<__nv_bfloat16*>(B.copy)[i[q]] = __float2bfloat16_rn(out);
     else if (B.copy_kind == 2) static_cast<__half*>(B.copy)[i[q]] = __float2half_rn(out);
   }
@@ -411,7 +432,7 @@ __device__ __forceinline__ void finish_voxels(const BrickOut& B, const int (&i)[
 __host__ __device__ constexpr size_t bp_table_bytes(int nz) { return (size_t)kWarps * nz * sizeof(float4); }
 
 template <int MODE, int VL, int NZ>
-__global__ void __launch_bounds__(kBpThreads, VL * NZ >= 64 || (MODE == 0 && VL * NZ >= 32) ? 2 : VL * NZ >= 32 || MODE == 0 ? 3 : 4)
+__global__ void __launch_bounds__(kBpThreads, VL * NZ >= 64 || (MODE == kWbpTables && VL * NZ >= 32) ? 2 : VL * NZ >= 32 || MODE == kWbpTables ? 3 : 4)
 line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int BW = 32 * VL;
@@ -479,30 +500,27 @@ line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
 
   // value pair q of a lane: line positions w0 + 64 q + 2 lane and the next one
   f32x2 acc[NZ][VP];
-  float c[MODE == 0 ? NZ : 1][MODE == 0 ? VL : 1];  // WBP: weight sums
+  constexpr bool kTables = MODE == kWbpTables;
+  float c[kTables ? NZ : 1][kTables ? VL : 1];  // weight sums with a row table per angle
+  float csum = 0.f;  // with a shared one: the sum over the angles of the x weights of plane `lane`
 #pragma unroll
   for (int z = 0; z < NZ; ++z) {
 #pragma unroll
     for (int q = 0; q < VP; ++q) acc[z][q] = 0ull;
-    if (MODE == 0) {
+    if (kTables) {
 #pragma unroll
-      for (int q = 0; q < VL; ++q) c[z][q] = 0.f;
+      for (int q = 0; q < VL; ++q) c[kTables ? z : 0][kTables ? q : 0] = 0.f;
     }
   }
-  float cy[MODE == 0 ? VL : 1], call[MODE == 0 ? VL : 1];  // detector weights along y; sums of columns wholly inside
+  float cy[VL];  // WBP: detector weights along y of the lane's line positions
   auto load_weights = [&](int a) {
     const float* wt = P.tab.weight + (long long)a * P.tab.stride * P.Wp;
 #pragma unroll
     for (int q = 0; q < VL; ++q) {
       const int w = w0 + 64 * (q >> 1) + 2 * lane + (q & 1);
-      cy[MODE == 0 ? q : 0] = w < W ? __ldg(wt + w) : 0.f;
+      cy[q] = w < W ? __ldg(wt + w) : 0.f;
     }
   };
-  if (MODE == 0) {
-    load_weights(0);
-#pragma unroll
-    for (int q = 0; q < VL; ++q) call[MODE == 0 ? q : 0] = 0.f;
-  }
 #pragma unroll 1
   for (int a = 0; a < A; ++a) {
     const int st = a % kBpStages;
@@ -521,24 +539,19 @@ line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
       p0[q] = lds_pair(at + 256u * q);
       p1[q] = lds_pair(at + dstep + 256u * q);
     }
-    if (MODE == 0) {
-      if (P.tab.stride && a > 0) load_weights(a);
-      int pix = s.pix + k.ox;
-      const int last = pix + s.dir * (__popc(s.cross) + 1);
-      if (min(pix, last) >= 0 && max(pix, last) < L.ax.PX) {
-        // the two x weights of every voxel of the column sum to one
-#pragma unroll
-        for (int q = 0; q < VL; ++q) call[MODE == 0 ? q : 0] += cy[MODE == 0 ? q : 0];
-      } else {
+    if (MODE != kSirt) {
+      // weight of the lane's plane: its two taps where they lie on the detector (both: exactly one)
+      const int p = s.lane_pix + k.ox;
+      const bool in0 = (unsigned)p < (unsigned)L.ax.PX, in1 = (unsigned)(p + s.dir) < (unsigned)L.ax.PX;
+      const float cx = in0 ? (in1 ? 1.f : 1.f - s.lane_f) : in1 ? s.lane_f : 0.f;
+      if (MODE == kWbp) csum += cx;
+      if (kTables) {
+        load_weights(a);
 #pragma unroll
         for (int z = 0; z < NZ; ++z) {
-          if (z > 0 && (s.cross & (1u << z))) pix += s.dir;
-          const float4 w = table[z];
-          const float cx = ((unsigned)pix < (unsigned)L.ax.PX ? w.x : 0.f) +
-                           ((unsigned)(pix + s.dir) < (unsigned)L.ax.PX ? w.z : 0.f);
+          const float t = __shfl_sync(0xffffffffu, cx, z);
 #pragma unroll
-          for (int q = 0; q < VL; ++q)
-            c[MODE == 0 ? z : 0][MODE == 0 ? q : 0] = fmaf(cx, cy[MODE == 0 ? q : 0], c[MODE == 0 ? z : 0][MODE == 0 ? q : 0]);
+          for (int q = 0; q < VL; ++q) c[kTables ? z : 0][kTables ? q : 0] = fmaf(t, cy[q], c[kTables ? z : 0][kTables ? q : 0]);
         }
       }
     }
@@ -560,13 +573,6 @@ line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
     if (lane == 0) mbar_arrive(&empty[st]);
   }
 
-  if (MODE == 0) {
-#pragma unroll
-    for (int z = 0; z < NZ; ++z) {
-#pragma unroll
-      for (int q = 0; q < VL; ++q) c[MODE == 0 ? z : 0][MODE == 0 ? q : 0] += call[MODE == 0 ? q : 0];
-    }
-  }
   __syncthreads();  // every warp is done with the windows, and the producer with its loads
   const int sx = L.vol.NX, sxy = L.vol.NX * L.vol.NY;  // (16 planes stay below 2^31 voxels: plan_lines)
   const long long first = (long long)(Z0 - L.z0) * sxy + (L.along_x ? (long long)m0 * sx + w0 : (long long)w0 * sx + m0);
@@ -574,6 +580,11 @@ line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
                    static_cast<char*>(P.vol_copy) + (P.copy_kind ? 2 * first : 0), P.copy_kind, P.step};
   constexpr int ZB = VL == 4 ? 1 : 2;  // planes per batch: 4 voxels a lane
   const int nz = min(NZ, L.z1 - Z0);
+  if (MODE == kWbp) load_weights(0);
+  auto weight = [&](int z, int q) {  // WBP: weight sum of value q in plane z (every lane calls it)
+    if (kTables) return c[kTables ? z : 0][kTables ? q : 0];
+    return MODE == kWbp ? __shfl_sync(0xffffffffu, csum, z) * cy[q] : 0.f;
+  };
   if (L.along_x) {
     if (m0 + warp >= M) return;
 #pragma unroll
@@ -586,7 +597,7 @@ line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
         const float2 t = unpack2(acc[z][q >> 1]);
         at[e] = z < nz && w0 + w < W ? z * sxy + warp * sx + w : -1;
         sv[e] = q & 1 ? t.y : t.x;
-        cv[e] = c[MODE == 0 ? z : 0][MODE == 0 ? q : 0];
+        cv[e] = weight(z, q);
       }
       finish_voxels<MODE>(B, at, sv, cv);
     }
@@ -602,13 +613,13 @@ line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
       int at[ZB * VL];
       float sv[ZB * VL], cv[ZB * VL];
 #pragma unroll
-      for (int pass = 0; pass < (MODE == 0 ? 2 : 1); ++pass) {
+      for (int pass = 0; pass < (MODE == kSirt ? 1 : 2); ++pass) {
 #pragma unroll
         for (int e = 0; e < ZB * VL; ++e) {
           const int z = zb + e / VL, q = e % VL;
           const float2 t = unpack2(acc[z][q >> 1]);
           tile[(z - zb) * kTile + (64 * (q >> 1) + 2 * lane + (q & 1)) * 9 + warp] =
-              pass ? c[MODE == 0 ? z : 0][MODE == 0 ? q : 0] : q & 1 ? t.y : t.x;
+              pass ? weight(z, q) : q & 1 ? t.y : t.x;
         }
         named_sync(1, kThreads);
 #pragma unroll
@@ -620,7 +631,7 @@ line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
           } else {
             sv[e] = t;
             at[e] = z < nz && w0 + w < W && m0 + tm < M ? z * sxy + w * sx + tm : -1;
-            if (MODE != 0) cv[e] = 0.f;
+            if (MODE == kSirt) cv[e] = 0.f;
           }
         }
         named_sync(1, kThreads);
@@ -745,7 +756,7 @@ size_t rows_smem(int W, int PY) {
 size_t fwd_smem(const LinePlan& p, int angles) {
   return (((size_t)angles * sizeof(LineConst) + 127) & ~(size_t)127) + 128 +
          kWarps * p.fwd_nz * sizeof(float4) + kFwdStages * kMaxRows * sizeof(int) +
-         std::max((size_t)kFwdStages * p.fwd_rows * 32 * p.fwd_vl * 4, (size_t)32 * p.fwd_vl * 9 * 4);
+         std::max((size_t)kFwdStages * p.fwd_rows * 32 * p.fwd_vl * 4, (size_t)2 * 32 * p.fwd_vl * 9 * 4);
 }
 size_t bp_smem(int rows, int vl, int nz, int A) {
   return 128 + (((size_t)A * sizeof(LineConst) + 127) & ~(size_t)127) + bp_table_bytes(nz) +
@@ -787,6 +798,12 @@ cudaError_t run_bp(const CUtensorMap& map, LineBpArgs P, cudaStream_t st) {
   return e;
 }
 
+template <int MODE>
+cudaError_t run_bp_shape(int vl, int nz, const CUtensorMap& map, const LineBpArgs& P, cudaStream_t st) {
+  if (vl == 4) return run_bp<MODE, 4, 8>(map, P, st);
+  return nz == 16 ? run_bp<MODE, 2, 16>(map, P, st) : nz == 8 ? run_bp<MODE, 2, 8>(map, P, st) : run_bp<MODE, 2, 4>(map, P, st);
+}
+
 template <int MODE, typename BT, bool NORM>
 cudaError_t run_rows(const LinePlan& p, const LineTab& tab, const AxisDev& ax, const BT* b, float* sums, float* cf,
                      float* image, double* norm2, cudaStream_t st) {
@@ -814,11 +831,11 @@ cudaError_t launch_line_backproject(const CUtensorMap& map, const LinePlan& p, c
   const LineArgs L{ax, vol, p.along_x, z0, z1, mode == 0 ? p.wbp_rows : p.bp_rows, 1, ax.A};
   const LineBpArgs P{L, tab, p.Wp, step, vol_out, cbp, vol_copy, copy_kind, err, pipeline_wait_limit()};
   if (mode == 0) {
-    if (p.wbp_vl == 4) return run_bp<0, 4, 8>(map, P, st);
-    return p.wbp_nz == 8 ? run_bp<0, 2, 8>(map, P, st) : run_bp<0, 2, 4>(map, P, st);
+    if (p.n_tab == 1) return run_bp_shape<kWbp>(p.wbp_vl, p.wbp_nz, map, P, st);
+    if (p.wbp_vl == 4) return run_bp<kWbpTables, 4, 8>(map, P, st);
+    return p.wbp_nz == 8 ? run_bp<kWbpTables, 2, 8>(map, P, st) : run_bp<kWbpTables, 2, 4>(map, P, st);
   }
-  if (p.bp_vl == 4) return p.bp_nz == 16 ? run_bp<1, 4, 16>(map, P, st) : run_bp<1, 4, 8>(map, P, st);
-  return p.bp_nz == 16 ? run_bp<1, 2, 16>(map, P, st) : p.bp_nz == 8 ? run_bp<1, 2, 8>(map, P, st) : run_bp<1, 2, 4>(map, P, st);
+  return run_bp_shape<kSirt>(p.bp_vl, p.bp_nz, map, P, st);
 }
 
 template <typename BT>
@@ -872,7 +889,7 @@ LinePlan plan_lines(const std::vector<double>& xc, const std::vector<double>& yc
       return (double)((W + 32 * vl - 1) / (32 * vl) * 32 * vl) * ((depth + nz - 1) / nz * nz);
     };
     static const struct { int vl, nz; double fwd, bp, wbp; } kShapes[] = {
-        {4, 16, 1.00, 1.13, 0.}, {4, 8, 1.08, 1.00, 1.00}, {2, 16, 1.12, 1.23, 0.}, {2, 8, 1.41, 1.40, 1.10}};
+        {4, 16, 1.00, 0., 0.}, {4, 8, 1.08, 1.00, 1.00}, {2, 16, 1.12, 1.23, 0.}, {2, 8, 1.41, 1.40, 1.10}};
     double bf = 1e300, bb = 1e300, bw = 1e300;
     p.fwd_vl = p.bp_vl = p.wbp_vl = 2;
     p.fwd_nz = 8;  // (the forward splits the angles of few bricks over more CTAs)
@@ -881,8 +898,16 @@ LinePlan plan_lines(const std::vector<double>& xc, const std::vector<double>& yc
       const double wk = work(sh.vl, sh.nz);
       if (wk * sh.fwd < bf) { bf = wk * sh.fwd; p.fwd_vl = sh.vl; p.fwd_nz = sh.nz; }
       if (ctas(sh.vl, sh.nz) < 2 * sms) continue;
-      if (wk * sh.bp < bb) { bb = wk * sh.bp; p.bp_vl = sh.vl; p.bp_nz = sh.nz; }
+      if (sh.bp > 0 && wk * sh.bp < bb) { bb = wk * sh.bp; p.bp_vl = sh.vl; p.bp_nz = sh.nz; }
       if (sh.wbp > 0 && wk * sh.wbp < bw) { bw = wk * sh.wbp; p.wbp_vl = sh.vl; p.wbp_nz = sh.nz; }
+    }
+    p.n_tab = 1;
+    for (int a = 1; a < A; ++a)
+      for (int c = 0; c < 4; ++c)
+        if (yc[4 * (size_t)a + c] != yc[c]) p.n_tab = A;
+    if (p.n_tab == 1) {  // (a WBP without weight sums to carry: as the SIRT update)
+      p.wbp_vl = p.bp_vl;
+      p.wbp_nz = p.bp_nz;
     }
     auto rows = [&](int nz) {  // detector columns of a brick, at the widest angle
       double e = 0;
@@ -899,10 +924,6 @@ LinePlan plan_lines(const std::vector<double>& xc, const std::vector<double>& yc
            fwd_smem(p, A) <= 100 * 1024 && bp_smem(p.bp_rows, p.bp_vl, p.bp_nz, A) <= 110 * 1024 &&
            bp_smem(p.wbp_rows, p.wbp_vl, p.wbp_nz, A) <= 110 * 1024 && rows_smem(W, PY) <= 200 * 1024;
     if (!p.ok) continue;
-    p.n_tab = 1;
-    for (int a = 1; a < A; ++a)
-      for (int c = 0; c < 4; ++c)
-        if (yc[4 * (size_t)a + c] != yc[c]) p.n_tab = A;
     const int ws = along_x ? vol.Xs : vol.Ys, ms = along_x ? vol.Ys : vol.Xs;
     const size_t nw = (size_t)p.n_tab * p.Wp, ny = (size_t)p.n_tab * PY;
     p.off_rows = 2 * nw;

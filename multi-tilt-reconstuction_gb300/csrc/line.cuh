@@ -25,7 +25,7 @@ struct LinePlan {
   int along_x = 0;        // lines along X (else along Y)
   int W = 0, Wp = 0;      // line length and pitch of a line image's rows
   int fwd_vl = 4, fwd_nz = 16, fwd_rows = 0;  // forward: values per lane, depth, window rows
-  int bp_vl = 4, bp_nz = 16, bp_rows = 0;     // SIRT update
+  int bp_vl = 4, bp_nz = 8, bp_rows = 0;     // SIRT update
   int wbp_vl = 4, wbp_nz = 8, wbp_rows = 0;   // WBP
   int n_tab = 1;          // angles in the row tables (1: the same y-map at every angle)
   // row tables (host), uploaded by the reconstruction as one array:

@@ -93,6 +93,19 @@ def test_lines_equal_windows(ctx, monkeypatch, prec, flags, slab):
     assert rel_l2(got, want) < tol and rel_l2(norms, norms_w) < tol
 
 
+@pytest.mark.parametrize("views", [None, _shift_views], ids=["shared", "shifted"])
+@pytest.mark.parametrize("phi", [0.0, 90.0])
+@pytest.mark.parametrize("shape", ["128x8", "64x16", "64x8"])
+def test_wbp_brick_shapes_match_fp64_oracle(ctx, shape, phi, views):
+    """WBP in every brick shape (the small one: above), one row table or one per
+    angle, with columns that leave the detector on both sides."""
+    w, m, z = {"128x8": (250, 190, 56), "64x16": (190, 208, 64), "64x8": (60, 490, 40)}[shape]
+    vol = (0, m, 0, w, 0, z) if phi == 0.0 else (0, w, 0, m, 0, z)
+    c = _case(vol, int(0.8 * m), w + 8, (-52, -17, 0, 31), phi, 11, views)
+    got = ctx.wbp(c.axes[0], c.vol)
+    assert rel_l2(got, oracle.wbp(oracle.FP64, c.axes[0], c.vol)) < TOL
+
+
 @pytest.mark.parametrize("change", ["lean", "turn", "squeeze", "narrow"])
 def test_axes_that_do_not_separate_keep_the_windows(ctx, change):
     c = _case((0, 40, 0, 48, 0, 12), 56, 56, range(-60, 61, 20), 0.0, 5)
