@@ -200,6 +200,11 @@ mtr_status mtr_wbp(mtr_context* ctx, const mtr_axis* axis, mtr_volume_size vol, 
 mtr_status mtr_sirt(mtr_context* ctx, const mtr_axis* axis, mtr_volume_size vol, int slice_start,
                     int slice_end, int n_inner, float sirt_step, float* slab_inout);
 
+/* mtr_sirt from one host slab into another (or the same), without the copy a
+ * caller that keeps its start would make. */
+mtr_status mtr_sirt_from(mtr_context* ctx, const mtr_axis* axis, mtr_volume_size vol, int slice_start,
+                         int slice_end, int n_inner, float sirt_step, const float* slab_in, float* slab_out);
+
 /* No counterpart in the reference.  The computation of mtr_sirt for callers
  * that cannot allocate device memory where they call it (cudaMalloc and
  * cudaFree synchronise the device and can fail, which a pipeline stage that

@@ -26,8 +26,9 @@ mtr_status check_slab(mtr_context* ctx, const mtr_volume_size& vol, int z0, int 
 // object, which waits for the work that used its arrays.
 struct SlabRecon {
   mtr_recon* r = nullptr;
+  // row_sums: false for a WBP alone, which has no residual
   mtr_status create(mtr_context* ctx, const mtr_axis& axis, const mtr_volume_size& vol, int z0, int z1, int n_inner,
-                    float step) {
+                    float step, bool row_sums) {
     mtr_volume_size sv = vol;
     sv.Zstart = z0;
     sv.Zend = z1;
@@ -39,7 +40,7 @@ struct SlabRecon {
     p.sirt_step = step;
     p.precision = MTR_PREC_FP32;
     p.flags = 0;
-    return mtr_recon_create(ctx, 1, &axis, sv, &p, MTR_MEM_HOST, &r);
+    return recon_create(ctx, 1, &axis, sv, &p, MTR_MEM_HOST, row_sums, &r);
   }
   ~SlabRecon() { mtr_recon_destroy(r); }
 };
@@ -57,11 +58,12 @@ mtr_status mtr_wbp(mtr_context* ctx, const mtr_axis* axis, mtr_volume_size vol, 
   if (s != MTR_OK) return s;
   DeviceGuard g(ctx->device);
   SlabRecon sr;
-  s = sr.create(ctx, *axis, vol, slice_start, slice_end, 0, 0.f);
+  s = sr.create(ctx, *axis, vol, slice_start, slice_end, 0, 0.f, false);
   if (s != MTR_OK) return s;
   mtr_recon* r = sr.r;
   s = recon_enqueue_wbp(r, 0);  // x = s/c, cbp = c over the slab
   if (s != MTR_OK) return s;
+  touch_host_pages(slab_out, (size_t)r->nv * 4);  // while the GPU works
   MTR_CK(ctx, cudaMemcpyAsync(slab_out, r->ax[0].x.p, (size_t)r->nv * 4, cudaMemcpyDeviceToHost, ctx->stream));
   MTR_CK(ctx, cudaStreamSynchronize(ctx->stream));
   return mtr_recon_check(r);
@@ -69,7 +71,12 @@ mtr_status mtr_wbp(mtr_context* ctx, const mtr_axis* axis, mtr_volume_size vol, 
 
 mtr_status mtr_sirt(mtr_context* ctx, const mtr_axis* axis, mtr_volume_size vol, int slice_start, int slice_end,
                     int n_inner, float sirt_step, float* slab_inout) {
-  if (!ctx || !axis || !slab_inout) return set_error(ctx, MTR_ERR_INVALID_ARGUMENT, "null argument");
+  return mtr_sirt_from(ctx, axis, vol, slice_start, slice_end, n_inner, sirt_step, slab_inout, slab_inout);
+}
+
+mtr_status mtr_sirt_from(mtr_context* ctx, const mtr_axis* axis, mtr_volume_size vol, int slice_start, int slice_end,
+                         int n_inner, float sirt_step, const float* slab_in, float* slab_out) {
+  if (!ctx || !axis || !slab_in || !slab_out) return set_error(ctx, MTR_ERR_INVALID_ARGUMENT, "null argument");
   if (n_inner < 0) return set_error(ctx, MTR_ERR_INVALID_ARGUMENT, "negative iteration count");
   mtr_status s = check_volume(ctx, vol);
   if (s == MTR_OK) s = check_axis(ctx, *axis);
@@ -77,7 +84,7 @@ mtr_status mtr_sirt(mtr_context* ctx, const mtr_axis* axis, mtr_volume_size vol,
   if (s != MTR_OK) return s;
   DeviceGuard g(ctx->device);
   SlabRecon sr;
-  s = sr.create(ctx, *axis, vol, slice_start, slice_end, n_inner, sirt_step);
+  s = sr.create(ctx, *axis, vol, slice_start, slice_end, n_inner, sirt_step, true);
   if (s != MTR_OK) return s;
   mtr_recon* r = sr.r;
   // The WBP pass yields the back-projection weight sums C = A^T 1 of the slab
@@ -86,13 +93,14 @@ mtr_status mtr_sirt(mtr_context* ctx, const mtr_axis* axis, mtr_volume_size vol,
   // caller's slab.
   s = recon_enqueue_wbp(r, 0);
   if (s != MTR_OK) return s;
-  MTR_CK(ctx, cudaMemcpyAsync(r->ax[0].x.p, slab_inout, (size_t)r->nv * 4, cudaMemcpyHostToDevice, ctx->stream));
+  MTR_CK(ctx, cudaMemcpyAsync(r->ax[0].x.p, slab_in, (size_t)r->nv * 4, cudaMemcpyHostToDevice, ctx->stream));
   for (int it = 0; it < n_inner; ++it) {
     if ((s = recon_enqueue_forward(r, 0)) != MTR_OK) return s;
     if ((s = recon_enqueue_residual(r, 0)) != MTR_OK) return s;
     if ((s = recon_enqueue_sirt_bp(r, 0)) != MTR_OK) return s;
   }
-  MTR_CK(ctx, cudaMemcpyAsync(slab_inout, r->ax[0].x.p, (size_t)r->nv * 4, cudaMemcpyDeviceToHost, ctx->stream));
+  touch_host_pages(slab_out, (size_t)r->nv * 4);  // while the GPU works
+  MTR_CK(ctx, cudaMemcpyAsync(slab_out, r->ax[0].x.p, (size_t)r->nv * 4, cudaMemcpyDeviceToHost, ctx->stream));
   MTR_CK(ctx, cudaStreamSynchronize(ctx->stream));
   return mtr_recon_check(r);
 }

@@ -444,7 +444,13 @@ namespace mtr {
 mtr_status recon_enqueue_forward_span(mtr_recon* r, int k, const VolSpan& sp);
 // mode 0 WBP, 1 SIRT update; widen: widen FP16 projections for a windowed WBP first.
 mtr_status recon_enqueue_bp_span(mtr_recon* r, int k, int mode, const VolSpan& sp, bool widen);
+// mtr_recon_create; row_sums false leaves out the forward row sums, for an
+// object that is only back-projected (no residual).
+mtr_status recon_create(mtr_context* ctx, int n_axes, const mtr_axis* axes, mtr_volume_size vol,
+                        const mtr_params* params, int mem_kind, bool row_sums, mtr_recon** out);
 mtr_status recon_enqueue_widen(mtr_recon* r, int k);
+// Makes a host array's pages resident ahead of a copy into it (contents kept).
+void touch_host_pages(void* p, size_t bytes);
 // Residual of axis k; norm: FP64 sum of r^2 (null: not recorded).
 mtr_status recon_enqueue_residual_norm(mtr_recon* r, int k, double* norm);
 // Where the squared residual norm of (outer it, axis k, inner j) is recorded, or null.

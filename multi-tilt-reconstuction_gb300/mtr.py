@@ -129,6 +129,7 @@ _SIGNATURES = {
     "mtr_context_profile_reset": (C.c_int, [_P]),
     "mtr_wbp": (C.c_int, [_P, C.POINTER(AxisC), VolumeSize, C.c_int, C.c_int, _P]),
     "mtr_sirt": (C.c_int, [_P, C.POINTER(AxisC), VolumeSize, C.c_int, C.c_int, C.c_int, C.c_float, _P]),
+    "mtr_sirt_from": (C.c_int, [_P, C.POINTER(AxisC), VolumeSize, C.c_int, C.c_int, C.c_int, C.c_float, _P, _P]),
     "mtr_sirt_noalloc": (C.c_int, [_P, ProjectionSize, _P, _P, _P, VolumeSize, C.c_int, C.c_int, C.c_int, C.c_float,
                                    _P]),
     "mtr_initial_z": (C.c_int, [_P, VolumeSize, _P, _P, _P]),
@@ -329,7 +330,7 @@ class Context:
     def wbp(self, axis: AxisData, vol: VolumeSize, z0: int | None = None, z1: int | None = None) -> np.ndarray:
         z0 = vol.Zstart if z0 is None else z0
         z1 = vol.Zend if z1 is None else z1
-        out = np.zeros((z1 - z0, vol.Y, vol.X), np.float32)
+        out = np.empty((z1 - z0, vol.Y, vol.X), np.float32)  # (written whole)
         a = axis.c_struct()
         self.check(self.lib.mtr_wbp(self.h, C.byref(a), vol, z0, z1, _ptr(out)), "mtr_wbp")
         return out
@@ -337,9 +338,11 @@ class Context:
     def sirt(self, axis: AxisData, vol: VolumeSize, slab: np.ndarray, n_inner=10, step=0.5, z0=None, z1=None):
         z0 = vol.Zstart if z0 is None else z0
         z1 = vol.Zend if z1 is None else z1
-        out = np.ascontiguousarray(slab, dtype=np.float32).copy()
+        start = np.ascontiguousarray(slab, dtype=np.float32)
+        out = np.empty(start.shape, np.float32)
         a = axis.c_struct()
-        self.check(self.lib.mtr_sirt(self.h, C.byref(a), vol, z0, z1, n_inner, step, _ptr(out)), "mtr_sirt")
+        self.check(self.lib.mtr_sirt_from(self.h, C.byref(a), vol, z0, z1, n_inner, step, _ptr(start), _ptr(out)),
+                   "mtr_sirt")
         return out
 
     def initial_z(self, vol: VolumeSize, w: np.ndarray, wavg: np.ndarray) -> np.ndarray:
