@@ -371,6 +371,7 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
     kc[a] = k;
   }
   __syncthreads();
+  stream_wait();
 
   if (warp == kConsumerWarps) {
     // ---------------- producer warp: one elected lane issues the TMA loads
@@ -639,7 +640,7 @@ cudaError_t launch_one(const CUtensorMap& map, const BpArgs& P, size_t smem, cud
   if (e != cudaSuccess) return e;
   constexpr int BX = bp_brick_x(LANES, PAIR), BY = bp_brick_y(LANES, PAIR);
   const dim3 grid((P.vol.NX + BX - 1) / BX, (P.z1 - P.z0 + NZ - 1) / NZ, (P.vol.NY + BY - 1) / BY);
-  kern<<<grid, kThreads, smem, st>>>(map, P);
+  launch_overlapped(kern, grid, kThreads, smem, st, map, P);
   const cudaError_t le = cudaGetLastError();
   if (le == cudaSuccess) g_windowed_launches.fetch_add(1, std::memory_order_relaxed);
   return le;

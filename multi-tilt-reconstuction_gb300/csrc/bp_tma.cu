@@ -96,8 +96,8 @@ cudaError_t launch_backproject_batch(const BpBatchDesc* descs, const long long* 
                                      size_t smem, int grid, int* err, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(bp_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  bp_batch_kernel<<<grid, kThreads, smem, st>>>(descs, first, n_desc, n_items, err,
-                                                 g_wait_iters.load(std::memory_order_relaxed));
+  launch_overlapped(bp_batch_kernel, grid, kThreads, smem, st, descs, first, n_desc, n_items, err,
+                                           g_wait_iters.load(std::memory_order_relaxed));
   const cudaError_t le = cudaGetLastError();
   if (le == cudaSuccess) g_windowed_launches.fetch_add(1, std::memory_order_relaxed);
   return le;

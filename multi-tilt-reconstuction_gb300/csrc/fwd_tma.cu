@@ -291,7 +291,7 @@ __device__ __forceinline__ void prefix_brick(const CUtensorMap* smap, const FwdA
   float vmax = 0.f;
   {
     const long long sx = P.vol.NX, sxy = (long long)P.vol.NX * P.vol.NY;
-    const long long base = (long long)(X0 + tx - P.vol.Xs) + (long long)(Y0 + ty - P.vol.Ys) * sx;
+    const long long base = (long long)(X0 + tx - P.vol.Xs) + (long long)(Y0 + ty - P.vol.Ys) * sx + stream_wait();
     const int c0 = NZ >> 1;
     float s0 = 0.f, s1 = 0.f;
     pre[0] = make_float2(0.f, 0.f);
@@ -537,7 +537,7 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
   float vmax = 0.f;
   {
     const long long sx = P.vol.NX, sxy = (long long)P.vol.NX * P.vol.NY;
-    const long long base = (long long)(X0 + tx - P.vol.Xs) + (long long)(Y0 + ty - P.vol.Ys) * sx;
+    const long long base = (long long)(X0 + tx - P.vol.Xs) + (long long)(Y0 + ty - P.vol.Ys) * sx + stream_wait();
 #pragma unroll
     for (int z = 0; z < NZ; ++z) {
       const int zz = Z0 + z;
@@ -652,7 +652,7 @@ cudaError_t launch_one(const CUtensorMap& map, FwdArgs P, int lanes, int num_sms
   const size_t smem = fwd_smem(P.WX, P.WY, P.nz, NZ == 0, P.max_angles);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<dim3(b3.x, b3.y, b3.z * groups), kThreads, smem, st>>>(map, P, lanes);
+  launch_overlapped(kern, dim3(b3.x, b3.y, b3.z * groups), kThreads, smem, st, map, P, lanes);
   const cudaError_t le = cudaGetLastError();
   if (le == cudaSuccess) g_windowed_launches.fetch_add(1, std::memory_order_relaxed);
   return le;
@@ -715,7 +715,7 @@ cudaError_t launch_forward_batch(const FwdBatchDesc* descs, const long long* fir
                                  size_t smem, int grid, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(fwd_batch_kernel<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  fwd_batch_kernel<VT><<<grid, kThreads, smem, st>>>(descs, first, n_desc, n_items);
+  launch_overlapped(fwd_batch_kernel<VT>, grid, kThreads, smem, st, descs, first, n_desc, n_items);
   const cudaError_t le = cudaGetLastError();
   if (le == cudaSuccess) g_windowed_launches.fetch_add(1, std::memory_order_relaxed);
   return le;

@@ -189,12 +189,13 @@ line_forward_kernel(const __grid_constant__ CUtensorMap map, const LineArgs P, c
   const int W = P.along_x ? P.vol.NX : P.vol.NY, M = P.along_x ? P.vol.NY : P.vol.NX;
   const long long sx = P.vol.NX, sxy = (long long)P.vol.NX * P.vol.NY;
 
+  const long long after = stream_wait();  // (added to the loads' index)
   // own voxels: value j of a lane is line position w0 + 32 j + lane
   f32x2 v[NZ][VP];
   float vmax = 0.f;
   if (P.along_x) {
     const bool col = m0 + warp < M;
-    const long long base = (long long)(m0 + warp) * sx + w0 + lane;
+    const long long base = (long long)(m0 + warp) * sx + w0 + lane + after;
 #pragma unroll
     for (int z = 0; z < NZ; ++z) {
       float t[VL];
@@ -219,7 +220,7 @@ line_forward_kernel(const __grid_constant__ CUtensorMap map, const LineArgs P, c
         t[j] = 0.f;
         const int w = w0 + 32 * j + tw;
         if (z < NZ && m0 + tm < M && Z0 + z < P.z1 && w < W)
-          t[j] = x ? ldv<VT>(x, (long long)w * sx + (m0 + tm) + (long long)(Z0 + z - P.z0) * sxy) : 1.f;
+          t[j] = x ? ldv<VT>(x, (long long)w * sx + (m0 + tm) + after + (long long)(Z0 + z - P.z0) * sxy) : 1.f;
         vmax = fmaxf(vmax, fabsf(t[j]));
       }
     };
@@ -472,6 +473,7 @@ line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
     kc[a] = k;
   }
   __syncthreads();
+  stream_wait();
 
   if (warp == kWarps) {  // producer: one elected lane issues the loads
     if (lane == 0) {
@@ -666,6 +668,10 @@ line_rows_kernel(AxisDev ax, int W, int Wp, LineTab tab, const BT* __restrict__ 
   const int2* span = tab.span + (long long)a * tab.stride * ax.PY;
   double acc = 0.0;
   for (int w = threadIdx.x; w < W; w += 256) trow[w] = __ldg(row + w);
+  const long long after = stream_wait();
+  b += after;
+  sums += after;
+  cf += after;
   if (MODE != 2) {
     if (x0 + warp < ax.PX) {
       float* src = sums + ((long long)a * ax.PX + x0 + warp) * Wp;
@@ -777,7 +783,7 @@ cudaError_t run_forward(const CUtensorMap& map, const LinePlan& p, LineArgs L, c
   const size_t smem = fwd_smem(p, L.max_angles);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<dim3(gx, gy, gz * groups), kThreads, smem, st>>>(map, L, x);
+  launch_overlapped(kern, dim3(gx, gy, gz * groups), kThreads, smem, st, map, L, x);
   e = cudaGetLastError();
   if (e == cudaSuccess) g_windowed_launches.fetch_add(1, std::memory_order_relaxed);
   return e;
@@ -792,7 +798,7 @@ cudaError_t run_bp(const CUtensorMap& map, LineBpArgs P, cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const dim3 grid((W + 32 * VL - 1) / (32 * VL), (L.z1 - L.z0 + NZ - 1) / NZ, (M + kWarps - 1) / kWarps);
-  kern<<<grid, kBpThreads, smem, st>>>(map, P);
+  launch_overlapped(kern, grid, kBpThreads, smem, st, map, P);
   e = cudaGetLastError();
   if (e == cudaSuccess) g_windowed_launches.fetch_add(1, std::memory_order_relaxed);
   return e;
@@ -811,7 +817,8 @@ cudaError_t run_rows(const LinePlan& p, const LineTab& tab, const AxisDev& ax, c
   const size_t smem = rows_smem(p.W, ax.PY);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  kern<<<dim3((ax.PX + kCols - 1) / kCols, ax.A), 256, smem, st>>>(ax, p.W, p.Wp, tab, b, sums, cf, image, norm2);
+  launch_overlapped(kern, dim3((ax.PX + kCols - 1) / kCols, ax.A), 256, smem, st, ax, p.W, p.Wp, tab, b, sums, cf, image,
+                    norm2);
   return cudaGetLastError();
 }
 

@@ -18,6 +18,7 @@
 #include <type_traits>
 
 #include "mtr_internal.h"
+#include "tma.cuh"
 
 namespace mtr {
 namespace {
@@ -340,6 +341,10 @@ residual_pairs_kernel(long long rows, int pitch, int pitch2, const BT* __restric
                       const float* __restrict__ c, float* __restrict__ rp, double* __restrict__ norm2) {
   const int lane = threadIdx.x & 31;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long after = stream_wait();
+  b += after;
+  s += after;
+  c += after;
   double acc = 0.0;
   for (long long row = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; row < rows; row += nwarps) {
     const float sq = residual_pair_row<BT, FORM>(b + row * pitch, s + row * pitch, c + row * pitch,
@@ -431,6 +436,10 @@ row_pairs_kernel(int A, int PY, int pitch, int pp, const BT* __restrict__ b, flo
                  const float* __restrict__ c, float* __restrict__ out, double* __restrict__ norm2) {
   const int lane = threadIdx.x & 31, nb = blocks_of(pp), ns = strips_of(PY);
   const long long items = (long long)A * ns * nb, nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long after = stream_wait();
+  b += after;
+  s += after;
+  c += after;
   double acc = 0.0;
   for (long long it = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; it < items; it += nwarps) {
     const int xb = (int)(it % nb), st = (int)(it / nb % ns), a = (int)(it / nb / ns);
@@ -453,23 +462,24 @@ row_pairs_kernel(int A, int PY, int pitch, int pp, const BT* __restrict__ b, flo
 // Residual over many axes: item = (descriptor, 64 strips, 8 per warp).
 constexpr int kStripsPerItem = 64;
 template <typename BT>
-__device__ __forceinline__ void residual_batch_item(const ResBatchDesc& D, int first) {
+__device__ __forceinline__ void residual_batch_item(const ResBatchDesc& D, int first, long long after) {
   const int lane = threadIdx.x & 31, nb = blocks_of(D.pp), ns = strips_of(D.PY);
   const int end = min(first + kStripsPerItem, D.A * ns * nb);
   for (int it = first + (int)(threadIdx.x >> 5); it < end; it += 8) {
     const int xb = it % nb, st = it / nb % ns, a = it / nb / ns;
-    row_pair_strip<BT, false>(static_cast<const BT*>(D.b), D.s, D.cf, D.r, D.PY, D.pitch, D.pp, a, st * kStripRows,
-                              128 * xb + 4 * lane);
+    row_pair_strip<BT, false>(static_cast<const BT*>(D.b) + after, D.s + after, D.cf + after, D.r, D.PY, D.pitch, D.pp,
+                              a, st * kStripRows, 128 * xb + 4 * lane);
   }
 }
 template <bool HALF_B>
 __global__ void __launch_bounds__(256)
 residual_batch_kernel(const ResBatchDesc* __restrict__ descs, const long long* __restrict__ first, int n_desc,
                       long long n_items) {
+  const long long after = stream_wait();
   for (long long it = blockIdx.x; it < n_items; it += gridDim.x) {
     const int2 item = work_item(first, n_desc, it);
-    if (HALF_B) residual_batch_item<__half>(descs[item.x], item.y * kStripsPerItem);
-    else residual_batch_item<float>(descs[item.x], item.y * kStripsPerItem);
+    if (HALF_B) residual_batch_item<__half>(descs[item.x], item.y * kStripsPerItem, after);
+    else residual_batch_item<float>(descs[item.x], item.y * kStripsPerItem, after);
   }
 }
 
@@ -526,9 +536,9 @@ void launch_row_pairs(int mode, const AxisDev& ax, const BT* b, float* s, const 
   const long long warps = (long long)ax.A * strips_of(ax.PY) * blocks_of(pp);
   // grid-stride over the rest
   const unsigned g = (unsigned)std::max(1LL, std::min((warps + 7) / 8, (long long)device_sm_count() * 16));
-  if (mode == 1) row_pairs_kernel<BT, true, false><<<g, 256, 0, st>>>(ax.A, ax.PY, ax.pitch, pp, b, s, c, out, nullptr);
-  else if (norm2) row_pairs_kernel<BT, false, true><<<g, 256, 0, st>>>(ax.A, ax.PY, ax.pitch, pp, b, s, c, out, norm2);
-  else row_pairs_kernel<BT, false, false><<<g, 256, 0, st>>>(ax.A, ax.PY, ax.pitch, pp, b, s, c, out, nullptr);
+  if (mode == 1) launch_overlapped(row_pairs_kernel<BT, true, false>, g, 256, 0, st, ax.A, ax.PY, ax.pitch, pp, b, s, c, out, nullptr);
+  else if (norm2) launch_overlapped(row_pairs_kernel<BT, false, true>, g, 256, 0, st, ax.A, ax.PY, ax.pitch, pp, b, s, c, out, norm2);
+  else launch_overlapped(row_pairs_kernel<BT, false, false>, g, 256, 0, st, ax.A, ax.PY, ax.pitch, pp, b, s, c, out, nullptr);
 }
 template void launch_row_pairs<float>(int, const AxisDev&, const float*, float*, const float*, float*, double*,
                                       cudaStream_t);
@@ -537,8 +547,8 @@ template void launch_row_pairs<__half>(int, const AxisDev&, const __half*, float
 
 void launch_residual_batch(const ResBatchDesc* descs, const long long* first, int n_desc, long long n_items, int half_b,
                            int grid, cudaStream_t st) {
-  if (half_b) residual_batch_kernel<true><<<grid, 256, 0, st>>>(descs, first, n_desc, n_items);
-  else residual_batch_kernel<false><<<grid, 256, 0, st>>>(descs, first, n_desc, n_items);
+  if (half_b) launch_overlapped(residual_batch_kernel<true>, grid, 256, 0, st, descs, first, n_desc, n_items);
+  else launch_overlapped(residual_batch_kernel<false>, grid, 256, 0, st, descs, first, n_desc, n_items);
 }
 
 template <typename BT>
@@ -550,14 +560,14 @@ void launch_residual_pairs(long long rows, int pitch, int pitch2, const BT* b, f
   if (blocks < 1) blocks = 1;
   const unsigned g = (unsigned)blocks;
   if (form == 2) {
-    if (norm2) residual_pairs_kernel<BT, true, 2><<<g, 256, 0, st>>>(rows, pitch, pitch2, b, s, c, rp, norm2);
-    else residual_pairs_kernel<BT, false, 2><<<g, 256, 0, st>>>(rows, pitch, pitch2, b, s, c, rp, nullptr);
+    if (norm2) launch_overlapped(residual_pairs_kernel<BT, true, 2>, g, 256, 0, st, rows, pitch, pitch2, b, s, c, rp, norm2);
+    else launch_overlapped(residual_pairs_kernel<BT, false, 2>, g, 256, 0, st, rows, pitch, pitch2, b, s, c, rp, nullptr);
   } else if (form == 1) {
-    if (norm2) residual_pairs_kernel<BT, true, 1><<<g, 256, 0, st>>>(rows, pitch, pitch2, b, s, c, rp, norm2);
-    else residual_pairs_kernel<BT, false, 1><<<g, 256, 0, st>>>(rows, pitch, pitch2, b, s, c, rp, nullptr);
+    if (norm2) launch_overlapped(residual_pairs_kernel<BT, true, 1>, g, 256, 0, st, rows, pitch, pitch2, b, s, c, rp, norm2);
+    else launch_overlapped(residual_pairs_kernel<BT, false, 1>, g, 256, 0, st, rows, pitch, pitch2, b, s, c, rp, nullptr);
   } else {
-    if (norm2) residual_pairs_kernel<BT, true, 0><<<g, 256, 0, st>>>(rows, pitch, pitch2, b, s, c, rp, norm2);
-    else residual_pairs_kernel<BT, false, 0><<<g, 256, 0, st>>>(rows, pitch, pitch2, b, s, c, rp, nullptr);
+    if (norm2) launch_overlapped(residual_pairs_kernel<BT, true, 0>, g, 256, 0, st, rows, pitch, pitch2, b, s, c, rp, norm2);
+    else launch_overlapped(residual_pairs_kernel<BT, false, 0>, g, 256, 0, st, rows, pitch, pitch2, b, s, c, rp, nullptr);
   }
 }
 
