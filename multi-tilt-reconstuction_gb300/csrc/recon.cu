@@ -654,8 +654,11 @@ mtr_status mtr::recon_create(mtr_context* ctx, int n_axes, const mtr_axis* axes,
       MTR_CK(ctx, cudaMemsetAsync(a.b.p, 0, (size_t)a.np * pe, ctx->stream));
     }
     // Line kernels where the maps separate, else TMA-windowed kernels where the
-    // window geometry fits (else the plain kernels run).
-    if (!tma_disabled() && !windows_forced()) {
+    // window geometry fits (else the plain kernels run).  Volumes in mapped host
+    // memory stay with the windows, whose deeper bricks cross the host link in
+    // fewer, longer runs (512x512x128 in FP16, 61 angles, WBP and two iterations:
+    // 22.4 ms, line kernels 29.9 at 0 degrees; 22.5 and 26.1 at 90).
+    if (!tma_disabled() && !windows_forced() && (!hv || streamed)) {
       s = setup_lines(r.get(), a, streamed ? r->slabs->depth : r->vol.NZ);
       if (s != MTR_OK) return s;
     }

@@ -126,3 +126,13 @@ def test_axes_that_do_not_separate_keep_the_windows(ctx, change):
     r.run()
     want = oracle.reconstruct(oracle.FP64, [mtr.AxisData(x, y, d)], c.vol, 1, 2, 0.5, 0.7)
     assert rel_l2(r.download(), want) < 1e-4
+
+
+@pytest.mark.parametrize("phi", [0.0, 90.0])
+def test_volumes_in_host_memory_keep_the_windows(ctx, phi):
+    c = _case((0, 40, 0, 48, 0, 12), 56, 56, range(-60, 61, 20), phi, 6)
+    p = mtr.params(1, 2, 0.5, 0.7, mtr.PREC_FP32, mtr.FLAG_HOST_VOLUMES)
+    r = mtr.Recon(ctx, c.axes, c.vol, p)
+    assert r.describe()[0]["back_projection"]["window_format"] != "line image"
+    r.run()
+    assert rel_l2(r.download(), oracle.reconstruct(oracle.FP64, c.axes, c.vol, 1, 2, 0.5, 0.7)) < TOL
