@@ -52,15 +52,17 @@ CONFIGS = {
 }
 
 
-# Per-launch DRAM traffic and instruction count of the dominant kernel, from
-# the ncu captures summarised in profiles/ (one launch of axis 0).
+# Per-launch DRAM traffic of the dominant kernel and use of the resource that
+# binds it, from the ncu captures summarised in profiles/ (one launch of the
+# axis at 60 degrees; `count` per clock and SM against `per_clk`).
 NCU_PROFILES = {
-    ("c2", "backproject"): {"traffic": 390_982_656 + 167_104_768, "warp_inst": 828_349_812,
-                            "duration_ms": 0.937248, "sm_ghz": 2.070, "sms": 152,
+    ("c2", "backproject"): {"traffic": 486_389_760, "resource": "instruction issue", "unit": "warp-instructions/s",
+                            "count": 1_278_589_418, "per_clk": 4, "duration_ms": 1.178944, "sm_ghz": 2.064,
+                            "sms": 152, "warp_inst": 1_278_589_418,
                             "source": "profiles/bp_tma_kernel_3axis_512x512x128.md"},
-    ("c2", "forward"): {"traffic": 128_399_104 + 40_043_008, "warp_inst": 1_279_387_488,
-                        "duration_ms": 1.282304, "sm_ghz": 2.047, "sms": 152,
-                        "source": "profiles/fwd_tma_kernel_3axis_512x512x128.md"},
+    ("c2", "forward"): {"traffic": 167_595_264, "resource": "shared-memory wavefronts", "unit": "wavefronts/s",
+                        "count": 338_130_462, "per_clk": 1, "duration_ms": 1.322816, "sm_ghz": 2.068, "sms": 152,
+                        "warp_inst": 1_181_442_990, "source": "profiles/fwd_tma_kernel_3axis_512x512x128.md"},
 }
 
 
@@ -822,14 +824,12 @@ def main() -> int:
                 "avg_launch_ms": per_launch_ms, "launches": n_l,
                 "kernel_share": {k: prof[k][1] / max(sum(x[1] for x in prof.values()), 1e-9) for k in prof}}
         if ncu:
-            # the roof that binds is instruction issue; figures of the captured
-            # launch (axis 0) against 4 issue slots per SM per clock
-            issue_peak = ncu["sms"] * 4 * ncu["sm_ghz"] * 1e9
-            inst_rate = ncu["warp_inst"] / (ncu["duration_ms"] * 1e-3)
-            roof["binding"] = {"resource": "instruction issue", "achieved": inst_rate, "peak": issue_peak,
-                               "unit": "warp-instructions/s", "frac": inst_rate / issue_peak,
+            peak = ncu["sms"] * ncu["per_clk"] * ncu["sm_ghz"] * 1e9
+            rate = ncu["count"] / (ncu["duration_ms"] * 1e-3)
+            roof["binding"] = {"resource": ncu["resource"], "achieved": rate, "peak": peak, "unit": ncu["unit"],
+                               "frac": rate / peak,
                                "warp_inst_per_voxel_angle": ncu["warp_inst"] / cfg_voxel_angles(cfg),
-                               "launch": "axis 0 (ncu)", "source": ncu["source"]}
+                               "launch": "axis at 60 degrees (ncu)", "source": ncu["source"]}
         vu = r["vu"] * world
         value = replica_value(r["vu"], world, r["ms"])
         line = {

@@ -5,10 +5,11 @@
 // with global float atomics (FunctionOnGPU.cu:27-52, 316-333): eight atomics
 // per voxel and angle, contending along every ray.  Here one CTA owns a
 // brick of BX x BY x NZ voxels for the whole launch (prefix sums in shared
-// memory, or voxels in registers where the y-map has a Z term).  For each of its angles it splats the brick into a private detector window in
-// shared memory, then one thread flushes the window into the ray-sum array
-// with a single 3-D tiled cp.reduce.async.bulk.tensor add (the L2 reduces
-// whole sectors).  Three window stages rotate: the flush of one angle
+// memory, or voxels in registers where the y-map has a Z term).  For each of
+// its angles it splats the brick into a private detector window in shared
+// memory, then one thread flushes the window into the ray-sum array with a
+// single 3-D tiled cp.reduce.async.bulk.tensor add (the L2 reduces whole
+// sectors).  Three window stages rotate: the flush of one angle
 // overlaps the splat of the next, and the stage after it is zeroed during the
 // conversion pass, so an angle costs two block barriers.
 //

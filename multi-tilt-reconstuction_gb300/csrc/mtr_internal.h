@@ -129,7 +129,7 @@ struct BpPlan {
   bool bz0 = false;    // y map independent of Z for every angle
   int WX = 0, WY = 0;  // window box (elements)
   int align = 2;       // TMA x alignment (elements)
-  int nz = 8;          // brick depth (voxels per thread along Z): 4, 8 or 16
+  int nz = 8;          // brick depth (voxels per thread along Z): 4, 8, 16 or 32
   bool pairs = false;  // windows of pairs along x (SIRT update) rather than row pairs
   bool planar = false; // pairs as two FP32 planes per row (values, differences) instead of interleaved
   bool half = false;   // pairs as FP16 (value, difference) in 32 bits (mixed precision)
