@@ -60,13 +60,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 // stream_wait() it reads only its arguments and tables that were copied to the
 // device and writes nothing in global memory; every thread that touches other
 // data comes through the wait, which ends when the kernels before it have
-// completed and what they wrote is visible.  It returns a zero that the compiler
-// cannot see; the pointers of the read-only loads that follow take it as an
-// offset, so that none of those loads moves above the wait.  The CTAs are not let in any earlier
-// (griddepcontrol.launch_dependents): those of a small grid then crowd on the
-// SMs that empty first (10 SIRT iterations at 128x128x32: 0.72 against 0.60 ms).
-// What it hides is the launch itself, 1-2 us of each: 256x256x64, 61 angles, 10
-// iterations 2.01 -> 1.94 ms; two leaning axes of 192x160x48 1.68 -> 1.65 ms.
+// completed and what they wrote is visible.  It returns a zero that the
+// compiler cannot see; the pointers of the read-only loads that follow take it
+// as an offset, so that none of those loads moves above the wait.  The CTAs are
+// not let in any earlier (griddepcontrol.launch_dependents): those of a small
+// grid then crowd on the SMs that empty first (10 SIRT iterations at
+// 128x128x32: 0.72 against 0.60 ms).  What it hides is the launch itself, 1-2 us
+// of each: 256x256x64, 61 angles, 8 iterations 2.01 -> 1.94 ms; two leaning axes
+// of 192x160x48 1.68 -> 1.65 ms.
 __device__ __forceinline__ long long stream_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   long long zero = 0;
