@@ -339,7 +339,11 @@ class Context:
         z0 = vol.Zstart if z0 is None else z0
         z1 = vol.Zend if z1 is None else z1
         start = np.ascontiguousarray(slab, dtype=np.float32)
+        n = (z1 - z0) * vol.Y * vol.X  # the planes read and written; what follows them is kept
+        if start.size < n:
+            raise ValueError(f"sirt: the slab holds {start.size} values, planes {z0} to {z1} need {n}")
         out = np.empty(start.shape, np.float32)
+        out.reshape(-1)[max(n, 0):] = start.reshape(-1)[max(n, 0):]
         a = axis.c_struct()
         self.check(self.lib.mtr_sirt_from(self.h, C.byref(a), vol, z0, z1, n_inner, step, _ptr(start), _ptr(out)),
                    "mtr_sirt")
