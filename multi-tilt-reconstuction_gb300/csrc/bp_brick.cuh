@@ -58,6 +58,9 @@ struct __align__(16) WinConst {
 // the angle is skipped and the launch flagged); every tap lies on the detector.
 constexpr int kHolds = 1, kOnDetector = 2;
 
+// A fractional base that the clamp to +-1e9 px left large: the position is
+// beyond what its integer part and the windows' float arithmetic hold.
+__device__ __forceinline__ bool far(float f) { return !(fabsf(f) <= 65536.f); }
 __device__ __forceinline__ int floor_div(int a, int b) { return (a >= 0) ? a / b : -((-a + b - 1) / b); }
 
 __device__ __forceinline__ int magic_int(float integral) { return __float_as_int(__fadd_rn(integral, kMagic)); }
@@ -365,7 +368,8 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
       // first and last tap, with a pixel of slack for the rounding of a thread's own position
       const int x0 = xi + (int)floorf(xmin) - 1, x1 = xi + (int)floorf(xmax) + 2;
       const int y0 = yi + (int)floorf(ymin) - 1, y1 = yi + (int)floorf(ymax) + 2;
-      if (x0 >= ox && x1 < ox + P.WX && y0 >= oy && y1 <= oy + P.WY) k.flags |= kHolds;
+      // (far(): integers and positions beyond their range say nothing about the window)
+      if (!far(k.xf) && !far(k.yf) && x0 >= ox && x1 < ox + P.WX && y0 >= oy && y1 <= oy + P.WY) k.flags |= kHolds;
       if (x0 >= 0 && x1 < P.ax.PX && y0 >= 0 && y1 < P.ax.PY) k.flags |= kOnDetector;
     }
     kc[a] = k;

@@ -880,6 +880,15 @@ LinePlan plan_lines(const std::vector<double>& xc, const std::vector<double>& yc
             std::fabs(cy[cw]) >= 0.5 && std::fabs(cy[cw]) <= 2.0 && std::fabs(cx[cm]) <= 4.0 &&
             std::fabs(cx[3]) < 0.999 && std::fabs(cx[0]) < 1e9 && std::fabs(cy[0]) < 1e9;
     }
+    // (positions stay within the integers and floats that the kernels index with)
+    const double m0 = along_x ? vol.Ys : vol.Xs, w0 = along_x ? vol.Xs : vol.Ys;
+    for (int a = 0; a < A && sep; ++a)
+      for (int c = 0; c < 8 && sep; ++c) {
+        const double* cx = &xc[4 * (size_t)a];
+        const double x = cx[0] + cx[cw] * (w0 + (c & 1 ? W : 0)) + cx[cm] * (m0 + (c & 2 ? M : 0)) +
+                         cx[3] * ((double)vol.Zs + (c & 4 ? vol.NZ : 0));
+        sep = std::fabs(x) < 9e8;
+      }
     if (!sep) continue;
     p.along_x = along_x;
     p.W = W;
