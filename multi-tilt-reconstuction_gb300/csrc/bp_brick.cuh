@@ -368,8 +368,13 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
       // first and last tap, with a pixel of slack for the rounding of a thread's own position
       const int x0 = xi + (int)floorf(xmin) - 1, x1 = xi + (int)floorf(xmax) + 2;
       const int y0 = yi + (int)floorf(ymin) - 1, y1 = yi + (int)floorf(ymax) + 2;
+      // The window's rows are the extent's ceiling and three more (a pixel of slack
+      // below, the last pixel's row, a pixel above), as the host planned them, which
+      // no rounding of the two ends decides: ymin and ymax rounded apart reach a row
+      // further where the extent is whole and the fraction a few 1e-7 below one.
+      const double ey = fabs(cy[1]) * (BX - 1) + fabs(cy[2]) * (BY - 1) + fabs(cy[3]) * (NZ - 1);
       // (far(): integers and positions beyond their range say nothing about the window)
-      if (!far(k.xf) && !far(k.yf) && x0 >= ox && x1 < ox + P.WX && y0 >= oy && y1 <= oy + P.WY) k.flags |= kHolds;
+      if (!far(k.xf) && !far(k.yf) && x0 >= ox && x1 < ox + P.WX && (int)ceil(ey - 1e-9) + 3 <= P.WY) k.flags |= kHolds;
       if (x0 >= 0 && x1 < P.ax.PX && y0 >= 0 && y1 < P.ax.PY) k.flags |= kOnDetector;
     }
     kc[a] = k;
