@@ -152,7 +152,7 @@ struct __align__(16) PreConst {  // per-angle constants of a brick
   float xf, a1, a2, a3;   // (|a3| at least 1e-7: 2e-6 px over a column)
   float yf, b1, b2, inv;  // inv = 1 / a3
   int lxm, lym;           // window-local integer base minus the magic bits
-  int nx;                 // pixel boundaries that every column crosses: floor(|a3| (depth - 1)); negative: no column splats
+  int nx;                 // pixel boundaries that every column crosses: floor(|a3| (depth - 1))
   float scale;            // fixed-point scale of this angle (power of two)
   int ox, oy;             // window origin (clamped inside the detector, ox aligned)
   int wlx;                // valid window columns; negative where every tap is valid (window not clamped)
@@ -358,8 +358,12 @@ __device__ __forceinline__ void prefix_brick(const CUtensorMap* smap, const FwdA
     k.wlx = interior ? -1 : max(0, min(WX, P.ax.PX - k.ox));
     k.nx = (int)(st * (float)(NZ - 1));
     // A base that the clamp to +-1e9 px left large: no tap near the detector, and
-    // its float positions index neither the prefix sums nor the window.
-    if (!(fabsf(k.xf) <= 65536.f && fabsf(k.yf) <= 65536.f)) k.nx = -1;
+    // its float positions must index neither the prefix sums nor the window.  The
+    // columns walk from zero instead, over no valid window column.
+    if (!(fabsf(k.xf) <= 65536.f && fabsf(k.yf) <= 65536.f)) {
+      k.xf = k.yf = 0.f;
+      k.wlx = 0;
+    }
     // S = 2^(b-e) with max |v| < 2^e, so |v S| < 2^b.  A pixel receives at most
     // the weight w = min(depth, 1 + 1/slope) <= 2^lw from one column:
     // |addition| < 2^(b + lw) <= 2^21, the range of the magic rounding.  A
@@ -381,7 +385,7 @@ __device__ __forceinline__ void prefix_brick(const CUtensorMap* smap, const FwdA
     const int st = j % kStages;
     int* wi = reinterpret_cast<int*>(win0 + st * stage_bytes);
     const PreConst k = kc[j];  // (a copy: the adds order memory)
-    if (active && k.nx >= 0) {
+    if (active) {
       const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
       const float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
       const float fly = floorf(yr);
