@@ -165,6 +165,11 @@ __device__ __forceinline__ f32x2 lds_pair(uint32_t a) {
   asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
   return v;
 }
+__device__ __forceinline__ float lds_float(uint32_t a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+  return v;
+}
 __device__ __forceinline__ float2 sub2(f32x2 a, f32x2 b) {  // a - b in one packed instruction
   f32x2 r;
   float2 d;
@@ -264,10 +269,40 @@ __device__ __forceinline__ void splat_column(uint32_t pre, int nz, uint32_t row,
   if (last != end) add(Off<8>{}, k.a3 * before);
 }
 
+// The same column voxel by voxel: its values are the differences of the prefix
+// sums, its four taps are added one by one.  A pixel costs splat_column 14
+// instructions and 4-6 shared wavefronts, a voxel costs this 20 and 6-10, so it
+// takes the slopes of kSteep pixels per voxel and more (detectors finer than the
+// volume): 256x256x64, 61 angles, 45 degrees, 3 and 4 pixels per voxel, 0.60 and
+// 0.85 ms against 0.66 and 1.02 (0.60 and 0.86 from 1.3 and from 2.0).
+constexpr float kSteep = 1.6f;
+template <bool CHK>
+__device__ __forceinline__ void splat_voxels(uint32_t pre, int nz, uint32_t row, uint32_t drow, float xr,
+                                             const PreConst& k, float wy0, float wy1, uint32_t span, bool y0ok,
+                                             bool y1ok) {
+  float prev = 0.f;
+#pragma unroll 4
+  for (int z = 0; z < nz; ++z) {
+    pre += kPreStride;
+    const float s = lds_float(pre), v = s - prev;
+    prev = s;
+    const float x = fmaf(k.a3, (float)z, xr);
+    const float t = __fadd_rd(x, kMagic);  // floor, in the low bits
+    const float fx = x - (t - kMagic);
+    const uint32_t at = row + 4u * (uint32_t)(__float_as_int(t) + k.lxm), at1 = at + drow;
+    const float v1 = fx * v, v0 = v - v1;
+    const bool x0ok = !CHK || at - row < span, x1ok = !CHK || at + 4u - row < span;
+    if (x0ok && (!CHK || y0ok)) red_shared_at<0>(at, fixq(wy0, v0));
+    if (x1ok && (!CHK || y0ok)) red_shared_at<4>(at, fixq(wy0, v1));
+    if (x0ok && (!CHK || y1ok)) red_shared_at<0>(at1, fixq(wy1, v0));
+    if (x1ok && (!CHK || y1ok)) red_shared_at<4>(at1, fixq(wy1, v1));
+  }
+}
+
 // One brick (bx, by, zb) and angle group g of one axis whose y-map has no Z
 // term; `smem` is the CTA's dynamic shared memory.  On return every bulk
-// reduce it issued is complete.
-template <typename VT>
+// reduce it issued is complete.  STEEP: some angles may reach kSteep.
+template <typename VT, bool STEEP>
 __device__ __forceinline__ void prefix_brick(const CUtensorMap* smap, const FwdArgs& P, int lanes, int bx, int by,
                                              int zb, int g, unsigned char* smem) {
   const int BX = brick_x(lanes), BY = brick_y(lanes), NZ = P.nz;
@@ -393,7 +428,13 @@ __device__ __forceinline__ void prefix_brick(const CUtensorMap* smap, const FwdA
       const int rowi = magic_int(fly) + k.lym;
       const uint32_t rowa = smem_u32(wi) + 4u * (uint32_t)(rowi * WX);
       const float wy0 = (1.f - fy) * k.scale, wy1 = fy * k.scale;
-      if (k.wlx < 0)
+      if (STEEP && fabsf(k.a3) >= kSteep) {
+        if (k.wlx < 0)
+          splat_voxels<false>(pre_a, NZ, rowa, 4u * (uint32_t)WX, xr, k, wy0, wy1, 0u, true, true);
+        else
+          splat_voxels<true>(pre_a, NZ, rowa, 4u * (uint32_t)WX, xr, k, wy0, wy1, 4u * (uint32_t)k.wlx,
+                             (unsigned)rowi < (unsigned)WY, (unsigned)(rowi + 1) < (unsigned)WY);
+      } else if (k.wlx < 0)
         splat_column<false>(pre_a, NZ, rowa, 4u * (uint32_t)WX, xr, k, wy0, wy1, 0u, true, true);
       else
         splat_column<true>(pre_a, NZ, rowa, 4u * (uint32_t)WX, xr, k, wy0, wy1, 4u * (uint32_t)k.wlx,
@@ -626,13 +667,15 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
 }
 
 // One CTA per (brick, angle group) of one axis.  NZ: the depth of the voxel
-// walk (z-dependent y-maps), or 0 for the prefix sums, whose depth is P.nz.
+// walk (z-dependent y-maps), or for the prefix sums, whose depth is P.nz, 0, or
+// kSteepAxis with the voxel by voxel path (which costs the others 0.5 %).
+constexpr int kSteepAxis = -1;
 template <typename VT, int NZ>
 __global__ void __launch_bounds__(kThreads)
 fwd_tma_kernel(const __grid_constant__ CUtensorMap smap, const __grid_constant__ FwdArgs P, int lanes) {
   extern __shared__ __align__(128) unsigned char smem[];
-  if constexpr (NZ == 0)
-    prefix_brick<VT>(&smap, P, lanes, blockIdx.x, blockIdx.y, blockIdx.z / P.groups, blockIdx.z % P.groups, smem);
+  if constexpr (NZ <= 0)
+    prefix_brick<VT, NZ == kSteepAxis>(&smap, P, lanes, blockIdx.x, blockIdx.y, blockIdx.z / P.groups, blockIdx.z % P.groups, smem);
   else
     fwd_brick<VT, NZ>(&smap, P, lanes, blockIdx.x, blockIdx.y, blockIdx.z / P.groups, blockIdx.z % P.groups, smem);
 }
@@ -657,7 +700,7 @@ cudaError_t launch_one(const CUtensorMap& map, FwdArgs P, int lanes, int num_sms
   if (groups < 1) groups = 1;
   P.groups = groups;
   P.max_angles = (P.ax.A + groups - 1) / groups;
-  const size_t smem = fwd_smem(P.WX, P.WY, P.nz, NZ == 0, P.max_angles);
+  const size_t smem = fwd_smem(P.WX, P.WY, P.nz, NZ <= 0, P.max_angles);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   launch_overlapped(kern, dim3(b3.x, b3.y, b3.z * groups), kThreads, smem, st, map, P, lanes);
@@ -697,7 +740,7 @@ fwd_batch_kernel(const FwdBatchDesc* __restrict__ descs, const long long* __rest
       sB[4] = D.lanes * 2 + D.bz0;
     }
     __syncthreads();
-    if (sB[4] & 1) prefix_brick<VT>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
+    if (sB[4] & 1) prefix_brick<VT, true>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
     else if (sB[3] == 8) fwd_brick<VT, 8>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
     else if (sB[3] == 32) fwd_brick<VT, 32>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
     else fwd_brick<VT, 16>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
@@ -754,6 +797,8 @@ FwdPlan plan_forward_uncached(const std::vector<double>& xc, const std::vector<d
   // lane: -1 heuristic (lines along X or Y), 0 lines along X, 1 along Y, 2 8x4 patches
   p.lanes = lane < 0 ? (sy > sx ? 1 : 0) : std::min(lane, 2);
   p.bz0 = bz0;
+  for (int a = 0; a < A; ++a)
+    if (std::fabs((float)xc[4 * a + 3]) >= kSteep) p.steep = true;
   p.nz = nz;
   const int BX = brick_x(p.lanes), BY = brick_y(p.lanes), BZ = p.nz;
   double ex = 0, ey = 0;
@@ -815,6 +860,7 @@ cudaError_t launch_forward_tma(const CUtensorMap& smap, const FwdPlan& plan, con
                                const VT* x, int z0, int z1, cudaStream_t st) {
   const int sms = device_sm_count();
   const FwdArgs P{ax, vol, z0, z1, plan.WX, plan.WY, 1, ax.A, plan.mass_shift, plan.nz, x};
+  if (plan.bz0 && plan.steep) return launch_one<VT, kSteepAxis>(smap, P, plan.lanes, sms, st);
   if (plan.bz0) return launch_one<VT, 0>(smap, P, plan.lanes, sms, st);
   if (plan.nz == 8) return launch_one<VT, 8>(smap, P, plan.lanes, sms, st);
   if (plan.nz == 32) return launch_one<VT, 32>(smap, P, plan.lanes, sms, st);

@@ -1,0 +1,51 @@
+"""Reconstructions with several detector pixels per voxel (binned volumes) against
+the FP64 oracle."""
+import numpy as np
+import pytest
+
+import mtr
+import oracle
+import phantom
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+# positions to ~4e-6 px, sums in fixed point at 2^-17 of a brick's largest value
+# or finer: the bounds of the windowed kernels' tests
+TOL = {mtr.PREC_FP32: 1e-4, mtr.PREC_MIXED_FP16: 1e-3}
+
+
+def binned(mag, phi, vol=(2, 47, -3, 36, 0, 21), lean=0.0, cover=1.1, seed=4):
+    """One axis whose detector has `mag` pixels to a voxel and covers the volume `cover` times."""
+    v = mtr.VolumeSize.make(*vol)
+    px = int(mag * cover * max(v.X, v.Y)) + 8
+    c = phantom.make_case(v, px, np.arange(-60.0, 61.0, 15.0), [phi], 5, "gaussian", 0.02, seed, axis_cls=mtr.AxisData,
+                          py=px + 3)
+    a = c.axes[0]
+    mid = np.array([(v.Xstart + v.Xend - 1) / 2, (v.Ystart + v.Yend - 1) / 2, (v.Zstart + v.Zend - 1) / 2])
+    maps = []
+    for q, n in ((a.x_coef, px), (a.y_coef, px + 3)):
+        m = q.reshape(-1, 4).copy()
+        m[:, 1:] *= mag
+        if q is a.y_coef:
+            m[:, 3] += lean
+        m[:, 0] = (n + 1) / 2 - m[:, 1:] @ mid
+        maps.append(m.ravel())
+    return v, [mtr.AxisData(maps[0], maps[1], a.data)]
+
+
+def check(ctx, v, axes, prec=mtr.PREC_FP32, **kw):
+    r = mtr.Recon(ctx, axes, v, mtr.params(1, 2, 0.5, 0.7, prec, **kw))
+    r.run()
+    want = oracle.reconstruct(oracle.FP64, axes, v, 1, 2, 0.5, 0.7)
+    assert rel_l2(r.download(), want) < TOL[prec]
+    return r.describe()[0]
+
+
+@pytest.mark.parametrize("depths", ["8,8,0,0,0", "8,16,1,1,0", "8,32,2,2,0", "8,5,0,2,0"])
+@pytest.mark.parametrize("mag,cover", [(1.7, 1.1), (2.5, 0.7), (4.0, 1.1)])
+@pytest.mark.parametrize("phi", [30.0, 135.0])
+def test_steep_columns_match_oracle(ctx, monkeypatch, depths, phi, mag, cover):
+    """Slopes from zero to 3.5 pixels per voxel of both signs, windows inside and at the detector's edges."""
+    monkeypatch.setenv("MTR_FORCE_DEPTHS", depths)
+    check(ctx, *binned(mag, phi, cover=cover))
