@@ -103,7 +103,7 @@ mtr_status mtr::build_sirt_tables(mtr_context* ctx, const std::vector<mtr_recon*
       const bool bp_ok = a.tma && !tma_disabled() && bp.lanes != 2 && !bp.pairs && bp.nz <= 16 &&
                          (long long)bgx * bgy * ((v.NZ + bp.nz - 1) / bp.nz) <
                              (long long)kOwnWaves * ctx->num_sms * backproject_batch_ctas_per_sm(bp.smem);
-      const bool fwd_ok = a.ftma && !tma_disabled() &&
+      const bool fwd_ok = a.ftma && !tma_disabled() && !fp.rows &&
                           (long long)fgx * fgy * ((v.NZ + fp.nz - 1) / fp.nz) <
                               (long long)kOwnWaves * ctx->num_sms * forward_ctas_per_sm(ck, fp.smem);
       if (a.lines || !bp_ok || !fwd_ok) {  // the whole SIRT chain of this axis runs on its own launches

@@ -5,7 +5,8 @@
 // with global float atomics (FunctionOnGPU.cu:27-52, 316-333): eight atomics
 // per voxel and angle, contending along every ray.  Here one CTA owns a
 // brick of BX x BY x NZ voxels for the whole launch (prefix sums in shared
-// memory, or voxels in registers where the y-map has a Z term).  For each of
+// memory, or voxels in registers where the y-map has a Z term or a warp sums
+// rows of its own).  For each of
 // its angles it splats the brick into a private detector window in shared
 // memory, then one thread flushes the window into the ray-sum array with a
 // single 3-D tiled cp.reduce.async.bulk.tensor add (the L2 reduces whole
@@ -524,9 +525,96 @@ __device__ __forceinline__ void stream_column_zy(uint32_t win, int WX, int WY, c
   emit1(at + dstep, X1);
 }
 
+// ---- rows shared by a warp: voxel by voxel into one row ---------------------------
+//
+// Axes along a volume axis whose columns are too steep for the line kernels: the
+// lanes of a warp share their two detector rows and weights, so the warp sums its
+// columns into one row of its own, which is split over the two detector rows once
+// per angle.  The columns stay in registers; prefix sums would take the shared
+// memory that the wide windows of such an axis need (one CTA an SM against three).
+//
+// One column (fixed X, Y) whose x moves by |a3| < 1 per voxel, upwards in z and
+// where a3 < 0 in the mirrored coordinate u = -x, from fraction fx of the pixel at
+// shared address `at`: a pixel is emitted when the column has left it.  L > 1
+// (slope below 1 / L): a chunk of L voxels crosses one boundary at most, so it
+// accumulates without a branch.  S is the weight not yet emitted, a1 its part on
+// the next pixel; inside a chunk the fraction runs on past 1, and C collects
+// (f - 1) v of the voxels beyond the crossing, which moves them to their true
+// pixels when the chunk ends.
+template <int NZ, int L, typename Emit>
+__device__ __forceinline__ void walk_column(const float (&v)[NZ], uint32_t at, uint32_t dstep, float fx, float step,
+                                            const Emit& emit) {
+  float S = v[0], a1 = fx * v[0];
+#pragma unroll
+  for (int z0 = 1; z0 < NZ; z0 += L) {
+    float C = 0.f;
+#pragma unroll
+    for (int j = 0; j < L; ++j) {
+      if (z0 + j < NZ) {
+        fx += step;
+        S += v[z0 + j];
+        a1 = fmaf(fx, v[z0 + j], a1);
+        C = fmaf(__saturatef(fx - 1.f), v[z0 + j], C);
+      }
+    }
+    if (fx >= 1.f) {
+      emit(at, (S - a1) + C);
+      S = a1 - C;
+      a1 = C;
+      fx -= 1.f;
+      at += dstep;
+    }
+  }
+  emit(at, S - a1);
+  emit(at + dstep, a1);
+}
+// One column at any slope, with the longest chunk its slope allows.
+template <int NZ, typename Emit>
+__device__ __forceinline__ void splat_walk(const float (&v)[NZ], uint32_t row, float xr, float a3, int lxm,
+                                           const Emit& emit) {
+  const float st = fabsf(a3);
+  if (st < 0.999f) {
+    const float u = a3 >= 0.f ? xr : -xr;
+    const float fl = floorf(u);
+    const int p = magic_int(fl) - kMagicBits;
+    const uint32_t at = row + 4u * (uint32_t)((lxm + kMagicBits) + (a3 >= 0.f ? p : -p));
+    const uint32_t dstep = a3 >= 0.f ? 4u : 0xFFFFFFFCu;
+    if (st < 0.2499f) walk_column<NZ, 4>(v, at, dstep, u - fl, st, emit);
+    else if (st < 0.4999f) walk_column<NZ, 2>(v, at, dstep, u - fl, st, emit);
+    else walk_column<NZ, 1>(v, at, dstep, u - fl, st, emit);
+    return;
+  }
+#pragma unroll
+  for (int z = 0; z < NZ; ++z) {
+    const float x = fmaf(a3, (float)z, xr);
+    const float t = __fadd_rd(x, kMagic);  // floor, in the low bits
+    const float fx = x - (t - kMagic);
+    const uint32_t at = row + 4u * (uint32_t)(__float_as_int(t) + lxm);
+    const float v1 = fx * v[z];
+    emit(at, v[z] - v1);
+    emit(at + 4u, v1);
+  }
+}
+// Adds the warp's row of WX fixed-point sums (to 24 bits) to the two detector rows
+// at `row` with weights 1 - fy and fy, and zeroes it.
+__device__ __forceinline__ void split_row(int* urow, int WX, uint32_t row, float fy) {
+  __syncwarp();
+  for (int i = threadIdx.x & 31; i < WX; i += 32) {
+    const int q = urow[i];
+    if (q != 0) {
+      const float f = (float)q;
+      red_shared(row + 4u * (uint32_t)i, __float2int_rn((1.f - fy) * f));
+      red_shared(row + 4u * (uint32_t)(WX + i), __float2int_rn(fy * f));
+      urow[i] = 0;
+    }
+  }
+  __syncwarp();
+}
+
 // One brick (bx, by, zb) and angle group g of one axis; `smem` is the CTA's
 // dynamic shared memory.  On return every bulk reduce it issued is complete.
-template <typename VT, int NZ>
+// ROWS: the lanes of a warp share their rows at every angle.
+template <typename VT, int NZ, bool ROWS>
 __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs& P, int lanes, int bx, int by, int zb, int g,
                                           unsigned char* smem) {
   const int BX = brick_x(lanes), BY = brick_y(lanes);
@@ -539,6 +627,8 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
   float* red = reinterpret_cast<float*>(smem + kc_bytes);  // 32 floats for the block max
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  int* urow = reinterpret_cast<int*>(win0 + kStages * stage_bytes) + warp * WX;  // kept zero between uses
+  for (int i = lane; ROWS && i < WX; i += 32) urow[i] = 0;
   const int A = P.ax.A;
   const int a_begin = (int)((long long)A * g / P.groups), a_end = (int)((long long)A * (g + 1) / P.groups);
   const int na = a_end - a_begin;
@@ -624,7 +714,26 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
     const int st = j % kStages;
     int* wi = reinterpret_cast<int*>(win0 + st * stage_bytes);
     const FwdConst k = kc[j];
-    if (active && fabsf(k.a3) < 0.999f && fabsf(k.b3) < 0.999f) {
+    if constexpr (ROWS) {
+      const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
+      const float yr = lanes == 1 ? fmaf(k.b1, (float)tx, k.yf) : fmaf(k.b2, (float)ty, k.yf);  // (the warp's)
+      const float fly = floorf(yr);
+      const float fy = yr - fly;
+      const int rowi = magic_int(fly) + k.lym;
+      const uint32_t row = smem_u32(wi) + 4u * (uint32_t)(rowi * WX);
+      if (k.interior) {
+        if (active) splat_walk<NZ>(v, smem_u32(urow), xr, k.a3, k.lxm, [](uint32_t q, float e) { red_shared(q, fixq(1.f, e)); });
+        split_row(urow, WX, row, fy);
+      } else if (active) {  // clamped at the detector edge: taps off it are dropped
+        const uint32_t span = 4u * (uint32_t)k.wlx, drow = 4u * (uint32_t)WX;
+        const bool y0ok = (unsigned)rowi < (unsigned)WY, y1ok = (unsigned)(rowi + 1) < (unsigned)WY;
+        splat_walk<NZ>(v, row, xr, k.a3, k.lxm, [&](uint32_t q, float e) {
+          const bool xok = q - row < span;
+          if (xok && y0ok) red_shared(q, fixq(1.f - fy, e));
+          if (xok && y1ok) red_shared(q + drow, fixq(fy, e));
+        });
+      }
+    } else if (active && fabsf(k.a3) < 0.999f && fabsf(k.b3) < 0.999f) {
       const float xr = fmaf(k.a2, (float)ty, fmaf(k.a1, (float)tx, k.xf));
       const float yr = fmaf(k.b2, (float)ty, fmaf(k.b1, (float)tx, k.yf));
       if (k.interior) stream_column_zy<NZ, false>(smem_u32(wi), WX, WY, v, xr, yr, k);
@@ -670,27 +779,28 @@ __device__ __forceinline__ void fwd_brick(const CUtensorMap* smap, const FwdArgs
 // walk (z-dependent y-maps), or for the prefix sums, whose depth is P.nz, 0, or
 // kSteepAxis with the voxel by voxel path (which costs the others 0.5 %).
 constexpr int kSteepAxis = -1;
-template <typename VT, int NZ>
+template <typename VT, int NZ, bool ROWS>
 __global__ void __launch_bounds__(kThreads)
 fwd_tma_kernel(const __grid_constant__ CUtensorMap smap, const __grid_constant__ FwdArgs P, int lanes) {
   extern __shared__ __align__(128) unsigned char smem[];
   if constexpr (NZ <= 0)
     prefix_brick<VT, NZ == kSteepAxis>(&smap, P, lanes, blockIdx.x, blockIdx.y, blockIdx.z / P.groups, blockIdx.z % P.groups, smem);
   else
-    fwd_brick<VT, NZ>(&smap, P, lanes, blockIdx.x, blockIdx.y, blockIdx.z / P.groups, blockIdx.z % P.groups, smem);
+    fwd_brick<VT, NZ, ROWS>(&smap, P, lanes, blockIdx.x, blockIdx.y, blockIdx.z / P.groups, blockIdx.z % P.groups, smem);
 }
 
 // Dynamic shared memory: per-angle constants, block-max scratch, window stages
-// and, where the y-map has no Z term, the columns' prefix sums.
-size_t fwd_smem(int WX, int WY, int nz, bool bz0, int angles) {
+// and the columns' prefix sums or (rows) a row per warp.
+size_t fwd_smem(int WX, int WY, int nz, bool prefix, bool rows, int angles) {
   const size_t stage = (((size_t)WX * WY * 4) + 127) & ~(size_t)127;
-  const size_t k = (size_t)angles * (bz0 ? sizeof(PreConst) : sizeof(FwdConst));
-  return ((k + 127) & ~(size_t)127) + 128 + kStages * stage + (bz0 ? (size_t)(nz + 1) * kPreStride : 0);
+  const size_t k = (size_t)angles * (prefix ? sizeof(PreConst) : sizeof(FwdConst));
+  return ((k + 127) & ~(size_t)127) + 128 + kStages * stage + (prefix ? (size_t)(nz + 1) * kPreStride : 0) +
+         (rows ? (size_t)kWarps * WX * 4 : 0);
 }
 
-template <typename VT, int NZ>
+template <typename VT, int NZ, bool ROWS = false>
 cudaError_t launch_one(const CUtensorMap& map, FwdArgs P, int lanes, int num_sms, cudaStream_t st) {
-  auto kern = fwd_tma_kernel<VT, NZ>;
+  auto kern = fwd_tma_kernel<VT, NZ, ROWS>;
   const int BX = brick_x(lanes), BY = brick_y(lanes);
   const dim3 b3((P.vol.NX + BX - 1) / BX, (P.vol.NY + BY - 1) / BY, (P.z1 - P.z0 + P.nz - 1) / P.nz);
   const long long bricks = (long long)b3.x * b3.y * b3.z;
@@ -700,7 +810,7 @@ cudaError_t launch_one(const CUtensorMap& map, FwdArgs P, int lanes, int num_sms
   if (groups < 1) groups = 1;
   P.groups = groups;
   P.max_angles = (P.ax.A + groups - 1) / groups;
-  const size_t smem = fwd_smem(P.WX, P.WY, P.nz, NZ <= 0, P.max_angles);
+  const size_t smem = fwd_smem(P.WX, P.WY, P.nz, NZ <= 0, ROWS, P.max_angles);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   launch_overlapped(kern, dim3(b3.x, b3.y, b3.z * groups), kThreads, smem, st, map, P, lanes);
@@ -741,9 +851,9 @@ fwd_batch_kernel(const FwdBatchDesc* __restrict__ descs, const long long* __rest
     }
     __syncthreads();
     if (sB[4] & 1) prefix_brick<VT, true>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
-    else if (sB[3] == 8) fwd_brick<VT, 8>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
-    else if (sB[3] == 32) fwd_brick<VT, 32>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
-    else fwd_brick<VT, 16>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
+    else if (sB[3] == 8) fwd_brick<VT, 8, false>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
+    else if (sB[3] == 32) fwd_brick<VT, 32, false>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
+    else fwd_brick<VT, 16, false>(sMap, sP, sB[4] >> 1, sB[0], sB[1], sB[2], 0, smem);
   }
 }
 
@@ -784,6 +894,11 @@ template cudaError_t launch_forward_batch<__half>(const FwdBatchDesc*, const lon
 
 namespace {
 
+// Largest z slope from which an axis along a volume axis sums rows per warp (those
+// below 0.999 run on lines): at 1.04, 1.30, 1.73, 2.6 and 3.5 pixels per voxel
+// (256x256x64, 61 angles) 0.200, 0.188, 0.186, 0.219 and 0.303 ms against 0.172,
+// 0.203, 0.245, 0.331 and 0.455 over prefix sums.
+constexpr double kRowsSlope = 1.2;
 FwdPlan plan_forward_uncached(const std::vector<double>& xc, const std::vector<double>& yc, int A, int PX, int PY,
                               int pitch, int nz, int lane) {
   FwdPlan p;
@@ -800,6 +915,14 @@ FwdPlan plan_forward_uncached(const std::vector<double>& xc, const std::vector<d
   for (int a = 0; a < A; ++a)
     if (std::fabs((float)xc[4 * a + 3]) >= kSteep) p.steep = true;
   p.nz = nz;
+  // the rows are the warp's own (their y moves by less than 1e-6 px along the lanes)
+  double top = 0.0;
+  p.rows = bz0 && p.lanes != 2 && (nz == 8 || nz == 16 || nz == 32);
+  for (int a = 0; a < A; ++a) {
+    top = std::max(top, std::fabs(xc[4 * a + 3]));
+    if (!(std::fabs(yc[4 * a + (p.lanes == 1 ? 2 : 1)]) < 3e-8)) p.rows = false;
+  }
+  if (!(top >= kRowsSlope)) p.rows = false;
   const int BX = brick_x(p.lanes), BY = brick_y(p.lanes), BZ = p.nz;
   double ex = 0, ey = 0;
   for (int a = 0; a < A; ++a) {
@@ -810,7 +933,7 @@ FwdPlan plan_forward_uncached(const std::vector<double>& xc, const std::vector<d
   }
   const int wx_min = ((int)std::ceil(ex) + 4 + 4 + 3) / 4 * 4;
   p.WY = (int)std::ceil(ey) + 4;
-  auto smem_for = [&](int WX) { return fwd_smem(WX, p.WY, p.nz, bz0, A); };  // (one angle group)
+  auto smem_for = [&](int WX) { return fwd_smem(WX, p.WY, p.nz, bz0 && !p.rows, p.rows, A); };  // (one angle group)
   // Row pitch (= box width) with the fewest shared-memory bank conflicts of
   // the warp's splat atomics, searched over a few widths only: a wider window
   // leaves the interior fast path at more bricks near the detector edge.
@@ -860,6 +983,11 @@ cudaError_t launch_forward_tma(const CUtensorMap& smap, const FwdPlan& plan, con
                                const VT* x, int z0, int z1, cudaStream_t st) {
   const int sms = device_sm_count();
   const FwdArgs P{ax, vol, z0, z1, plan.WX, plan.WY, 1, ax.A, plan.mass_shift, plan.nz, x};
+  if (plan.rows) {
+    if (plan.nz == 8) return launch_one<VT, 8, true>(smap, P, plan.lanes, sms, st);
+    if (plan.nz == 32) return launch_one<VT, 32, true>(smap, P, plan.lanes, sms, st);
+    return launch_one<VT, 16, true>(smap, P, plan.lanes, sms, st);
+  }
   if (plan.bz0 && plan.steep) return launch_one<VT, kSteepAxis>(smap, P, plan.lanes, sms, st);
   if (plan.bz0) return launch_one<VT, 0>(smap, P, plan.lanes, sms, st);
   if (plan.nz == 8) return launch_one<VT, 8>(smap, P, plan.lanes, sms, st);

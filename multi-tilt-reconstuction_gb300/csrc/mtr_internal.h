@@ -190,6 +190,7 @@ struct FwdPlan {
   int lanes = 0;       // warp layout: 0 lines along X, 1 lines along Y, 2 8x4 patches
   bool bz0 = false;
   int WX = 0, WY = 0;
+  bool rows = false;   // the lanes of a warp share their detector rows: summed in a row per warp
   bool steep = false;  // x moves by several pixels a voxel at some angle
   int mass_shift = 0;  // log2 bound of a pixel's weight from one brick
   int nz = 16;         // brick depth: 8, 16 or 32; up to 32 where the y-map has no Z term
