@@ -28,7 +28,7 @@ NVCC_FLAGS = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-Wall", "-Wno-unused-function", "-I", str(INCLUDE)]
 
 CU_SOURCES = ["projector.cu", "bp_tma.cu", "fwd_tma.cu", "mace.cu", "api.cu", "recon.cu", "entry.cu", "ref64.cu",
-              "noalloc.cu", "tune.cu", "batch.cu", "serve.cu", "mrc_device.cu", "stream.cu", "bp_pairs.cu", "line.cu"]
+              "noalloc.cu", "tune.cu", "batch.cu", "serve.cu", "mrc_device.cu", "stream.cu", "bp_pairs.cu", "bp_rows.cu", "line.cu"]
 CXX_SOURCES = ["mrc_io.cpp", "options.cpp", "geometry.cpp"]
 
 

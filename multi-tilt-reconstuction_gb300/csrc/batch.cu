@@ -100,7 +100,7 @@ mtr_status mtr::build_sirt_tables(mtr_context* ctx, const std::vector<mtr_recon*
       const int fgy = (v.NY + brick_y(fp.lanes) - 1) / brick_y(fp.lanes);
       // the persistent kernels take lines along X or Y over FP32 windows,
       // depths up to 16, of small axes
-      const bool bp_ok = a.tma && !tma_disabled() && bp.lanes != 2 && !bp.pairs && bp.nz <= 16 &&
+      const bool bp_ok = a.tma && !tma_disabled() && bp.lanes != 2 && !bp.pairs && !bp.rows && bp.nz <= 16 &&
                          (long long)bgx * bgy * ((v.NZ + bp.nz - 1) / bp.nz) <
                              (long long)kOwnWaves * ctx->num_sms * backproject_batch_ctas_per_sm(bp.smem);
       const bool fwd_ok = a.ftma && !tma_disabled() && !fp.rows &&

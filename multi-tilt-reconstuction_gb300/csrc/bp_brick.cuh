@@ -33,6 +33,9 @@ struct BpArgs {
 // The SIRT update over residual-pair windows (bp_pairs.cu).
 cudaError_t launch_backproject_tma_pairs(const CUtensorMap& map, const BpPlan& plan, const BpArgs& P,
                                          cudaStream_t st);
+// WBP and SIRT update over windows of plain rows (bp_rows.cu).
+cudaError_t launch_backproject_tma_rows(const CUtensorMap& map, const BpPlan& plan, const BpArgs& P,
+                                        cudaStream_t st);
 
 namespace {
 
@@ -101,8 +104,11 @@ template <int OFF> __device__ __forceinline__ float2 lds_h2_widened(uint32_t a) 
 // p and p + 1 are the window's columns -p and -p - 1, so that one copy of the
 // code serves both signs.  Rounding of the stepped fraction stays below 4e-6 px
 // over 32 voxels; the window has one pixel of slack for it.
-template <int NZ>
-__device__ __forceinline__ void bp_column_rows(float (&s)[NZ], const float2* row0, float xr, float a3, int lxm,
+//
+// ROWS: the window holds plain rows of `pitch` pixels and a pixel of both rows is
+// two 4-byte loads, one instruction more a voxel and half the shared memory.
+template <int NZ, bool ROWS, typename WT>
+__device__ __forceinline__ void bp_column_rows(float (&s)[NZ], const WT* row0, int pitch, float xr, float a3, int lxm,
                                                float fy) {
   const bool up = a3 >= 0.f;
   const float u = up ? xr : -xr;
@@ -110,11 +116,17 @@ __device__ __forceinline__ void bp_column_rows(float (&s)[NZ], const float2* row
   float fx = u - (tu - kMagic);
   const float step = fabsf(a3);
   const int pix = __float_as_int(tu) - kMagicBits;
-  const uint32_t dp = up ? 8u : 0u - 8u;
-  uint32_t p = smem_u32(row0) + 8u * (uint32_t)((lxm + kMagicBits) + (up ? pix : -pix));
-  const float2 q0 = lds_f32x2<0>(p), q1 = lds_f32x2<0>(p + dp);
+  constexpr uint32_t kEs = ROWS ? 4u : 8u;
+  const uint32_t dp = up ? kEs : 0u - kEs;
+  uint32_t p = smem_u32(row0) + kEs * (uint32_t)((lxm + kMagicBits) + (up ? pix : -pix));
+  const uint32_t dr = 4u * (uint32_t)pitch;
+  auto pixel = [&](uint32_t q) {
+    if constexpr (ROWS) return make_float2(lds_f32<0>(q), lds_f32<0>(q + dr));
+    else return lds_f32x2<0>(q);
+  };
+  const float2 q0 = pixel(p), q1 = pixel(p + dp);
   p += 2u * dp;
-  float2 n = lds_f32x2<0>(p);  // the pixel after the next (not used unless the column reaches it)
+  float2 n = pixel(p);  // the pixel after the next (not used unless the column reaches it)
   float b0 = fmaf(fy, q0.y - q0.x, q0.x), b1 = fmaf(fy, q1.y - q1.x, q1.x);
   float d = b1 - b0;
 #pragma unroll
@@ -128,7 +140,7 @@ __device__ __forceinline__ void bp_column_rows(float (&s)[NZ], const float2* row
         p += dp;
       }
       d = b1 - b0;
-      n = lds_f32x2<0>(p);
+      n = pixel(p);
     }
     s[z] = fmaf(fx, d, s[z] + b0);
   }
@@ -265,6 +277,10 @@ __device__ __forceinline__ void bp_column_zy(float (&s)[NZ], const WT* win, int 
       const float2 q0 = lds_f32x2<0>(p), q1 = lds_f32x2<0>(p + dr);
       r0 = fmaf(fx, q0.y, q0.x);
       r1 = fmaf(fx, q1.y, q1.x);
+    } else if constexpr (sizeof(WT) == 4) {  // plain rows
+      const float p00 = lds_f32<0>(p), p10 = lds_f32<4>(p), p01 = lds_f32<0>(p + dr), p11 = lds_f32<4>(p + dr);
+      r0 = fmaf(fx, p10 - p00, p00);
+      r1 = fmaf(fx, p11 - p01, p01);
     } else {
       const float2 q0 = lds_f32x2<0>(p), q1 = lds_f32x2<8>(p);  // both rows at two pixels
       r0 = fmaf(fx, q1.x - q0.x, q0.x);
@@ -295,19 +311,20 @@ __device__ __forceinline__ float tap_weight(float x, int off, int n) {
 // already ran a brick.  PF (pair format, with PAIR): 0 interleaved FP32
 // pairs; 1 planar FP32 pairs, each detector row as two FP32 rows, its values
 // and then its differences; 2 FP16 pairs (value, next - value) in 32 bits.
+// Without PAIR: 0 row pairs, 3 plain rows.
 template <typename PT, int MODE, bool PAIR, int LANES, bool BZ0, int NZ, int PF = 0>
 __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& P, int bx, int by, int bz,
                                          unsigned char* smem, bool reinit) {
   constexpr int BX = bp_brick_x(LANES, PAIR), BY = bp_brick_y(LANES, PAIR);
   // Windows hold row pairs (of the residual, or for the WBP of the
-  // projections), an element (x, y) the pixels (x, y) and (x, y + 1); or, with
-  // PAIR, residual pairs along x (value, next - value), one per pixel, from a
+  // projections), an element (x, y) the pixels (x, y) and (x, y + 1), or its plain
+  // rows; or, with PAIR, residual pairs along x (value, next - value), one per pixel, from a
   // pair array whose column c is pixel c - 1.
   static_assert(!PAIR || MODE == 1, "residual pairs feed the SIRT update only");
-  constexpr bool PLANAR = PAIR && PF == 1, HALF = PAIR && PF == 2;
+  constexpr bool PLANAR = PAIR && PF == 1, HALF = PAIR && PF == 2, ROWS = !PAIR && PF == 3;
   static_assert(!PLANAR || BZ0, "planar windows are a pair format, for y-maps without a Z term");
   using WT = typename std::conditional<
-      PLANAR, float,
+      PLANAR || ROWS, float,
       typename std::conditional<HALF, __half2, float2>::type>::type;
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
   uint64_t* empty = full + NST;
@@ -369,12 +386,14 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
       const int x0 = xi + (int)floorf(xmin) - 1, x1 = xi + (int)floorf(xmax) + 2;
       const int y0 = yi + (int)floorf(ymin) - 1, y1 = yi + (int)floorf(ymax) + 2;
       // The window's rows are the extent's ceiling and three more (a pixel of slack
-      // below, the last pixel's row, a pixel above), as the host planned them, which
+      // below, the last pixel's row, a pixel above; for plain rows the row after it),
+      // as the host planned them, which
       // no rounding of the two ends decides: ymin and ymax rounded apart reach a row
       // further where the extent is whole and the fraction a few 1e-7 below one.
       const double ey = fabs(cy[1]) * (BX - 1) + fabs(cy[2]) * (BY - 1) + fabs(cy[3]) * (NZ - 1);
       // (far(): integers and positions beyond their range say nothing about the window)
-      if (!far(k.xf) && !far(k.yf) && x0 >= ox && x1 < ox + P.WX && (int)ceil(ey - 1e-9) + 3 <= P.WY) k.flags |= kHolds;
+      if (!far(k.xf) && !far(k.yf) && x0 >= ox && x1 < ox + P.WX && (int)ceil(ey - 1e-9) + (ROWS ? 4 : 3) <= P.WY)
+        k.flags |= kHolds;
       if (x0 >= 0 && x1 < P.ax.PX && y0 >= 0 && y1 < P.ax.PY) k.flags |= kOnDetector;
     }
     kc[a] = k;
@@ -400,8 +419,8 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
         // arrays of FP32 pairs are mapped as their floats: x = 2 * (first
         // column), a multiple of 4; planar ones as two FP32 rows per detector
         // row; row pairs have a row above the detector's first
-        tma_load_3d(dst, tmap, (PLANAR || HALF) ? kc[a].ox + 1 : PAIR ? 2 * (kc[a].ox + 1) : 2 * kc[a].ox,
-                    PLANAR ? 2 * kc[a].oy : PAIR ? kc[a].oy : kc[a].oy + 1, a, &full[s]);
+        tma_load_3d(dst, tmap, ROWS ? kc[a].ox : (PLANAR || HALF) ? kc[a].ox + 1 : PAIR ? 2 * (kc[a].ox + 1) : 2 * kc[a].ox,
+                    PLANAR ? 2 * kc[a].oy : PAIR || ROWS ? kc[a].oy : kc[a].oy + 1, a, &full[s]);
         issued = a + 1;
       }
       // Drain: the last load issued into each stage must land before exit
@@ -474,131 +493,129 @@ __device__ __forceinline__ void bp_brick(const CUtensorMap* tmap, const BpArgs& 
           const float ty = __fadd_rd(yr, kMagic);  // floor, in the low bits
           const float fy = yr - (ty - kMagic);
           const WT* row0 = w + (__float_as_int(ty) + k.lym) * WX;
-          bp_column_rows<NZ>(s, row0, xr, k.a3, k.lxm, fy);
+          bp_column_rows<NZ, ROWS>(s, row0, WX, xr, k.a3, k.lxm, fy);
         } else {
           bp_column_zy<NZ, false, false>(s, w, WX, xr, yr, k);
         }
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[st]);
-      continue;
-    }
-    // Uniform rows: the detector y does not move along the lanes (|slope| * 31
-    // below 1e-6 px), so every lane of the warp reads the same two rows with
-    // the same weights; the warp blends them once per angle.
-    const bool uni = BZ0 && LANES != 2 && fabsf(LANES == 1 ? k.b2 : k.b1) < 3e-8f;
-    bool blended = false;
-    if (uni) {
-      yr = __shfl_sync(0xffffffffu, yr, 0);
-      const float fly = floorf(yr);
-      const float fy = yr - fly;
-      const int rowi = magic_int(fly) + k.lym;
-      if ((unsigned)rowi < lim_y) {
-        const WT* row0 = w + rowi * WX * (PLANAR ? 2 : 1);
-        for (int i = lane; i < WX; i += 32) {
-          if constexpr (PLANAR) {
-            const float v0 = row0[i], d0 = row0[i + WX], v1 = row0[i + 2 * WX], d1 = row0[i + 3 * WX];
-            blend[i] = make_float2(fmaf(fy, v1 - v0, v0), fmaf(fy, d1 - d0, d0));
-          } else if constexpr (HALF) {
-            const float2 q0 = __half22float2(row0[i]), q1 = __half22float2(row0[i + WX]);
-            blend[i] = make_float2(fmaf(fy, q1.x - q0.x, q0.x), fmaf(fy, q1.y - q0.y, q0.y));
-          } else {
-            const float2 q0 = row0[i], q1 = row0[i + WX];
-            blend[i] = make_float2(fmaf(fy, q1.x - q0.x, q0.x), fmaf(fy, q1.y - q0.y, q0.y));
-          }
-        }
-        blended = true;
-      }
-      __syncwarp();
-    }
-    bool done = !active;
-    if (active && !BZ0) {
-      // x and y are affine in z: the column's end voxels bound every tap, so
-      // the window is checked once per column
-      const float xe = fmaf(k.a3, (float)(NZ - 1), xr), ye = fmaf(k.b3, (float)(NZ - 1), yr);
-      const int ixa = magic_int(floorf(xr)) + k.lxm, ixb = magic_int(floorf(xe)) + k.lxm;
-      const int iya = magic_int(floorf(yr)) + k.lym, iyb = magic_int(floorf(ye)) + k.lym;
-      bool inside = (unsigned)min(ixa, ixb) < lim_x && (unsigned)max(ixa, ixb) < lim_x &&
-                    (unsigned)min(iya, iyb) < lim_y && (unsigned)max(iya, iyb) < lim_y;
-      if (inside) {
-        bp_column_zy<NZ, PAIR, HALF>(s, w, WX, xr, yr, k);
-        done = true;
-      }
-    }
-    if (active && BZ0 && fabsf(k.a3) < 0.999f) {
-      // x is affine in z: the column's end voxels bound every tap index, so
-      // the window bound is checked once per column instead of per voxel; the
-      // stepped tap may run one pixel past the exact last one.
-      const float fly = floorf(yr);
-      const float fy = yr - fly;
-      const int rowi = magic_int(fly) + k.lym;
-      const int ixa = magic_int(floorf(xr)) + k.lxm;
-      const int ixb = magic_int(floorf(fmaf(k.a3, (float)(NZ - 1), xr))) + k.lxm;
-      bool inside = (unsigned)rowi < lim_y && (unsigned)min(ixa, ixb) < lim_x && (unsigned)(max(ixa, ixb) + 1) < lim_x;
-      if (inside) {
-        if (blended) {
-          if (k.a3 >= 0.f) bp_column_blended<true, NZ>(s, blend, xr, k.a3, k.lxm);
-          else bp_column_blended<false, NZ>(s, blend, xr, k.a3, k.lxm);
-        } else if constexpr (PLANAR) {
-          const float* row0 = w + rowi * 2 * WX;
-          if (k.a3 >= 0.f) bp_column_planar<true, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
-          else bp_column_planar<false, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
-        } else if constexpr (HALF) {
-          const __half2* row0 = w + rowi * WX;
-          if (k.a3 >= 0.f) bp_column_half<true, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
-          else bp_column_half<false, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
-        } else {
-          const WT* row0 = w + rowi * WX;
-          if (k.a3 >= 0.f) bp_column<true, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
-          else bp_column<false, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
-        }
-        done = true;
-      }
-    }
-    if (!done) {
-      // y part (per column when the map has no Z term)
-      float fy = 0.f, wy0 = 0.f, wy1 = 0.f;
-      int rowi = 0;
-      if (BZ0) {
+    } else {
+      // Uniform rows: the detector y does not move along the lanes (|slope| * 31
+      // below 1e-6 px), so every lane of the warp reads the same two rows with
+      // the same weights; the warp blends them once per angle.
+      const bool uni = BZ0 && LANES != 2 && fabsf(LANES == 1 ? k.b2 : k.b1) < 3e-8f;
+      bool blended = false;
+      if (uni) {
+        yr = __shfl_sync(0xffffffffu, yr, 0);
         const float fly = floorf(yr);
-        fy = yr - fly;
-        rowi = magic_int(fly) + k.lym;
-        if ((unsigned)rowi >= lim_y) bad = true;
-        wy0 = 1.f - fy;
-        wy1 = fy;
+        const float fy = yr - fly;
+        const int rowi = magic_int(fly) + k.lym;
+        if ((unsigned)rowi < lim_y) {
+          const WT* row0 = w + rowi * WX * (PLANAR ? 2 : 1);
+          for (int i = lane; i < WX; i += 32) {
+            if constexpr (PLANAR) {
+              const float v0 = row0[i], d0 = row0[i + WX], v1 = row0[i + 2 * WX], d1 = row0[i + 3 * WX];
+              blend[i] = make_float2(fmaf(fy, v1 - v0, v0), fmaf(fy, d1 - d0, d0));
+            } else if constexpr (HALF) {
+              const float2 q0 = __half22float2(row0[i]), q1 = __half22float2(row0[i + WX]);
+              blend[i] = make_float2(fmaf(fy, q1.x - q0.x, q0.x), fmaf(fy, q1.y - q0.y, q0.y));
+            } else {
+              const float2 q0 = row0[i], q1 = row0[i + WX];
+              blend[i] = make_float2(fmaf(fy, q1.x - q0.x, q0.x), fmaf(fy, q1.y - q0.y, q0.y));
+            }
+          }
+          blended = true;
+        }
+        __syncwarp();
       }
-#pragma unroll
-      for (int z = 0; z < NZ; ++z) {
-        if (!BZ0) {
-          const float y = fmaf(k.b3, (float)z, yr);
-          const float fly = floorf(y);
-          fy = y - fly;
+      bool done = !active;
+      if (active && !BZ0) {
+        // x and y are affine in z: the column's end voxels bound every tap, so
+        // the window is checked once per column
+        const float xe = fmaf(k.a3, (float)(NZ - 1), xr), ye = fmaf(k.b3, (float)(NZ - 1), yr);
+        const int ixa = magic_int(floorf(xr)) + k.lxm, ixb = magic_int(floorf(xe)) + k.lxm;
+        const int iya = magic_int(floorf(yr)) + k.lym, iyb = magic_int(floorf(ye)) + k.lym;
+        bool inside = (unsigned)min(ixa, ixb) < lim_x && (unsigned)max(ixa, ixb) < lim_x &&
+                      (unsigned)min(iya, iyb) < lim_y && (unsigned)max(iya, iyb) < lim_y;
+        if (inside) {
+          bp_column_zy<NZ, PAIR, HALF>(s, w, WX, xr, yr, k);
+          done = true;
+        }
+      }
+      if (active && BZ0 && fabsf(k.a3) < 0.999f) {
+        // x is affine in z: the column's end voxels bound every tap index, so
+        // the window bound is checked once per column instead of per voxel; the
+        // stepped tap may run one pixel past the exact last one.
+        const float fly = floorf(yr);
+        const float fy = yr - fly;
+        const int rowi = magic_int(fly) + k.lym;
+        const int ixa = magic_int(floorf(xr)) + k.lxm;
+        const int ixb = magic_int(floorf(fmaf(k.a3, (float)(NZ - 1), xr))) + k.lxm;
+        bool inside = (unsigned)rowi < lim_y && (unsigned)min(ixa, ixb) < lim_x && (unsigned)(max(ixa, ixb) + 1) < lim_x;
+        if (inside) {
+          if (blended) {
+            if (k.a3 >= 0.f) bp_column_blended<true, NZ>(s, blend, xr, k.a3, k.lxm);
+            else bp_column_blended<false, NZ>(s, blend, xr, k.a3, k.lxm);
+          } else if constexpr (PLANAR) {
+            const float* row0 = w + rowi * 2 * WX;
+            if (k.a3 >= 0.f) bp_column_planar<true, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
+            else bp_column_planar<false, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
+          } else if constexpr (HALF) {
+            const __half2* row0 = w + rowi * WX;
+            if (k.a3 >= 0.f) bp_column_half<true, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
+            else bp_column_half<false, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
+          } else {
+            const WT* row0 = w + rowi * WX;
+            if (k.a3 >= 0.f) bp_column<true, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
+            else bp_column<false, NZ>(s, row0, WX, xr, k.a3, k.lxm, 1.f - fy, fy);
+          }
+          done = true;
+        }
+      }
+      if (!done) {
+        // y part (per column when the map has no Z term)
+        float fy = 0.f, wy0 = 0.f, wy1 = 0.f;
+        int rowi = 0;
+        if (BZ0) {
+          const float fly = floorf(yr);
+          fy = yr - fly;
           rowi = magic_int(fly) + k.lym;
           if ((unsigned)rowi >= lim_y) bad = true;
           wy0 = 1.f - fy;
           wy1 = fy;
         }
-        const float x = fmaf(k.a3, (float)z, xr);
-        const float flx = floorf(x);
-        const float fx = x - flx;
-        const int ix = magic_int(flx) + k.lxm;
-        if ((unsigned)ix >= lim_x) bad = true;
-        const int i0 = bad ? 0 : ix + rowi * WX * (PLANAR ? 2 : 1);  // never index outside the window
-        float r0, r1;
-        if constexpr (PLANAR) {
-          r0 = fmaf(fx, w[i0 + WX], w[i0]);
-          r1 = fmaf(fx, w[i0 + 3 * WX], w[i0 + 2 * WX]);
-        } else if constexpr (HALF) {
-          const float2 q0 = __half22float2(w[i0]), q1 = __half22float2(w[i0 + WX]);
-          r0 = fmaf(fx, q0.y, q0.x);
-          r1 = fmaf(fx, q1.y, q1.x);
-        } else {
-          const float2 q0 = w[i0], q1 = w[i0 + WX];
-          r0 = fmaf(fx, q0.y, q0.x);
-          r1 = fmaf(fx, q1.y, q1.x);
+#pragma unroll
+        for (int z = 0; z < NZ; ++z) {
+          if (!BZ0) {
+            const float y = fmaf(k.b3, (float)z, yr);
+            const float fly = floorf(y);
+            fy = y - fly;
+            rowi = magic_int(fly) + k.lym;
+            if ((unsigned)rowi >= lim_y) bad = true;
+            wy0 = 1.f - fy;
+            wy1 = fy;
+          }
+          const float x = fmaf(k.a3, (float)z, xr);
+          const float flx = floorf(x);
+          const float fx = x - flx;
+          const int ix = magic_int(flx) + k.lxm;
+          if ((unsigned)ix >= lim_x) bad = true;
+          const int i0 = bad ? 0 : ix + rowi * WX * (PLANAR ? 2 : 1);  // never index outside the window
+          float r0, r1;
+          if constexpr (PLANAR) {
+            r0 = fmaf(fx, w[i0 + WX], w[i0]);
+            r1 = fmaf(fx, w[i0 + 3 * WX], w[i0 + 2 * WX]);
+          } else if constexpr (HALF) {
+            const float2 q0 = __half22float2(w[i0]), q1 = __half22float2(w[i0 + WX]);
+            r0 = fmaf(fx, q0.y, q0.x);
+            r1 = fmaf(fx, q1.y, q1.x);
+          } else {
+            const float2 q0 = w[i0], q1 = w[i0 + WX];
+            r0 = fmaf(fx, q0.y, q0.x);
+            r1 = fmaf(fx, q1.y, q1.x);
+          }
+          s[z] = fmaf(wy0, r0, s[z]);
+          s[z] = fmaf(wy1, r1, s[z]);
         }
-        s[z] = fmaf(wy0, r0, s[z]);
-        s[z] = fmaf(wy1, r1, s[z]);
       }
     }
     __syncwarp();
@@ -658,9 +675,9 @@ cudaError_t launch_one(const CUtensorMap& map, const BpArgs& P, size_t smem, cud
 template <typename PT, int MODE, bool PAIR, int LANES, bool BZ0, int PF = 0>
 cudaError_t launch_nz(const CUtensorMap& map, const BpArgs& P, const BpPlan& plan, cudaStream_t st) {
   if constexpr (MODE == 0) {  // the WBP has no depth 4
-    if (plan.nz == 32) return launch_one<PT, 0, PAIR, LANES, BZ0, 32>(map, P, plan.smem, st);
-    if (plan.nz == 16) return launch_one<PT, 0, PAIR, LANES, BZ0, 16>(map, P, plan.smem, st);
-    return launch_one<PT, 0, PAIR, LANES, BZ0, 8>(map, P, plan.smem, st);
+    if (plan.nz == 32) return launch_one<PT, 0, PAIR, LANES, BZ0, 32, PF>(map, P, plan.smem, st);
+    if (plan.nz == 16) return launch_one<PT, 0, PAIR, LANES, BZ0, 16, PF>(map, P, plan.smem, st);
+    return launch_one<PT, 0, PAIR, LANES, BZ0, 8, PF>(map, P, plan.smem, st);
   } else {
     if (plan.nz == 8) return launch_one<PT, MODE, PAIR, LANES, BZ0, 8, PF>(map, P, plan.smem, st);
     if (plan.nz == 4) return launch_one<PT, MODE, PAIR, LANES, BZ0, 4, PF>(map, P, plan.smem, st);

@@ -213,12 +213,13 @@ double window_bank_cost(const std::vector<double>& xc, const std::vector<double>
 namespace {
 
 // Window box for a brick of depth nz over all angles of an axis.
-BpPlan plan_backproject_uncached(const std::vector<double>& xc, const std::vector<double>& yc, int A, int fmt,
-                                 int nz, int lane) {
+BpPlan plan_window(const std::vector<double>& xc, const std::vector<double>& yc, int A, int fmt, bool rows, int nz,
+                   int lane) {
   BpPlan p;
-  // planar and FP16 pair windows start on a 4-element (16-byte) boundary;
-  // those of 8-byte elements (row pairs, interleaved pairs) on an even column
-  const bool pairs = fmt == 0 || fmt == 1;
+  // windows of 4-byte elements start on a 4-element (16-byte) boundary; those of
+  // 8-byte elements (row pairs, interleaved pairs) on an even column
+  const bool pairs = (fmt == 0 && !rows) || fmt == 1;
+  p.rows = fmt == 0 && rows;
   p.align = pairs ? 2 : 4;
   p.pairs = fmt != 0;
   p.planar = fmt == 2;
@@ -249,7 +250,7 @@ BpPlan plan_backproject_uncached(const std::vector<double>& xc, const std::vecto
   // taps span [floor(min)-1, floor(max)+1], origin rounded down to the alignment
   const int wx = (int)std::ceil(ex) + 4 + p.align;
   const int wx_min = (wx + p.align - 1) / p.align * p.align;
-  p.WY = (int)std::ceil(ey) + (fmt == 0 ? 3 : 4);  // (a row pair holds the next row)
+  p.WY = (int)std::ceil(ey) + (fmt == 0 && !rows ? 3 : 4);  // (a row pair holds the next row)
   auto smem_for = [&](int WX) {
     const size_t stage = (((size_t)WX * p.WY * planes * es) + 127) & ~(size_t)127;
     return 128 + ((((size_t)A * sizeof(WinConst)) + 127) & ~(size_t)127) + NST * stage +
@@ -289,6 +290,21 @@ BpPlan plan_backproject_uncached(const std::vector<double>& xc, const std::vecto
   return p;
 }
 
+BpPlan plan_backproject_uncached(const std::vector<double>& xc, const std::vector<double>& yc, int A, int fmt,
+                                 int nz, int lane) {
+  const BpPlan pairs = plan_window(xc, yc, A, fmt, false, nz, lane);
+  if (fmt != 0) return pairs;
+  const BpPlan rows = plan_window(xc, yc, A, fmt, true, nz, lane);
+  // Row pairs (8 % fewer instructions) where at least three CTAs share an SM, or as
+  // many as with plain rows; else plain rows, half the bytes.  Tiles with three or
+  // four CTAs of row pairs (one pixel per voxel) ran 0.92-0.98 times as long on them,
+  // tiles with one or two mostly 1.0-2.0 times (256x256x64, 61 angles, update: 2
+  // pixels per voxel at 45 degrees 299 -> 242 us, 3 pixels 446 -> 352; 4 pixels at 30
+  // degrees, where no row pairs fit and the plain kernel ran, 1283 -> 422).
+  auto ctas = [](const BpPlan& p) { return p.ok ? (int)(228 * 1024 / (p.smem + 1024)) : 0; };
+  return !rows.ok || ctas(pairs) >= std::min(3, ctas(rows)) ? pairs : rows;
+}
+
 PlanMemo<BpPlan> g_bp_plans;
 
 }  // namespace
@@ -306,6 +322,7 @@ cudaError_t launch_backproject_tma(const CUtensorMap& map, const BpPlan& plan, c
   BpArgs P{ax,        vol,      z0,       z1,   plan.WX, plan.WY, plan.align,
            mode,      step,     vol_out,  cbp,  vol_copy, copy_kind, err,
            g_wait_iters.load(std::memory_order_relaxed)};
+  if (plan.rows) return launch_backproject_tma_rows(map, plan, P, st);
   if (mode == 0) {
     if (plan.lanes == 2) return plan.bz0 ? launch_nz<PT, 0, false, 2, true>(map, P, plan, st)
                                          : launch_nz<PT, 0, false, 2, false>(map, P, plan, st);

@@ -131,6 +131,7 @@ struct BpPlan {
   int align = 2;       // TMA x alignment (elements)
   int nz = 8;          // brick depth (voxels per thread along Z): 4, 8, 16 or 32
   bool pairs = false;  // windows of pairs along x (SIRT update) rather than row pairs
+  bool rows = false;   // windows of plain rows rather than row pairs
   bool planar = false; // pairs as two FP32 planes per row (values, differences) instead of interleaved
   bool half = false;   // pairs as FP16 (value, difference) in 32 bits (mixed precision)
   size_t smem = 0;     // dynamic shared memory per CTA
@@ -143,7 +144,7 @@ double window_bank_cost(const std::vector<double>& xc, const std::vector<double>
                         int WX, bool pairs = false);
 // lane: -1 picks lines along the larger x-map slope, 0 = lines along X,
 // 1 = lines along Y, 2 = 8x4 patches.
-// fmt: 0 FP32 row pairs (also the WBP's windows of the projections), 1
+// fmt: 0 FP32 row pairs or plain rows (also the WBP's windows of the projections), 1
 // interleaved residual pairs along x, 2 planar ones, 3 FP16 ones (mixed
 // precision).
 BpPlan plan_backproject(const std::vector<double>& xc, const std::vector<double>& yc, int A, int fmt, int nz,

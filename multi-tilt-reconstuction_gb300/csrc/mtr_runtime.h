@@ -324,8 +324,9 @@ inline bool encode_pair_map(CUtensorMap* m, const AxisState& a, const BpPlan& p)
   return encode_tensor_map_3d(m, a.r.p, false, 2 * a.pitch2, 2 * a.pitch2, a.PY, a.A, 2 * p.WX, p.WY);
 }
 // Tensor map over an axis' residual in the form its SIRT update reads: pairs
-// along x, or row pairs (PY + 1 rows of 2 * row_pair_pitch floats).
+// along x, row pairs (PY + 1 rows of 2 * row_pair_pitch floats) or plain rows.
 inline bool encode_residual_map(CUtensorMap* m, const AxisState& a, const BpPlan& p) {
+  if (p.rows) return encode_tensor_map_3d(m, a.r.p, false, a.PX, a.pitch, a.PY, a.A, p.WX, p.WY);
   return p.pairs ? encode_pair_map(m, a, p)
                  : encode_tensor_map_3d(m, a.r.p, false, 2 * a.PX, 2 * row_pair_pitch(a.PX), a.PY + 1, a.A, 2 * p.WX,
                                         p.WY);

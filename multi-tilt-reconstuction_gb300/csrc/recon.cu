@@ -257,7 +257,7 @@ mtr_status enqueue_residual(mtr_recon* r, AxisState& a, double* norm) {
     else
       launch_residual_pairs<float>(rows, a.pitch, a.pitch2, a.b.as<float>(), a.s.as<float>(), a.cf.as<float>(),
                                    a.r.as<float>(), a.plan.planar ? 1 : 0, norm, ctx->stream);
-  } else if (a.tma) {  // row pairs
+  } else if (a.tma && !a.plan.rows) {  // row pairs
     if (mixed(r->p.precision))
       launch_row_pairs<__half>(0, a.dev(), a.b.as<__half>(), a.s.as<float>(), a.cf.as<float>(), a.r.as<float>(), norm,
                                ctx->stream);
@@ -289,11 +289,14 @@ mtr_status enqueue_widen_for_wbp(mtr_recon* r, AxisState& a) {
     return e == cudaSuccess ? MTR_OK : cuda_error(r->ctx, e, "projections' line image");
   }
   if (!a.tma_b) return MTR_OK;
-  if (mixed(r->p.precision))
+  if (a.plan_b.rows) {  // FP32 projections are read as they are
+    if (!mixed(r->p.precision)) return MTR_OK;
+    launch_widen(a.b.as<__half>(), a.r.as<float>(), a.np, r->ctx->stream);
+  } else if (mixed(r->p.precision))
     launch_row_pairs<__half>(1, a.dev(), a.b.as<__half>(), nullptr, nullptr, a.r.as<float>(), nullptr, r->ctx->stream);
   else
     launch_row_pairs<float>(1, a.dev(), a.b.as<float>(), nullptr, nullptr, a.r.as<float>(), nullptr, r->ctx->stream);
-  MTR_CK_LAUNCH(r->ctx, "projections' row pairs");
+  MTR_CK_LAUNCH(r->ctx, "projections' rows");
   return MTR_OK;
 }
 
@@ -681,7 +684,10 @@ mtr_status mtr::recon_create(mtr_context* ctx, int n_axes, const mtr_axis* axes,
       // tuned for it (lines or 8x4 patches) and its depth, at least 8.
       a.plan_b = plan_backproject(a.hxc, a.hyc, a.A, 0, a.plan.ok ? std::max(8, a.plan.nz) : 8,
                                   a.plan.ok ? a.plan.lanes : -1);
-      a.tma_b = a.plan_b.ok && encode_residual_map(&a.map_b, a, a.plan_b);
+      a.tma_b = a.plan_b.ok &&
+                (a.plan_b.rows && !mx ? encode_tensor_map_3d(&a.map_b, a.b.p, false, a.PX, a.pitch, a.PY, a.A,
+                                                             a.plan_b.WX, a.plan_b.WY)
+                                      : encode_residual_map(&a.map_b, a, a.plan_b));
     }
   }
   if (params->flags & MTR_FLAG_RECORD_NORMS) {

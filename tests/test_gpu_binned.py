@@ -69,3 +69,27 @@ def test_rows_summed_per_warp_of_many_columns_on_one_pixel(ctx, monkeypatch):
     x = axes[0].x_coef.copy()
     x[1::4] *= 0.05
     check(ctx, v, [mtr.AxisData(x, axes[0].y_coef, axes[0].data)])
+
+
+@pytest.mark.parametrize("prec", [mtr.PREC_FP32, mtr.PREC_MIXED_FP16])
+@pytest.mark.parametrize("phi,lean", [(0.0, 0.0), (30.0, 0.0), (45.0, 0.05), (90.0, -0.3)])
+@pytest.mark.parametrize("mag", [2.0, 3.0, 4.0])
+def test_tuned_tiles_are_windowed_and_match_oracle(ctx, mag, phi, lean, prec):
+    plan = check(ctx, *binned(mag, phi, lean=lean, shift=0.3), prec)
+    assert plan["back_projection"]["tma"] and plan["forward"]["tma"]
+
+
+@pytest.mark.parametrize("depths", ["4,8,0,2,0", "8,16,1,2,0", "16,16,2,2,0", "32,8,2,2,0", "8,8,0,0,0"])
+@pytest.mark.parametrize("phi,lean,cover", [(45.0, 0.0, 1.1), (30.0, 0.07, 0.7), (135.0, -0.6, 1.1), (0.0, 0.0, 1.1)])
+@pytest.mark.parametrize("mag", [2.5, 4.0])
+def test_plain_row_windows_match_oracle(ctx, monkeypatch, depths, phi, lean, cover, mag):
+    """Windows of plain rows in every lane layout and depth, inside the detector and over its edges."""
+    monkeypatch.setenv("MTR_FORCE_DEPTHS", depths)
+    check(ctx, *binned(mag, phi, vol=(0, 47, 0, 39, 0, 37), lean=lean, cover=cover, shift=0.3))
+
+
+def test_untuned_tiles_are_windowed(ctx, monkeypatch):
+    monkeypatch.setenv("MTR_AUTOTUNE", "0")
+    for mag, phi in ((3.0, 45.0), (4.0, 30.0)):
+        v, axes = binned(mag, phi, vol=(1, 46, 0, 37, 0, 22), shift=0.3)
+        assert check(ctx, v, axes)["back_projection"]["tma"]
