@@ -481,6 +481,21 @@ mtr_status enqueue_run(mtr_recon* r) {
   return enqueue_outer(r, 0, r->p.iter_times);
 }
 
+// The WBP gathers windows like the SIRT update's: the lane layout tuned for it
+// (lines or 8x4 patches) and its depth, at least 8; where such a window does not
+// fit (the update's may hold smaller elements), a shallower one or another layout.
+BpPlan plan_wbp(const AxisState& a) {
+  const int depth = a.plan.ok ? std::max(8, a.plan.nz) : 8, tuned = a.plan.ok ? a.plan.lanes : -1;
+  BpPlan p;
+  for (int lanes : {tuned, 2, 0, 1})
+    for (int nz : {depth, 16, 8}) {
+      if (nz > depth) continue;
+      p = plan_backproject(a.hxc, a.hyc, a.A, 0, nz, lanes);
+      if (p.ok) return p;
+    }
+  return p;
+}
+
 // Line plan, tables and tensor maps of an axis whose maps separate (`depth`:
 // planes of a launch, a whole volume or a streamed slab).
 mtr_status setup_lines(mtr_recon* r, AxisState& a, int depth) {
@@ -680,10 +695,7 @@ mtr_status mtr::recon_create(mtr_context* ctx, int n_axes, const mtr_axis* axes,
         tune_axis(ctx, a, r->vol, params->precision, a.x.as<float>(), a.cbp.as<float>(), a.xcopy.p,
                   r->err.as<int>());
       }
-      // The WBP gathers the same windows as the SIRT update: the lane layout
-      // tuned for it (lines or 8x4 patches) and its depth, at least 8.
-      a.plan_b = plan_backproject(a.hxc, a.hyc, a.A, 0, a.plan.ok ? std::max(8, a.plan.nz) : 8,
-                                  a.plan.ok ? a.plan.lanes : -1);
+      a.plan_b = plan_wbp(a);
       a.tma_b = a.plan_b.ok &&
                 (a.plan_b.rows && !mx ? encode_tensor_map_3d(&a.map_b, a.b.p, false, a.PX, a.pitch, a.PY, a.A,
                                                              a.plan_b.WX, a.plan_b.WY)

@@ -93,3 +93,18 @@ def test_untuned_tiles_are_windowed(ctx, monkeypatch):
     for mag, phi in ((3.0, 45.0), (4.0, 30.0)):
         v, axes = binned(mag, phi, vol=(1, 46, 0, 37, 0, 22), shift=0.3)
         assert check(ctx, v, axes)["back_projection"]["tma"]
+
+
+@pytest.mark.parametrize("forced,phi,lean", [("32,16,2,2,3", 0.0, 0.05), ("4,16,1,2,0", 15.0, 0.0)])
+def test_wbp_takes_a_window_that_fits(ctx, monkeypatch, forced, phi, lean):
+    """An update whose tile leaves the WBP no window of its own depth and layout."""
+    monkeypatch.setenv("MTR_FORCE_DEPTHS", forced)
+    v, axes = binned(5.0, phi, vol=(0, 40, 0, 33, 0, 40), lean=lean, shift=0.3)
+    r = mtr.Recon(ctx, axes, v, mtr.params(1, 0, 0.5, 0.7, mtr.PREC_MIXED_FP16))
+    assert r.describe()[0]["back_projection"]["depth"] == int(forced.split(",")[0])
+    n = ctx.windowed_launch_count()
+    r.run()
+    got, launched = r.download(), ctx.windowed_launch_count() - n
+    r.close()
+    assert launched == 1  # the WBP: no SIRT iteration runs
+    assert rel_l2(got, oracle.wbp(oracle.FP64, axes[0], v)) < TOL[mtr.PREC_MIXED_FP16]
