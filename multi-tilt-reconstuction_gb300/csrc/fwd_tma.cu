@@ -404,8 +404,7 @@ __device__ __forceinline__ void prefix_brick(const CUtensorMap* smap, const FwdA
     // the weight w = min(depth, 1 + 1/slope) <= 2^lw from one column:
     // |addition| < 2^(b + lw) <= 2^21, the range of the magic rounding.  A
     // pixel's window sum stays below 2^(b + mass_shift) <= 2^30 (no overflow).
-    int lw = 0;
-    frexpf(fminf((float)NZ, 1.f + 1.f / st), &lw);
+    const int lw = log2_ceil(fminf((float)NZ, 1.f + 1.f / st));
     const int bits = min(21 - lw, 30 - P.mass_shift);
     const int sexp = max(-120, min(120, bits - e2));
     k.scale = ldexpf(1.f, sexp);

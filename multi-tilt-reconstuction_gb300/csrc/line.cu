@@ -266,9 +266,8 @@ line_forward_kernel(const __grid_constant__ CUtensorMap map, const LineArgs P, c
     // |v| < 2^e; an emission sums at most w = min(NZ, 1 + 1/slope) <= 2^lw of
     // them and stays below 2^21 (the rounding addition's range); a window
     // element gathers at most 8 NZ voxels, so its sum stays below 2^29
-    int lw = 0;
     const float st = fabsf(k.a3);
-    frexpf(fminf((float)NZ, 1.f + (st > 1e-30f ? 1.f / st : 1e30f)), &lw);
+    const int lw = log2_ceil(fminf((float)NZ, 1.f + (st > 1e-30f ? 1.f / st : 1e30f)));
     const int sexp = max(-120, min(120, 21 - lw - e2));
     k.scale = ldexpf(1.f, sexp);
     k.inv_scale = ldexpf(1.f, -sexp);

@@ -90,6 +90,13 @@ inline void launch_overlapped(void (*kern)(P...), dim3 grid, dim3 block, size_t 
   cudaLaunchKernelEx(&c, kern, static_cast<P>(q)...);  // (a failure is the caller's cudaGetLastError, as with <<<>>>)
 }
 
+// Smallest e with 2^e >= w, for a finite w > 0.
+__device__ __forceinline__ int log2_ceil(float w) {
+  int e;
+  const float m = frexpf(w, &e);  // w = m 2^e, m in [0.5, 1)
+  return m == 0.5f ? e - 1 : e;
+}
+
 // 3-D tiled TMA load of one box into shared memory, completing on bar.
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
   asm volatile(
