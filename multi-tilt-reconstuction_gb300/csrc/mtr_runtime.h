@@ -289,13 +289,13 @@ struct AxisState {
   bool ftma = false;
   // Axes whose maps separate run on line images instead of windows (line.cuh):
   // the line sums live in s ([A][PX][line.Wp]), the residual's (before the
-  // first SIRT iteration, the projections') line image in r.
+  // first SIRT iteration, the projections') line image in r, and the row tables
+  // in r behind np values, which the image and the uploads stay within.
   LinePlan line;
   CUtensorMap map_ls{}, map_lr{}, map_lb{};  // over s; over r for the SIRT update and the WBP
-  DevBuf line_tab;
   bool lines = false;
   LineTab tab() const {
-    const int* t = line_tab.as<int>();
+    const int* t = r.as<int>() + np;
     return LineTab{reinterpret_cast<const int2*>(t), reinterpret_cast<const int2*>(t + line.off_rows),
                    reinterpret_cast<const float*>(t + line.off_weight), line.n_tab > 1 ? 1 : 0};
   }

@@ -503,14 +503,15 @@ mtr_status setup_lines(mtr_recon* r, AxisState& a, int depth) {
   VolDev v = r->vol;
   a.line = plan_lines(a.hxc, a.hyc, a.A, a.PX, a.PY, a.pitch, v, depth, ctx->num_sms);
   LinePlan& p = a.line;
-  if (!p.ok) return MTR_OK;
+  // (12 bytes per line position and 8 per detector row and angle: they fit behind
+  // np values from a detector of four columns on, fewer than which has no lines)
+  const size_t tables = p.tables.size() * sizeof(int);
+  if (!p.ok || (size_t)a.np * 4 + tables > a.r.bytes) return MTR_OK;
   if (!encode_tensor_map_3d(&a.map_ls, a.s.p, false, p.W, p.Wp, a.PX, a.A, 32 * p.fwd_vl, p.fwd_rows) ||
       !encode_tensor_map_3d(&a.map_lr, a.r.p, false, p.W, p.Wp, a.PX, a.A, 32 * p.bp_vl, p.bp_rows) ||
       !encode_tensor_map_3d(&a.map_lb, a.r.p, false, p.W, p.Wp, a.PX, a.A, 32 * p.wbp_vl, p.wbp_rows))
     return MTR_OK;
-  MTR_CK(ctx, a.line_tab.alloc_pooled(p.tables.size() * sizeof(int), ctx));
-  MTR_CK(ctx, cudaMemcpyAsync(a.line_tab.p, p.tables.data(), p.tables.size() * sizeof(int), cudaMemcpyHostToDevice,
-                              ctx->stream));
+  MTR_CK(ctx, cudaMemcpyAsync(a.r.as<int>() + a.np, p.tables.data(), tables, cudaMemcpyHostToDevice, ctx->stream));
   a.lines = true;
   return MTR_OK;
 }
