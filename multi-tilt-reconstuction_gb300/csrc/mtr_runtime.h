@@ -347,9 +347,10 @@ bool windows_forced();
 void record_untimed_tiles(const AxisState& a, const VolDev& v, int precision);
 // Candidates run over the frame v on device scratch: scratch_vol / scratch_cbp
 // (FP32) and, in mixed precision, scratch_copy (the BF16 / FP16 copy the
-// forward splat reads); none of them holds data yet.
-bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, int precision, float* scratch_vol,
-               float* scratch_cbp, void* scratch_copy, int* err);
+// forward splat reads); none of them holds data yet.  whole: the volume that v
+// is a slab of.
+bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, const VolDev& whole, int precision,
+               float* scratch_vol, float* scratch_cbp, void* scratch_copy, int* err);
 
 // The Z planes [z0, z1) one launch works on and the arrays that hold exactly
 // those planes: an axis' whole volume arrays, or one slot of a streamed

@@ -689,11 +689,11 @@ mtr_status mtr::recon_create(mtr_context* ctx, int n_axes, const mtr_axis* axes,
       if (streamed) {  // candidates over one slab, in the slot arrays the run uses
         VolDev tv = r->vol;
         tv.NZ = r->slabs->depth;
-        tune_axis(ctx, a, tv, params->precision, r->slabs->x[0].as<float>(), r->slabs->cbp[0].as<float>(),
+        tune_axis(ctx, a, tv, r->vol, params->precision, r->slabs->x[0].as<float>(), r->slabs->cbp[0].as<float>(),
                   r->slabs->xc[0].p, r->err.as<int>());
       } else {
         // (x and cbp: FP32 volume arrays the WBP init writes afterwards)
-        tune_axis(ctx, a, r->vol, params->precision, a.x.as<float>(), a.cbp.as<float>(), a.xcopy.p,
+        tune_axis(ctx, a, r->vol, r->vol, params->precision, a.x.as<float>(), a.cbp.as<float>(), a.xcopy.p,
                   r->err.as<int>());
       }
       a.plan_b = plan_wbp(a);

@@ -15,7 +15,7 @@
 //    along x (faster where a warp's lanes share detector rows), or the same
 //    pairs as two FP32 planes per row (4-byte loads); in mixed precision FP16
 //    pairs in 32 bits on large oblique axes (fp16_residual).
-// For each tilt axis the tuner times every candidate (3 formats x depth
+// For each tilt axis the tuner times every candidate (3 FP32 formats, or FP16 pairs, x depth
 // 4/8/16/32 x lines along X / lines along Y / patches for the SIRT
 // back-projection, depth 8/16/32 x the same three layouts for the forward
 // splat) with CUDA events on the reconstruction's own buffers, over a Z-slab
@@ -25,7 +25,7 @@
 // when MTR_AUTOTUNE_CACHE names a file, persisted there as JSON ({"key":
 // [bp_depth, fwd_depth, bp_lane, fwd_lane, bp_format], ...}; bp_format 0 row
 // pairs, 1 interleaved pairs, 2 planar pairs, 3 FP16 pairs in mixed precision).  MTR_AUTOTUNE=0 disables
-// tuning (depths 8 and 16, lane axis by slope, row pairs);
+// tuning (depths 8 and 16, lane axis by slope, row pairs or FP16 pairs);
 // MTR_FORCE_DEPTHS=bp,fwd[,bp_lane,fwd_lane[,bp_format]] pins the choice;
 // MTR_AUTOTUNE_LOG=1 prints every candidate's time to stderr.
 #include <algorithm>
@@ -99,7 +99,25 @@ void save_file() {
   f << "}\n";
 }
 
-std::string geometry_key(const AxisState& a, const VolDev& v, int precision) {
+// Mixed precision stores the residual of a large oblique axis as FP16 pairs
+// (half the bytes of the row pairs or FP32 pairs): part of that mode's
+// rounding, so it follows from the axis and the whole volume alone, however the
+// tiles are chosen (timed, cached or not tuned, over the volume or a slab of it).
+// Axes whose rows lie within 6 degrees of a volume axis, z-dependent y-maps and
+// volumes of fewer than 608 bricks of 32x8x16 (four for each SM) keep FP32, as
+// the tuner chose for them when it timed all formats (256x256x64 at 17-60 degrees
+// FP16, 128x128x32 and 1 or 89 degrees FP32).
+bool fp16_residual(const AxisState& a, const VolDev& whole, int precision) {
+  if (precision == MTR_PREC_FP32) return false;
+  for (int k = 0; k < a.A; ++k) {
+    const double* c = &a.hyc[4 * (size_t)k];
+    const double low = std::min(std::fabs(c[1]), std::fabs(c[2]));
+    if (c[3] != 0.0 || low < 0.1 * std::hypot(c[1], c[2])) return false;
+  }
+  return (long long)((whole.NX + 31) / 32) * ((whole.NY + 7) / 8) * ((whole.NZ + 15) / 16) >= 608;
+}
+
+std::string geometry_key(const AxisState& a, const VolDev& v, int precision, bool fp16) {
   double m[6] = {0, 0, 0, 0, 0, 0};
   bool bz0 = true;
   for (int k = 0; k < a.A; ++k) {
@@ -109,24 +127,9 @@ std::string geometry_key(const AxisState& a, const VolDev& v, int precision) {
   }
   char buf[256];
   // the trailing tag names the timing method, so choices cached by an older one are not reused
-  std::snprintf(buf, sizeof(buf), "p%dx%dx%d_v%dx%dx%d_m%.2f,%.2f,%.2f,%.2f,%.2f,%.2f_z%d_prec%d_t12", a.PX, a.PY,
-                a.A, v.NX, v.NY, v.NZ, m[0], m[1], m[2], m[3], m[4], m[5], bz0 ? 0 : 1, precision);
+  std::snprintf(buf, sizeof(buf), "p%dx%dx%d_v%dx%dx%d_m%.2f,%.2f,%.2f,%.2f,%.2f,%.2f_z%d_prec%d%s_t13", a.PX, a.PY,
+                a.A, v.NX, v.NY, v.NZ, m[0], m[1], m[2], m[3], m[4], m[5], bz0 ? 0 : 1, precision, fp16 ? "h" : "");
   return buf;
-}
-
-// Mixed precision stores the residual of a large oblique axis as FP16 pairs
-// (half the bytes of the row pairs or FP32 pairs): part of that mode's
-// rounding, so it is decided by the geometry and not by a race between formats.
-// Axes whose rows lie within 6 degrees of a volume axis, z-dependent y-maps and
-// volumes of fewer than four 32x8x16 bricks per SM keep FP32, as the tuner
-// chose for them when it timed all formats (256x256x64 at 17-60 degrees FP16,
-// 128x128x32 and 1 or 89 degrees FP32).
-bool fp16_residual(const AxisState& a, const VolDev& v, int sms) {
-  for (int k = 0; k < a.A; ++k) {
-    const double* c = &a.hyc[4 * (size_t)k];
-    if (c[3] != 0.0 || std::min(std::fabs(c[1]), std::fabs(c[2])) < 0.1) return false;
-  }
-  return (long long)((v.NX + 31) / 32) * ((v.NY + 7) / 8) * ((v.NZ + 15) / 16) >= 4LL * sms;
 }
 
 // Times every candidate launch and returns the index of the fastest (-1 if
@@ -199,17 +202,18 @@ void record_untimed_tiles(const AxisState& a, const VolDev& v, int precision) {
   c.bp_lane = c.fwd_lane = a.line.along_x ? 0 : 1;
   std::lock_guard<std::mutex> lock(g_mu);
   load_file();
-  if (g_cache.emplace(geometry_key(a, v, precision) + "_lines", c).second) save_file();
+  if (g_cache.emplace(geometry_key(a, v, precision, false) + "_lines", c).second) save_file();
 }
 
 // Chooses a.plan (SIRT back-projection over r) and a.fplan (forward splat
 // over s) for one axis and encodes the matching tensor maps.  Leaves s zeroed.
-bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, int precision, float* scratch_vol,
-               float* scratch_cbp, void* scratch_copy, int* err) {
+bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, const VolDev& whole, int precision,
+               float* scratch_vol, float* scratch_cbp, void* scratch_copy, int* err) {
   const int copy_kind = precision == MTR_PREC_MIXED_BF16 ? 1 : precision == MTR_PREC_MIXED_FP16 ? 2 : 0;
-  const std::string key = geometry_key(a, v, precision);
+  const bool fp16 = fp16_residual(a, whole, precision);
+  const std::string key = geometry_key(a, v, precision, fp16);
   Choice ch;
-  bool known = false;
+  bool known = false, forced = false;
   if (const char* f = std::getenv("MTR_FORCE_DEPTHS")) {
     Choice c;
     const int n = std::sscanf(f, "%d,%d,%d,%d,%d", &c.bp_nz, &c.fwd_nz, &c.bp_lane, &c.fwd_lane, &c.bp_pairs);
@@ -217,7 +221,7 @@ bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, int precision, f
       if (n < 4) c.bp_lane = c.fwd_lane = -1;
       if (n < 5) c.bp_pairs = 0;
       ch = c;
-      known = true;
+      known = forced = true;
     }
   }
   if (!known) {
@@ -251,7 +255,6 @@ bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, int precision, f
     std::vector<BpPlan> bps;
     std::vector<CUtensorMap> bmaps;
     // (the candidates keep pointers into these: no reallocation)
-    const bool fp16 = copy_kind != 0 && fp16_residual(a, v, ctx->num_sms);
     const int fmt0 = fp16 ? 3 : 0, fmt1 = fp16 ? 4 : 3;
     bps.reserve(12 * std::size(kBpDepths));  // formats x 3 lane layouts x the depths
     bmaps.reserve(12 * std::size(kBpDepths));
@@ -336,8 +339,11 @@ bool tune_axis(mtr_context* ctx, AxisState& a, const VolDev& v, int precision, f
   }
   // the timing runs wrote into s and the tuner's scratch: restore the zeros
   cudaMemsetAsync(a.s.p, 0, (size_t)a.np * 4, ctx->stream);
-  a.plan = plan_backproject(a.hxc, a.hyc, a.A, std::min(std::max(ch.bp_pairs, 0), copy_kind != 0 ? 3 : 2), ch.bp_nz,
-                            ch.bp_lane);
+  const int format = forced ? std::min(std::max(ch.bp_pairs, 0), copy_kind != 0 ? 3 : 2)
+                            : fp16 ? 3 : std::min(std::max(ch.bp_pairs, 0), 2);
+  a.plan = plan_backproject(a.hxc, a.hyc, a.A, format, ch.bp_nz, ch.bp_lane);
+  if (!a.plan.ok && fp16 && !forced)  // no FP16 window fits: FP32 ones
+    a.plan = plan_backproject(a.hxc, a.hyc, a.A, 0, ch.bp_nz, ch.bp_lane);
   a.tma = a.plan.ok && encode_residual_map(&a.map_r, a, a.plan);
   a.fplan = plan_forward(a.hxc, a.hyc, a.A, a.PX, a.PY, a.pitch, ch.fwd_nz, ch.fwd_lane);
   a.ftma = a.fplan.ok &&
