@@ -45,6 +45,12 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, 0xBF800000BF800000ull, a); }
 __device__ __forceinline__ f32x2 lds_pair(uint32_t a) {
   f32x2 v;
   asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
@@ -534,11 +540,12 @@ line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
     const uint32_t tab = smem_u32(table);
     const uint32_t dstep = s.dir > 0 ? 4u * BW : 0u - 4u * BW;
     uint32_t at = smem_u32(win0 + (size_t)st * stage_bytes) + 4u * (uint32_t)(s.pix * BW) + 8u * lane;
-    f32x2 p0[VP], p1[VP];
+    f32x2 p0[VP], p1[VP], d[VP];
 #pragma unroll
     for (int q = 0; q < VP; ++q) {
       p0[q] = lds_pair(at + 256u * q);
       p1[q] = lds_pair(at + dstep + 256u * q);
+      if (MODE != kSirt) d[q] = sub2(p1[q], p0[q]);
     }
     if (MODE != kSirt) {
       // weight of the lane's plane: its two taps where they lie on the detector (both: exactly one)
@@ -564,11 +571,18 @@ line_bp_kernel(const __grid_constant__ CUtensorMap map, const LineBpArgs P) {
         for (int q = 0; q < VP; ++q) {
           p0[q] = p1[q];
           p1[q] = lds_pair(at + dstep + 256u * q);
+          if (MODE != kSirt) d[q] = sub2(p1[q], p0[q]);
         }
       }
-      const Weights w = lds_weights(tab + 16u * z);
+      if (MODE == kSirt) {
+        const Weights w = lds_weights(tab + 16u * z);
 #pragma unroll
-      for (int q = 0; q < VP; ++q) acc[z][q] = fma2(w.b, p1[q], fma2(w.a, p0[q], acc[z][q]));
+        for (int q = 0; q < VP; ++q) acc[z][q] = fma2(w.b, p1[q], fma2(w.a, p0[q], acc[z][q]));
+      } else {  // (interpolated first: the sums of the projections round once per angle)
+        const f32x2 f = lds_pair(tab + 16u * z + 8u);
+#pragma unroll
+        for (int q = 0; q < VP; ++q) acc[z][q] = add2(acc[z][q], fma2(f, d[q], p0[q]));
+      }
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[st]);
