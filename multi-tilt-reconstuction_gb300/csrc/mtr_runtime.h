@@ -342,9 +342,10 @@ bool tma_disabled();
 bool autotune_enabled();
 // MTR_FORCE_DEPTHS pins the windowed kernels' tiles (no axis runs on lines).
 bool windows_forced();
-// An axis on line kernels is not tuned; the cache file lists the windowed
-// kernels' heuristic tile for it under a key of its own.
-void record_untimed_tiles(const AxisState& a, const VolDev& v, int precision);
+// An axis on line kernels is not tuned: its shapes follow from the sizes
+// (plan_lines).  The cache file lists them for its reader, under a key of their
+// own with the suffix _lines that nothing looks up.
+void record_line_shapes(const AxisState& a, const VolDev& v, int precision);
 // Candidates run over the frame v on device scratch: scratch_vol / scratch_cbp
 // (FP32) and, in mixed precision, scratch_copy (the BF16 / FP16 copy the
 // forward splat reads); none of them holds data yet.  whole: the volume that v

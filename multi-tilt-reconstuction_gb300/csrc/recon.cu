@@ -682,7 +682,7 @@ mtr_status mtr::recon_create(mtr_context* ctx, int n_axes, const mtr_axis* axes,
       if (s != MTR_OK) return s;
     }
     if (a.lines) {
-      record_untimed_tiles(a, r->vol, params->precision);
+      record_line_shapes(a, r->vol, params->precision);
     } else if (!tma_disabled()) {
       // WBP over the projections' row pairs in r (free until the first residual)
       // SIRT back-projection over the FP32 residual and the forward splat: tuned depths

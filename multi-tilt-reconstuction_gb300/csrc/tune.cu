@@ -196,9 +196,11 @@ bool windows_forced() {
   return f && std::sscanf(f, "%d,%d", &bp, &fwd) == 2;
 }
 
-void record_untimed_tiles(const AxisState& a, const VolDev& v, int precision) {
+void record_line_shapes(const AxisState& a, const VolDev& v, int precision) {
   if (!cache_path()) return;
   Choice c;
+  c.bp_nz = a.line.bp_nz;
+  c.fwd_nz = a.line.fwd_nz;
   c.bp_lane = c.fwd_lane = a.line.along_x ? 0 : 1;
   std::lock_guard<std::mutex> lock(g_mu);
   load_file();
