@@ -306,7 +306,7 @@ __device__ __forceinline__ float tap_weight(float x, int off, int n) {
 // fall on a diagonal of the window that maps several lanes to one shared-memory
 // bank; a patch keeps them compact).  Patches fill a 16x16 square, the smallest
 // footprint, or with the smaller elements of pairs along x a 32x8 brick (FP16
-// pairs, 512x512x64 at 60 degrees: 0.60 against 0.63 ms).  `smem` is the CTA's
+// pairs, 512x512x64 at 60 degrees: 0.60 against 0.63 ms; row pairs 0.52).  `smem` is the CTA's
 // dynamic shared memory; `reinit` re-initialises the mbarriers of a CTA that
 // already ran a brick.  PF (pair format, with PAIR): 0 interleaved FP32
 // pairs; 1 planar FP32 pairs, each detector row as two FP32 rows, its values

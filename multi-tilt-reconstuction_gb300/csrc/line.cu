@@ -180,7 +180,7 @@ line_forward_kernel(const __grid_constant__ CUtensorMap map, const LineArgs P, c
   const size_t kc_bytes = ((size_t)P.max_angles * sizeof(LineConst) + 127) & ~(size_t)127;
   float* red = reinterpret_cast<float*>(smem + kc_bytes);
   float4* table = reinterpret_cast<float4*>(smem + kc_bytes + 128) + (threadIdx.x >> 5) * NZ;
-  int* count0 = reinterpret_cast<int*>(smem + kc_bytes + 128 + kWarps * NZ * sizeof(float4));  // [stages][256]
+  int* count0 = reinterpret_cast<int*>(smem + kc_bytes + 128 + kWarps * NZ * sizeof(float4));  // [stages][kMaxRows]
   unsigned char* win0 = reinterpret_cast<unsigned char*>(count0 + kFwdStages * kMaxRows);
   const int win_elems = P.rows * BW;
   const size_t stage_bytes = (size_t)win_elems * 4;  // a multiple of 128: BW >= 64
@@ -696,7 +696,6 @@ line_rows_kernel(AxisDev ax, int W, int Wp, LineTab tab, const BT* __restrict__ 
         for (int q = 0; q < kBatch; ++q) {
           if (w + 32 * q < W) {
             lt[warp * ws + w + 32 * q] = t[q];
-            
           }
         }
       }

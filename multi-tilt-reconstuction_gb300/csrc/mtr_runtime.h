@@ -281,7 +281,7 @@ struct AxisState {
   long long np = 0;       // A*PY*pitch
   std::vector<double> hxc, hyc;  // host copies of the maps (kernel planning)
   BpPlan plan;            // TMA back-projection window plan over r (FP32)
-  BpPlan plan_b;          // WBP plan (FP32 windows, depth 8)
+  BpPlan plan_b;          // WBP plan: row pairs or plain rows of the projections (plan_wbp)
   CUtensorMap map_b{}, map_r{};  // WBP map over r holding b's row pairs; map over r in its SIRT update's form
   bool tma = false, tma_b = false;
   FwdPlan fplan;          // windowed forward splat plan
@@ -445,13 +445,15 @@ struct mtr_recon {
 namespace mtr {
 // Pieces of a reconstruction's schedule over one span of axis k's volume (recon.cu).
 mtr_status recon_enqueue_forward_span(mtr_recon* r, int k, const VolSpan& sp);
-// mode 0 WBP, 1 SIRT update; widen: widen FP16 projections for a windowed WBP first.
-mtr_status recon_enqueue_bp_span(mtr_recon* r, int k, int mode, const VolSpan& sp, bool widen);
+// mode 0 WBP, 1 SIRT update; prepare: the WBP's image first (recon_enqueue_wbp_image).
+mtr_status recon_enqueue_bp_span(mtr_recon* r, int k, int mode, const VolSpan& sp, bool prepare);
 // mtr_recon_create; row_sums false leaves out the forward row sums, for an
 // object that is only back-projected (no residual).
 mtr_status recon_create(mtr_context* ctx, int n_axes, const mtr_axis* axes, mtr_volume_size vol,
                         const mtr_params* params, int mem_kind, bool row_sums, mtr_recon** out);
-mtr_status recon_enqueue_widen(mtr_recon* r, int k);
+// What the WBP of an axis gathers, prepared in r from its projections in every
+// precision: their line image, row pairs, or (mixed) rows in FP32.
+mtr_status recon_enqueue_wbp_image(mtr_recon* r, int k);
 // Makes a host array's pages resident ahead of a copy into it (contents kept).
 void touch_host_pages(void* p, size_t bytes);
 // Residual of axis k; norm: FP64 sum of r^2 (null: not recorded).

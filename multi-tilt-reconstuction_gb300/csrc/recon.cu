@@ -276,8 +276,8 @@ mtr_status enqueue_residual(mtr_recon* r, AxisState& a, double* norm) {
 }
 
 // What the WBP gathers, prepared in r (free until the first residual): the
-// projections' line image, or their row pairs for the windows.
-mtr_status enqueue_widen_for_wbp(mtr_recon* r, AxisState& a) {
+// projections' line image, or for the windows their row pairs or (mixed) rows.
+mtr_status enqueue_wbp_image(mtr_recon* r, AxisState& a) {
   if (a.lines) {  // the WBP gathers the projections' line image
     const cudaError_t e =
         mixed(r->p.precision)
@@ -301,9 +301,9 @@ mtr_status enqueue_widen_for_wbp(mtr_recon* r, AxisState& a) {
 }
 
 // mode 0: WBP (x = s/c, cbp = c); mode 1: SIRT update from the residual.
-// widen: prepare the WBP's image first (a caller that runs several WBP spans of
+// prepare: the WBP's image first (a caller that runs several WBP spans of
 // one axis prepares it once).
-mtr_status enqueue_bp(mtr_recon* r, AxisState& a, int mode, const VolSpan& sp, bool widen = true) {
+mtr_status enqueue_bp(mtr_recon* r, AxisState& a, int mode, const VolSpan& sp, bool prepare = true) {
   mtr_context* ctx = r->ctx;
   const VolDev& v = r->vol;
   const int z0 = sp.z0, z1 = sp.z1;
@@ -312,8 +312,8 @@ mtr_status enqueue_bp(mtr_recon* r, AxisState& a, int mode, const VolSpan& sp, b
   // WBP reads the projections (fp16 when mixed), SIRT reads the FP32 residual.
   const bool half_img = mode == 0 && mixed(r->p.precision);
   if (a.lines) {
-    if (mode == 0 && widen) {
-      const mtr_status s = enqueue_widen_for_wbp(r, a);
+    if (mode == 0 && prepare) {
+      const mtr_status s = enqueue_wbp_image(r, a);
       if (s != MTR_OK) return s;
     }
     const cudaError_t e = launch_line_backproject(mode == 0 ? a.map_lb : a.map_lr, a.line, a.tab(), a.dev(), v, mode,
@@ -324,8 +324,8 @@ mtr_status enqueue_bp(mtr_recon* r, AxisState& a, int mode, const VolSpan& sp, b
     return MTR_OK;
   }
   if (mode == 0 ? a.tma_b : a.tma) {
-    if (mode == 0 && widen) {
-      mtr_status s = enqueue_widen_for_wbp(r, a);
+    if (mode == 0 && prepare) {
+      mtr_status s = enqueue_wbp_image(r, a);
       if (s != MTR_OK) return s;
     }
     cudaError_t e = launch_backproject_tma<float>(mode == 0 ? a.map_b : a.map_r, mode == 0 ? a.plan_b : a.plan,
@@ -397,10 +397,10 @@ mtr_status mtr::recon_enqueue_init(mtr_recon* r) {
 mtr_status mtr::recon_enqueue_forward_span(mtr_recon* r, int k, const VolSpan& sp) {
   return enqueue_forward(r, r->ax[k], sp);
 }
-mtr_status mtr::recon_enqueue_bp_span(mtr_recon* r, int k, int mode, const VolSpan& sp, bool widen) {
-  return enqueue_bp(r, r->ax[k], mode, sp, widen);
+mtr_status mtr::recon_enqueue_bp_span(mtr_recon* r, int k, int mode, const VolSpan& sp, bool prepare) {
+  return enqueue_bp(r, r->ax[k], mode, sp, prepare);
 }
-mtr_status mtr::recon_enqueue_widen(mtr_recon* r, int k) { return enqueue_widen_for_wbp(r, r->ax[k]); }
+mtr_status mtr::recon_enqueue_wbp_image(mtr_recon* r, int k) { return enqueue_wbp_image(r, r->ax[k]); }
 mtr_status mtr::recon_enqueue_residual_norm(mtr_recon* r, int k, double* norm) {
   return enqueue_residual(r, r->ax[k], norm);
 }

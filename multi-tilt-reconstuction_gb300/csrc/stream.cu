@@ -225,7 +225,7 @@ mtr_status mtr::stream_enqueue_init(mtr_recon* r) {
   if (st != MTR_OK) return st;
   MTR_CK(ctx, cudaMemsetAsync(r->err.p, 0, sizeof(int), c));
   for (int k = 0; k < K; ++k)
-    if ((st = recon_enqueue_widen(r, k)) != MTR_OK) return st;
+    if ((st = recon_enqueue_wbp_image(r, k)) != MTR_OK) return st;
   for (int j = 0; j < S.nslab; ++j) {
     const SlabRange R = slab_range(r, j, S.depth);
     const size_t nb = (size_t)R.n * 4;
