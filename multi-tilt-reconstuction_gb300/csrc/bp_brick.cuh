@@ -662,7 +662,7 @@ bp_tma_kernel(const __grid_constant__ CUtensorMap tmap, const BpArgs P) {
 template <typename PT, int MODE, bool PAIR, int LANES, bool BZ0, int NZ, int PF = 0>
 cudaError_t launch_one(const CUtensorMap& map, const BpArgs& P, size_t smem, cudaStream_t st) {
   auto kern = bp_tma_kernel<PT, MODE, PAIR, LANES, BZ0, NZ, PF>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory(kern, smem);
   if (e != cudaSuccess) return e;
   constexpr int BX = bp_brick_x(LANES, PAIR), BY = bp_brick_y(LANES, PAIR);
   const dim3 grid((P.vol.NX + BX - 1) / BX, (P.z1 - P.z0 + NZ - 1) / NZ, (P.vol.NY + BY - 1) / BY);

@@ -84,7 +84,7 @@ bp_batch_kernel(const BpBatchDesc* __restrict__ descs, const long long* __restri
 
 int backproject_batch_ctas_per_sm(size_t smem) {
   int n = 0;
-  if (cudaFuncSetAttribute(bp_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+  if (allow_shared_memory(bp_batch_kernel, smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bp_batch_kernel, kThreads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 1;
@@ -94,7 +94,7 @@ int backproject_batch_ctas_per_sm(size_t smem) {
 
 cudaError_t launch_backproject_batch(const BpBatchDesc* descs, const long long* first, int n_desc, long long n_items,
                                      size_t smem, int grid, int* err, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(bp_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory(bp_batch_kernel, smem);
   if (e != cudaSuccess) return e;
   launch_overlapped(bp_batch_kernel, grid, kThreads, smem, st, descs, first, n_desc, n_items, err,
                                            g_wait_iters.load(std::memory_order_relaxed));

@@ -810,7 +810,7 @@ cudaError_t launch_one(const CUtensorMap& map, FwdArgs P, int lanes, int num_sms
   P.groups = groups;
   P.max_angles = (P.ax.A + groups - 1) / groups;
   const size_t smem = fwd_smem(P.WX, P.WY, P.nz, NZ <= 0, ROWS, P.max_angles);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory(kern, smem);
   if (e != cudaSuccess) return e;
   launch_overlapped(kern, dim3(b3.x, b3.y, b3.z * groups), kThreads, smem, st, map, P, lanes);
   const cudaError_t le = cudaGetLastError();
@@ -861,8 +861,7 @@ fwd_batch_kernel(const FwdBatchDesc* __restrict__ descs, const long long* __rest
 template <typename VT>
 int forward_batch_ctas_per_sm(size_t smem) {
   int n = 0;
-  if (cudaFuncSetAttribute(fwd_batch_kernel<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-          cudaSuccess ||
+  if (allow_shared_memory(fwd_batch_kernel<VT>, smem) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fwd_batch_kernel<VT>, kThreads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 1;
@@ -873,7 +872,7 @@ int forward_batch_ctas_per_sm(size_t smem) {
 template <typename VT>
 cudaError_t launch_forward_batch(const FwdBatchDesc* descs, const long long* first, int n_desc, long long n_items,
                                  size_t smem, int grid, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(fwd_batch_kernel<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory(fwd_batch_kernel<VT>, smem);
   if (e != cudaSuccess) return e;
   launch_overlapped(fwd_batch_kernel<VT>, grid, kThreads, smem, st, descs, first, n_desc, n_items);
   const cudaError_t le = cudaGetLastError();

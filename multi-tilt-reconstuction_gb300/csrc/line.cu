@@ -793,7 +793,7 @@ cudaError_t run_forward(const CUtensorMap& map, const LinePlan& p, LineArgs L, c
   L.groups = groups;
   L.max_angles = (L.ax.A + groups - 1) / groups;
   const size_t smem = fwd_smem(p, L.max_angles);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory(kern, smem);
   if (e != cudaSuccess) return e;
   launch_overlapped(kern, dim3(gx, gy, gz * groups), kThreads, smem, st, map, L, x);
   e = cudaGetLastError();
@@ -807,7 +807,7 @@ cudaError_t run_bp(const CUtensorMap& map, LineBpArgs P, cudaStream_t st) {
   const LineArgs& L = P.l;
   const int W = L.along_x ? L.vol.NX : L.vol.NY, M = L.along_x ? L.vol.NY : L.vol.NX;
   const size_t smem = bp_smem(L.rows, VL, NZ, L.ax.A);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory(kern, smem);
   if (e != cudaSuccess) return e;
   const dim3 grid((W + 32 * VL - 1) / (32 * VL), (L.z1 - L.z0 + NZ - 1) / NZ, (M + kWarps - 1) / kWarps);
   launch_overlapped(kern, grid, kBpThreads, smem, st, map, P);
@@ -827,7 +827,7 @@ cudaError_t run_rows(const LinePlan& p, const LineTab& tab, const AxisDev& ax, c
                      float* image, double* norm2, cudaStream_t st) {
   auto kern = line_rows_kernel<MODE, BT, NORM>;
   const size_t smem = rows_smem(p.W, ax.PY);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared_memory(kern, smem);
   if (e != cudaSuccess) return e;
   launch_overlapped(kern, dim3((ax.PX + kCols - 1) / kCols, ax.A), 256, smem, st, ax, p.W, p.Wp, tab, b, sums, cf, image,
                     norm2);

@@ -1,6 +1,10 @@
 // Elementwise and MACE consensus kernels (sm_103a).  These are HBM-bound:
 // grid-stride loops over the volume, sized to a multiple of the SM count.
+#include <algorithm>
 #include <atomic>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include "mtr_internal.h"
 
@@ -376,6 +380,20 @@ mace_batch_kernel(const MaceBatchDesc* __restrict__ descs, const long long* __re
 }
 
 }  // namespace
+
+cudaError_t raise_shared_memory_limit(const void* kern, size_t bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> limit;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  size_t& top = limit[{dev, kern}];
+  const size_t want = std::max(top, bytes);
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+  if (e == cudaSuccess) top = want;
+  return e;
+}
 
 int device_sm_count() {
   constexpr int kMaxDevices = 64;

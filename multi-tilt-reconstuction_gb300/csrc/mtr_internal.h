@@ -282,6 +282,15 @@ void launch_mace_batch(const MaceBatchDesc* descs, const long long* first, int n
 // ---- elementwise / MACE (mace.cu) ----------------------------------------
 // Streaming multiprocessors of the current device (queried once per device).
 int device_sm_count();
+// Lets a kernel take `bytes` of dynamic shared memory on the current device.
+// The limit belongs to the kernel, not to a launch, and contexts of other host
+// threads launch the same kernel with other windows: it is only ever raised, so
+// that none lowers it between another's call and its launch.
+cudaError_t raise_shared_memory_limit(const void* kern, size_t bytes);
+template <typename... P>
+inline cudaError_t allow_shared_memory(void (*kern)(P...), size_t bytes) {
+  return raise_shared_memory_limit(reinterpret_cast<const void*>(kern), bytes);
+}
 void launch_fill(float* p, long long n, float v, cudaStream_t st);
 void launch_axpy_acc(float* dst, const float* src, long long n, cudaStream_t st);  // dst += src
 // Fused MACE step over K axes (see mace.cu).  w: the K states, FP32 or
