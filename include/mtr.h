@@ -48,7 +48,7 @@ typedef enum mtr_status {
  * axes of large volumes without a Z term in their y-map, the residual read by
  * the back-projection stored as FP16 (value, next - value) pairs computed in
  * FP32; interpolation and accumulation in FP32; residual norms in FP64, the
- * MACE consensus sum in FP64 or to its accuracy in pairs of FP32 values;
+ * MACE consensus sum in FP64 or in pairs of FP32 values (48 bits);
  * the SIRT iterate (updated every iteration), the weight sums and the
  * consensus stay FP32.  Mixed storage takes less device memory than FP32;
  * values (and residual differences) must lie within the FP16 range.

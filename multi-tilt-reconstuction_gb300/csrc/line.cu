@@ -388,6 +388,10 @@ line_forward_kernel(const __grid_constant__ CUtensorMap map, const LineArgs P, c
 // register in place of one per voxel, and the WBP takes the update's shapes:
 // 512x512x64, 61 angles, 0.32 / 0.31 ms (lines along Y / X) against 0.43 / 0.42
 // with a sum per voxel, which only maps with a row table per angle still need.
+// Its values are interpolated before they are added, from the taps' difference
+// formed at each crossing: one rounding per angle at the size of the sum in place
+// of two (400x384x40, 61 angles: 1.2e-7 of the 64-bit result against 1.7e-7), 0.31 /
+// 0.30 ms.  The update keeps the two multiply-adds, 1 % faster on small volumes.
 struct LineBpArgs {
   LineArgs l;
   LineTab tab;
