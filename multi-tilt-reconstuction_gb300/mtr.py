@@ -343,7 +343,8 @@ class Context:
         if start.size < n:
             raise ValueError(f"sirt: the slab holds {start.size} values, planes {z0} to {z1} need {n}")
         out = np.empty(start.shape, np.float32)
-        out.reshape(-1)[max(n, 0):] = start.reshape(-1)[max(n, 0):]
+        if start.size > n:
+            out.reshape(-1)[max(n, 0):] = start.reshape(-1)[max(n, 0):]
         a = axis.c_struct()
         self.check(self.lib.mtr_sirt_from(self.h, C.byref(a), vol, z0, z1, n_inner, step, _ptr(start), _ptr(out)),
                    "mtr_sirt")
